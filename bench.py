@@ -52,16 +52,18 @@ N_GRID = 512
 H = 0.5
 DT = 0.005
 KMAX = 1.0
-# algorithmic bytes per site per RK4 step with complex64 + Kahan, increment
-# form: stage 1 reads psi and writes d2 (2 x 8 B); stages 2-3 read psi and d
+# algorithmic bytes per site per RK4 step with complex64 + Kahan.  Two stages per
+# launch (single grids): the first pair reads psi and writes psi + d3 and the
+# increments' sum (3 x 8 B), the second reads both, psi and c and writes psi', c
+# (6 x 8 B) -> 72 B/site.  One stage per launch (z-slabs), increment form: stage 1 reads psi and writes d2 (2 x 8 B); stages 2-3 read psi and d
 # (both as stencils) and write the next d (3 x 8 B each); stage 4 reads psi,
 # d4, d2, d3, c and writes psi', c (7 x 8 B) -> 120 B/site (the stage-value +
 # accumulator form moves 152)
 BYTES_PER_FAMILY = {"stage_first": 16, "stage_mid": 24, "stage_last": 56}
 BYTES_PER_STEP = 120
+BYTES_PER_STEP_PAIRS = 72
 # the plain fine path of the learned workload steps at its largest stable dt
 FINE_PATH_DT = 0.02
-LAUNCHES_PER_STEP = 5
 
 
 def load_peaks():
@@ -237,7 +239,7 @@ ENS_KMAX = 0.8
 # complex64 without compensation, increment form: stage 1 reads psi, writes
 # d2 (16 B); stages 2-3 read psi, d and write the next d (24 B each); stage 4
 # reads psi, d4, d2, d3 and writes psi' (40 B)
-ENS_BYTES_PER_SITE = 104
+ENS_BYTES_PER_SITE = 56  # two stages per launch, no compensation: 24 + 32
 
 
 def ensemble_members(seed=0):
@@ -358,7 +360,7 @@ def measure_ensemble(args):
                                "order 2, reflective, RK4 dt=0.01",
                    "sizes": sorted(p.nx for p in prms), "sites": sites,
                    "l2": f"inputs larger than L2 ({8 * sites * 4 / 1e9:.2f} GB of fields)"},
-        "roofline": {"bound": "hbm", "kernel": "stage_kernel (batched, all four stages)",
+        "roofline": {"bound": "hbm", "kernel": "pair_kernel (batched, both pairs)",
                      "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
                      "peak_source": peak_kind, "alg_bytes_per_site_step": ENS_BYTES_PER_SITE,
                      "traffic": None},
@@ -900,8 +902,11 @@ def main():
     sampler = ClockSampler(uuid[-12:] if uuid else None)
     sampler.start()
     time.sleep(0.3)
-    s.set_timing(True)
-    s.timing()  # reset accumulators
+    # per-launch timing steps one stage per launch, as a slab does anyway; a
+    # whole grid is timed as it runs, two stages per launch
+    if slab:
+        s.set_timing(True)
+        s.timing()  # reset accumulators
     lc0 = s.launch_count()
     if dist:
         dist.barrier()
@@ -916,7 +921,7 @@ def main():
         dist.barrier()
     ms = ev0.elapsed_time(ev1)
     launches = s.launch_count() - lc0
-    fam = s.timing()
+    fam = s.timing() if slab else None
     s.set_timing(False)
     clocks = sampler.stop()
     ms_max = ms
@@ -931,26 +936,38 @@ def main():
 
     # roofline of the dominant kernel family and of the whole step
     peak, peak_kind = load_peaks()
-    dominant = max(("stage_first", "stage_mid", "stage_last"), key=lambda f: fam[f]["ms"])
-    d = fam[dominant]
-    per_launch_ms = d["ms"] / max(d["launches"], 1)
-    # bytes from the sites the family's launches covered (a slab's stage is
-    # two launches when its ghost exchange overlaps the interior planes)
-    alg_bytes = BYTES_PER_FAMILY[dominant] * d["sites"] / max(d["launches"], 1)
-    achieved = BYTES_PER_FAMILY[dominant] * d["sites"] / (d["ms"] / 1e3) / 1e9
-    traffic = load_traffic().get(dominant)
-    kernel_ms_step = sum(fam[f]["ms"] for f in ("stage_first", "stage_mid", "stage_last",
-                                                "reduce")) / args.steps
-    step_gbs = BYTES_PER_STEP * sites / (kernel_ms_step / 1e3) / 1e9
-    roofline = {"bound": "hbm", "kernel": f"stage_kernel ({dominant})",
-                "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "peak_source": peak_kind,
-                "traffic": traffic, "alg_bytes_per_launch": alg_bytes,
-                "per_launch_ms": per_launch_ms,
-                "step": {"alg_bytes_per_site": BYTES_PER_STEP, "kernel_ms_per_step": kernel_ms_step,
-                         "achieved": step_gbs, "frac": step_gbs / peak,
-                         "frac_vs_nominal_8000": step_gbs / 8000.0},
-                "families": fam}
+    if slab:
+        dominant = max(("stage_first", "stage_mid", "stage_last"), key=lambda f: fam[f]["ms"])
+        d = fam[dominant]
+        per_launch_ms = d["ms"] / max(d["launches"], 1)
+        # bytes from the sites the family's launches covered (a slab's stage is
+        # two launches when its ghost exchange overlaps the interior planes)
+        alg_bytes = BYTES_PER_FAMILY[dominant] * d["sites"] / max(d["launches"], 1)
+        achieved = BYTES_PER_FAMILY[dominant] * d["sites"] / (d["ms"] / 1e3) / 1e9
+        traffic = load_traffic().get(dominant)
+        kernel_ms_step = sum(fam[f]["ms"] for f in ("stage_first", "stage_mid", "stage_last",
+                                                    "reduce")) / args.steps
+        step_gbs = BYTES_PER_STEP * sites / (kernel_ms_step / 1e3) / 1e9
+        roofline = {"bound": "hbm", "kernel": f"stage_kernel ({dominant})",
+                    "achieved": achieved, "peak": peak, "unit": "GB/s",
+                    "frac": achieved / peak, "peak_source": peak_kind,
+                    "traffic": traffic, "alg_bytes_per_launch": alg_bytes,
+                    "per_launch_ms": per_launch_ms,
+                    "step": {"alg_bytes_per_site": BYTES_PER_STEP, "kernel_ms_per_step": kernel_ms_step,
+                             "achieved": step_gbs, "frac": step_gbs / peak,
+                             "frac_vs_nominal_8000": step_gbs / 8000.0},
+                    "families": fam}
+    else:
+        kernel_ms_step = ms / args.steps
+        step_gbs = BYTES_PER_STEP_PAIRS * sites / (kernel_ms_step / 1e3) / 1e9
+        roofline = {"bound": "hbm", "kernel": "pair_kernel (both pairs of the step, with the "
+                                              "ghost and norm launches after them)",
+                    "achieved": step_gbs, "peak": peak, "unit": "GB/s", "frac": step_gbs / peak,
+                    "peak_source": peak_kind, "traffic": load_traffic().get("pairs"),
+                    "alg_bytes_per_step": BYTES_PER_STEP_PAIRS * sites,
+                    "step": {"alg_bytes_per_site": BYTES_PER_STEP_PAIRS,
+                             "kernel_ms_per_step": kernel_ms_step,
+                             "frac_vs_nominal_8000": step_gbs / 8000.0}}
 
     # end to end through the C-ABI with host buffers (pinned), host<->device
     # copies inside the timed region: the literal solver(var_in, var_out) form

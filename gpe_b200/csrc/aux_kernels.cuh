@@ -2,6 +2,7 @@
 #pragma once
 
 #include "device_utils.cuh"
+#include "vec2.cuh"
 
 namespace gpe {
 
@@ -14,52 +15,169 @@ struct Geom {
 
 __device__ __forceinline__ size_t padded_index(const Geom& g, int i, int j,
                                                int k) {
-  return ((size_t)(k + 2) * g.Ny + (size_t)(j + 2)) * g.Nx + (size_t)(i + 2);
+  return ((size_t)(k + GH) * g.Ny + (size_t)(j + GH)) * g.Nx + (size_t)(i + GH);
 }
 
+// One warp per row of a field: rows r, r + (all warps), ... of `nrows`.
+#define GPE_FOR_ROWS(r, nrows)                                        \
+  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   \
+       r < (nrows); r += gridDim.x * (blockDim.x >> 5))
+
 // Dense interior array (any complex type TI) -> padded field of TS, with the
-// boundary ghosts filled (the caller's halo exchange, src/gpe.f90:165-174).
+// boundary ghosts filled, edges included (the caller's halo exchange,
+// src/gpe.f90:165-174).  One warp per padded row, which it gathers from the
+// interior row it is an image of: every store is in row order.  HBM-bound.
 template <typename TS, typename TI>
-__global__ void unpack_kernel(const TI* __restrict__ src, TS* __restrict__ dst,
-                              Geom g) {
-  const size_t n = (size_t)g.nx * g.ny * g.nz;
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-       q += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(q % g.nx);
-    const size_t r = q / g.nx;
-    const int j = (int)(r % g.ny);
-    const int k = (int)(r / g.ny);
-    const TS vr = (TS)src[2 * q], vi = (TS)src[2 * q + 1];
-    st_one<TS>(dst + 2 * padded_index(g, i, j, k), vr, vi);
-    int a, b;
-    ghost_targets(i, g.nx, g.bcs, a, b);
-    if (a != NO_GHOST) st_one<TS>(dst + 2 * padded_index(g, a, j, k), vr, vi);
-    if (b != NO_GHOST) st_one<TS>(dst + 2 * padded_index(g, b, j, k), vr, vi);
-    ghost_targets(j, g.ny, g.bcs, a, b);
-    if (a != NO_GHOST) st_one<TS>(dst + 2 * padded_index(g, i, a, k), vr, vi);
-    if (b != NO_GHOST) st_one<TS>(dst + 2 * padded_index(g, i, b, k), vr, vi);
-    ghost_targets(k, g.nz, g.bcs, a, b);
-    if (a != NO_GHOST && ((a < 0) ? g.zg_lo : g.zg_hi))
-      st_one<TS>(dst + 2 * padded_index(g, i, j, a), vr, vi);
-    if (b != NO_GHOST && ((b < 0) ? g.zg_lo : g.zg_hi))
-      st_one<TS>(dst + 2 * padded_index(g, i, j, b), vr, vi);
+__global__ void unpack_kernel(const TI* __restrict__ src, TS* __restrict__ dst, Geom g) {
+  const int lane = threadIdx.x & 31;
+  const int Nz = g.nz + 2 * GH;
+  GPE_FOR_ROWS(r, g.Ny * Nz) {
+    const int kp = r / g.Ny, jp = r - kp * g.Ny;
+    const int k = kp - GH, j = jp - GH;
+    if ((k < 0 && !g.zg_lo) || (k >= g.nz && !g.zg_hi)) continue;  // a neighbour sends these
+    const int ks = ghost_source(k, g.nz, g.bcs), js = ghost_source(j, g.ny, g.bcs);
+    const TI* s = src + 2 * ((size_t)ks * g.ny + js) * (size_t)g.nx;
+    TS* d = dst + 2 * ((size_t)r * g.Nx + GH);
+#pragma unroll 4
+    for (int i = lane; i < g.nx; i += 32) {
+      const typename VT<TI>::T v = reinterpret_cast<const typename VT<TI>::T*>(s)[i];
+      st_one<TS>(d + 2 * i, (TS)v.x, (TS)v.y);
+    }
+    if (lane < 2 * GH) {
+      const int i = lane < GH ? lane - GH : g.nx + lane - GH;
+      const typename VT<TI>::T v =
+          reinterpret_cast<const typename VT<TI>::T*>(s)[ghost_source(i, g.nx, g.bcs)];
+      st_one<TS>(d + 2 * i, (TS)v.x, (TS)v.y);
+    }
   }
 }
 
-// Padded field -> dense interior array of TO.
+// Every boundary ghost of a field from its own interior, `depth` deep, edges
+// included.  Rows that lie in the y or z ghosts are copied whole, one per
+// warp; of the interior rows four per warp, eight lanes each, copy the
+// x ghosts.
+template <typename TS>
+__device__ __forceinline__ void fill_ghost_rows(TS* __restrict__ f, const Geom& g, int depth,
+                                                int block, int nblocks) {
+  using V = typename VT<TS>::T;
+  V* F = reinterpret_cast<V*>(f);
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int warps = nblocks * nw, me = block * nw + (threadIdx.x >> 5);
+  // whole rows: z-ghost planes (2 depth of ny + 2 depth rows), then the y-ghost
+  // rows of the interior planes
+  const int Yd = g.ny + 2 * depth, zrows = 2 * depth * Yd, whole = zrows + 2 * depth * g.nz;
+  for (int r = me; r < whole; r += warps) {
+    int j, k;
+    if (r < zrows) {
+      const int kk = r / Yd;
+      k = kk < depth ? kk - depth : g.nz + kk - depth;
+      j = r - kk * Yd - depth;
+    } else {
+      const int q = r - zrows;
+      k = q / (2 * depth);
+      const int jj = q - k * 2 * depth;
+      j = jj < depth ? jj - depth : g.ny + jj - depth;
+    }
+    const size_t from =
+        padded_index(g, 0, ghost_source(j, g.ny, g.bcs), ghost_source(k, g.nz, g.bcs));
+    const size_t to = padded_index(g, 0, j, k);
+    // 16 bytes a lane (rows start 32-byte aligned, GH complexes in)
+    constexpr int W = 16 / (int)sizeof(V);
+    const float4* s4 = reinterpret_cast<const float4*>(F + from);
+    float4* d4 = reinterpret_cast<float4*>(F + to);
+#pragma unroll 4
+    for (int i = lane; i < g.nx / W; i += 32) d4[i] = s4[i];
+    if (W > 1 && lane < g.nx % W) F[to + g.nx - 1] = F[from + g.nx - 1];
+    if (lane < 2 * depth) {
+      const int i = lane < depth ? lane - depth : g.nx + lane - depth;
+      F[to + i] = F[from + ghost_source(i, g.nx, g.bcs)];
+    }
+  }
+  const int rows = g.ny * g.nz, sub = lane >> 3, l = lane & 7;
+  const int i = l < depth ? l - depth : g.nx + l - depth;
+  const int is = ghost_source(i, g.nx, g.bcs);
+#pragma unroll 4
+  for (int r4 = me; r4 * 4 < rows; r4 += warps) {
+    const int r = r4 * 4 + sub;
+    if (r < rows && l < 2 * depth) {
+      const int k = r / g.ny, j = r - k * g.ny;
+      const size_t at = padded_index(g, 0, j, k);
+      F[at + i] = F[at + is];
+    }
+  }
+}
+
+template <typename TS>
+__global__ void fill_ghosts_kernel(TS* __restrict__ f, Geom g, int depth) {
+  fill_ghost_rows<TS>(f, g, depth, blockIdx.x, gridDim.x);
+}
+
+// Fixed-order reduction of slot `slot` of the per-CTA partials by one block
+// (sum, or max for op 1); the result is s[0] for every thread on return.
+__device__ __forceinline__ void reduce_partials(const double* __restrict__ partials, int nblk,
+                                                int slot, int op, double* s) {
+  double a = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    const double v = partials[2 * (size_t)b + slot];
+    a = op ? fmax(a, v) : a + v;
+  }
+  s[threadIdx.x] = a;
+  __syncthreads();
+  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) {
+      const double v = s[threadIdx.x + w];
+      s[threadIdx.x] = op ? fmax(s[threadIdx.x], v) : s[threadIdx.x] + v;
+    }
+    __syncthreads();
+  }
+}
+
+// The end of a step in pairs, blocks of 1024 threads: block 0 reduces the norm
+// as finalize_kernel does, the others fill the new psi's ghosts.
+template <typename TS>
+__global__ void __launch_bounds__(1024) ghosts_norm_kernel(TS* __restrict__ f, Geom g, int depth,
+                                                            const double* __restrict__ partials,
+                                                            int nblk, double scale,
+                                                            double* __restrict__ out,
+                                                            double* __restrict__ series) {
+  __shared__ double s[1024];
+  if (blockIdx.x > 0) {
+    fill_ghost_rows<TS>(f, g, depth, blockIdx.x - 1, gridDim.x - 1);
+    return;
+  }
+  reduce_partials(partials, nblk, 0, 0, s);
+  if (threadIdx.x == 0) {
+    const double r = s[0] * scale;
+    out[0] = r;
+    if (series) *series = r;
+  }
+}
+
+// The ghosts of one field per member of a batch (blockIdx.y).
+struct GhostRun {
+  void* field;
+  Geom g;
+};
+template <typename TS>
+__global__ void batch_ghosts_kernel(const GhostRun* __restrict__ runs, int depth) {
+  const GhostRun r = runs[blockIdx.y];
+  fill_ghost_rows<TS>(static_cast<TS*>(r.field), r.g, depth, blockIdx.x, gridDim.x);
+}
+
+// Padded field -> dense interior array of TO, one warp per row.
 template <typename TS, typename TO>
-__global__ void pack_kernel(const TS* __restrict__ src, TO* __restrict__ dst,
-                            Geom g) {
-  const size_t n = (size_t)g.nx * g.ny * g.nz;
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-       q += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(q % g.nx);
-    const size_t r = q / g.nx;
-    const int j = (int)(r % g.ny);
-    const int k = (int)(r / g.ny);
-    const size_t s = padded_index(g, i, j, k);
-    dst[2 * q] = (TO)src[2 * s];
-    dst[2 * q + 1] = (TO)src[2 * s + 1];
+__global__ void pack_kernel(const TS* __restrict__ src, TO* __restrict__ dst, Geom g) {
+  const int lane = threadIdx.x & 31;
+  GPE_FOR_ROWS(r, g.ny * g.nz) {
+    const int k = r / g.ny, j = r - k * g.ny;
+    const typename VT<TS>::T* s =
+        reinterpret_cast<const typename VT<TS>::T*>(src) + padded_index(g, 0, j, k);
+    TO* d = dst + 2 * (size_t)r * g.nx;
+#pragma unroll 4
+    for (int i = lane; i < g.nx; i += 32) {
+      const typename VT<TS>::T v = s[i];
+      st_one<TO>(d + 2 * i, (TO)v.x, (TO)v.y);
+    }
   }
 }
 
@@ -95,17 +213,19 @@ __global__ void norm_kernel(const TS* __restrict__ f, Geom g,
                             const double* __restrict__ wz,
                             double* __restrict__ partials) {
   __shared__ double s[32];
-  const size_t n = (size_t)g.nx * g.ny * g.nz;
+  const int lane = threadIdx.x & 31;
   double acc = 0.0;
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-       q += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(q % g.nx);
-    const size_t r = q / g.nx;
-    const int j = (int)(r % g.ny);
-    const int k = (int)(r / g.ny);
-    const size_t pi = padded_index(g, i, j, k);
-    const double a = (double)f[2 * pi], b = (double)f[2 * pi + 1];
-    acc += (wx[i] * wy[j]) * wz[k] * (a * a + b * b);
+  GPE_FOR_ROWS(r, g.ny * g.nz) {
+    const int k = r / g.ny, j = r - k * g.ny;
+    const typename VT<TS>::T* row =
+        reinterpret_cast<const typename VT<TS>::T*>(f) + padded_index(g, 0, j, k);
+    const double wyj = wy[j], wzk = wz[k];
+#pragma unroll 4
+    for (int i = lane; i < g.nx; i += 32) {
+      const typename VT<TS>::T v = row[i];
+      const double a = (double)v.x, b = (double)v.y;
+      acc += (wx[i] * wyj) * wzk * (a * a + b * b);
+    }
   }
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
@@ -119,42 +239,18 @@ __global__ void norm_kernel(const TS* __restrict__ f, Geom g,
 }
 
 // Fixed-order reduction of partials[2*b + slot], b < nblk, by one CTA of
-// 1024 threads.  op 0 = sum, 1 = max.  out[0] = result * scale; when
-// `series` is non-null also series[*counter] = out[0] and ++*counter.
-// Fixed-order reduction of slot `slot` of the per-CTA partials by one block
-// (sum, or max for op 1); the result is s[0] for every thread on return.
-__device__ __forceinline__ void reduce_partials(const double* __restrict__ partials, int nblk,
-                                                int slot, int op, double* s) {
-  double a = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-    const double v = partials[2 * (size_t)b + slot];
-    a = op ? fmax(a, v) : a + v;
-  }
-  s[threadIdx.x] = a;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      const double v = s[threadIdx.x + w];
-      s[threadIdx.x] = op ? fmax(s[threadIdx.x], v) : s[threadIdx.x] + v;
-    }
-    __syncthreads();
-  }
-}
-
+// 1024 threads.  op 0 = sum, 1 = max.  out[0] = result * scale, written to
+// *series too when it is non-null.
 __global__ void finalize_kernel(const double* __restrict__ partials, int nblk,
                                 int slot, int op, double scale,
                                 double* __restrict__ out,
-                                double* __restrict__ series,
-                                int* __restrict__ counter) {
+                                double* __restrict__ series) {
   __shared__ double s[1024];
   reduce_partials(partials, nblk, slot, op, s);
   if (threadIdx.x == 0) {
     const double r = s[0] * scale;
     out[0] = r;
-    if (series) {
-      series[*counter] = r;
-      *counter = *counter + 1;
-    }
+    if (series) *series = r;
   }
 }
 

@@ -117,7 +117,7 @@ struct ConvParams {
   __nv_bfloat16* pre_out;           // EPI_GELU_PRE
   const __nv_bfloat16* pre_in;      // EPI_DGELU
   float* delta;                     // EPI_DELTA: dense [nz][ny][nx][2]
-  float* psi;                       // EPI_RESID: solver field (complex64, 2 ghosts)
+  float* psi;                       // EPI_RESID: solver field (complex64, GH ghosts)
   int psi_Nx, psi_Ny;
   float out_scale;
   int* status;
@@ -260,7 +260,7 @@ struct EpiAux {
 };
 
 __device__ __forceinline__ size_t psi_index(const ConvParams& p, int x, int y, int z) {
-  return ((size_t)(z + 2) * p.psi_Ny + (y + 2)) * p.psi_Nx + (x + 2);
+  return ((size_t)(z + GH) * p.psi_Ny + (y + GH)) * p.psi_Nx + (x + GH);
 }
 
 template <int EPI>
@@ -304,16 +304,16 @@ __device__ __forceinline__ void conv_epilogue(const ConvParams& p, const float (
     const size_t s = ((size_t)z * p.ny + y) * p.nx + x;
     reinterpret_cast<float2*>(p.delta)[s] =
         make_float2((acc[0] + bias[0]) * p.out_scale, (acc[1] + bias[1]) * p.out_scale);
-  } else {  // EPI_RESID: psi += delta on the solver's field, ghosts (2, periodic) too
+  } else {  // EPI_RESID: psi += delta on the solver's field, its periodic ghosts too
     float2 v = aux.psi;
     v.x += (acc[0] + bias[0]) * p.out_scale;
     v.y += (acc[1] + bias[1]) * p.out_scale;
     float2* f = reinterpret_cast<float2*>(p.psi);
     int gx[3] = {x, NO_GHOST, NO_GHOST}, gy[3] = {y, NO_GHOST, NO_GHOST},
         gz[3] = {z, NO_GHOST, NO_GHOST};
-    ghost_targets(x, p.nx, 1, gx[1], gx[2]);
-    ghost_targets(y, p.ny, 1, gy[1], gy[2]);
-    ghost_targets(z, p.nz, 1, gz[1], gz[2]);
+    ghost_targets(x, p.nx, 1, GH, gx[1], gx[2]);
+    ghost_targets(y, p.ny, 1, GH, gy[1], gy[2]);
+    ghost_targets(z, p.nz, 1, GH, gz[1], gz[2]);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       if (gz[c] == NO_GHOST) continue;
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
 // --------------------------------------------------------------------------
 // Element-wise and reduction kernels.
 
-// Solver field (2 ghosts, pitches Nx, Ny; complex of TS) -> first-layer input
+// Solver field (GH ghosts, pitches Nx, Ny; complex of TS) -> first-layer input
 // (channels Re, Im, 0, ...; H halves), ghosts included.  Every padded site
 // reads its periodic interior source (the solver keeps only the face ghosts
 // a star stencil needs, not edges and corners): one block per padded (y, z)
@@ -739,7 +739,7 @@ __global__ void pack_input_kernel(const TS* __restrict__ psi, int Nx, int Ny, in
   const int yp = row % Yp, zp = row / Yp;
   const int y = yp == 0 ? ny - 1 : (yp == ny + 1 ? 0 : yp - 1);
   const int z = zp == 0 ? nz - 1 : (zp == nz + 1 ? 0 : zp - 1);
-  const size_t q0 = ((size_t)(z + 2) * Ny + (y + 2)) * Nx + 2;
+  const size_t q0 = ((size_t)(z + GH) * Ny + (y + GH)) * Nx + GH;
   __nv_bfloat16* dst = act + (size_t)row * H * Xp * 8;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   for (int xp = threadIdx.x; xp < Xp; xp += blockDim.x) {
@@ -769,7 +769,7 @@ __global__ void loss_kernel(const float* __restrict__ delta, const TS* __restric
     const int x = (int)(s % nx);
     const size_t t = s / nx;
     const int y = (int)(t % ny), z = (int)(t / ny);
-    const size_t q = ((size_t)(z + 2) * Ny + (y + 2)) * Nx + (x + 2);
+    const size_t q = ((size_t)(z + GH) * Ny + (y + GH)) * Nx + (x + GH);
     const double er = (double)u[2 * q] + (double)delta[2 * s] - (double)target[2 * s];
     const double ei = (double)u[2 * q + 1] + (double)delta[2 * s + 1] - (double)target[2 * s + 1];
     acc += er * er + ei * ei;
@@ -890,7 +890,7 @@ __global__ void pack_out2_kernel(const float* __restrict__ w, __nv_bfloat16* __r
   wf2[i] = __float2bfloat16_rn(v);
 }
 
-// 2:1 restriction (2x2x2 average) of a solver field (2 ghosts) to a dense
+// 2:1 restriction (2x2x2 average) of a solver field (GH ghosts) to a dense
 // complex array of TO on the coarse grid.
 template <typename TS, typename TO>
 __global__ void restrict_kernel(const TS* __restrict__ f, int Nx, int Ny, int nxc, int nyc,
@@ -905,7 +905,8 @@ __global__ void restrict_kernel(const TS* __restrict__ f, int Nx, int Ny, int nx
     for (int c = 0; c < 2; c++)
       for (int b = 0; b < 2; b++)
         for (int a = 0; a < 2; a++) {
-          const size_t q = ((size_t)(2 * z + c + 2) * Ny + (2 * y + b + 2)) * Nx + (2 * x + a + 2);
+          const size_t q =
+              ((size_t)(2 * z + c + GH) * Ny + (2 * y + b + GH)) * Nx + (2 * x + a + GH);
           re += (double)f[2 * q];
           im += (double)f[2 * q + 1];
         }

@@ -70,6 +70,21 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
+// try_wait that may suspend the warp for up to `hint_ns` before it gives up:
+// a warp that waits long leaves its issue slots to its siblings.
+__device__ __forceinline__ bool mbar_try_wait_for(uint64_t* bar, uint32_t parity,
+                                                  uint32_t hint_ns) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
+      : "memory");
+  return ok != 0;
+}
+
 // Wait for phase `parity` of an mbarrier, giving up after limit_ns.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar,
                                                   uint32_t parity,
@@ -77,7 +92,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar,
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = global_timer_ns();
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait_for(bar, parity, 20000u)) return true;
     if (global_timer_ns() - t0 > limit_ns) return false;
   }
 }
@@ -172,25 +187,27 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// Ghost layers every stored field has on each side of each axis: two stages of
+// an order-4 stencil reach 4 sites, which pair_kernel.cuh evaluates in one
+// launch (the one-stage kernels read and fill the inner 2).
+constexpr int GH = 4;
+
 // Ghost targets of interior index i along an axis of n points: the ghost
-// positions (-2, -1, n, n+1) whose value is a copy of point i.  Periodic
-// (bcs 1): ghost g holds f(g mod n).  Reflective (bcs 2): mirror about the
-// end nodes, f(-1)=f(1), f(-2)=f(2), f(n)=f(n-2), f(n+1)=f(n-3).
+// positions within `depth` of the ends whose value is a copy of point i.
+// Periodic (bcs 1): ghost g holds f(g mod n).  Reflective (bcs 2): mirror about
+// the end nodes, f(-g) = f(g), f(n-1+g) = f(n-1-g).  At most two for n >= 6.
 constexpr int NO_GHOST = -1000000;
-__device__ __forceinline__ void ghost_targets(int i, int n, int bcs, int& g0,
-                                              int& g1) {
-  g0 = NO_GHOST;
-  g1 = NO_GHOST;
-  int s0, s1, s2, s3;
-  if (bcs == 1) {
-    s0 = n - 2; s1 = n - 1; s2 = 0; s3 = 1;
-  } else {
-    s0 = 2; s1 = 1; s2 = n - 2; s3 = n - 3;
-  }
-  if (s0 == i) { g0 = -2; }
-  if (s1 == i) { if (g0 == NO_GHOST) g0 = -1; else g1 = -1; }
-  if (s2 == i) { if (g0 == NO_GHOST) g0 = n; else g1 = n; }
-  if (s3 == i) { if (g0 == NO_GHOST) g0 = n + 1; else g1 = n + 1; }
+__device__ __forceinline__ void ghost_targets(int i, int n, int bcs, int depth, int& g0, int& g1) {
+  const int lo = bcs == 1 ? i - n : -i;              // image below 0
+  const int hi = bcs == 1 ? i + n : 2 * (n - 1) - i;  // image above n - 1
+  g0 = (lo < 0 && lo >= -depth && i >= 0 && i < n) ? lo : NO_GHOST;
+  g1 = (hi >= n && hi < n + depth && i >= 0 && i < n) ? hi : NO_GHOST;
+}
+
+// Interior index whose value position g (-GH <= g < n + GH) holds.
+__device__ __forceinline__ int ghost_source(int g, int n, int bcs) {
+  if (bcs == 1) return g < 0 ? g + n : g >= n ? g - n : g;
+  return g < 0 ? -g : g >= n ? 2 * (n - 1) - g : g;
 }
 
 }  // namespace gpe

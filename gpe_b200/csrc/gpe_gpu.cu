@@ -1,7 +1,7 @@
 // gpe_gpu.cu -- context, stage scheduling and the C-ABI of include/gpe_gpu.h.
 //
 // One context = one run on one device.  Fields live in a ghost-padded layout
-// (2 ghost layers on every axis, x pitch rounded to 4 elements) so that each
+// (GH ghost layers on every axis, x pitch rounded to 4 elements) so that each
 // stage kernel reads its stencil plane as one TMA box; ghosts are refreshed by
 // the kernel that writes the field (see stage_kernel.cuh), which replaces the
 // reference's halo exchange (src/variables.f90:186-358).
@@ -25,6 +25,8 @@
 #include "aux_kernels.cuh"
 #include "gpe_gpu.h"
 #include "internal.h"
+#include "pair.h"
+#include "pair_kernel.cuh"
 #include "stage_kernel.cuh"
 
 using cd = std::complex<double>;
@@ -118,6 +120,15 @@ struct LaunchShape {
   unsigned halo_box, pt_box, halo_smem, pt_smem;
 };
 
+struct PairShape {
+  int TY = 0, S = 0;
+  unsigned s_bytes = 0, base_bytes = 0, pt_bytes = 0, base_off = 0, comp_off = 0,
+           slot_stride = 0, pt_stride = 0, u_stride = 0, pt_ring = 0, u_ring = 0, d_ring = 0;
+  size_t smem = 0;
+  int threads_y = 0;  // warps
+  int occ = 0;
+};
+
 struct Launch {
   int family;
   cudaEvent_t a, b;
@@ -161,12 +172,12 @@ struct gpe_ctx {
   double* d_series = nullptr;
   size_t series_cap = 0;
   int64_t series_steps = 0;  // steps the last rk45 advance recorded
-  int* d_counter = nullptr;
   int* d_status = nullptr;
   void* d_stage = nullptr;  // dense staging, nint * 16 bytes
   void* h_pinned = nullptr;
   size_t h_pinned_bytes = 0;
   bool norm_valid = false;
+  double* step_series = nullptr;  // where the running step's norm goes too (advance)
   unsigned long long wait_limit_ns = 2000000000ull;
   int stall_plane = -1;  // failure-detection test hook (gpe_gpu_test_stall)
   int64_t launches = 0;
@@ -174,6 +185,7 @@ struct gpe_ctx {
   int64_t device_bytes = 0;
   std::map<std::tuple<int, int, int, int>, CUtensorMap> maps;
   std::map<const void*, LaunchShape> shapes;
+  std::map<const void*, PairShape> pair_shapes;
   bool timing = false;
   std::vector<Launch> timed;
   gpe_timing acc_timing;
@@ -198,6 +210,7 @@ struct gpe_ctx {
   cudaGraphExec_t rk_exec[2] = {nullptr, nullptr};
   int rk_psi[2] = {-1, -1};  // psi buffer each captured step starts from
   bool ghosts_dirty = false;  // psi loaded alone; its z ghosts await the group
+  bool wide = false;  // psi's ghosts are filled 2R deep, edges included (pair_kernel.cuh)
   std::string err;
 };
 
@@ -222,6 +235,7 @@ int gpe_internal_field_view(gpe_ctx* c, gpe::FieldView* v) {
   if (!c || !v) return GPE_ERR_INVALID;
   v->psi = c->fld[c->psi_id];
   v->nx = c->nx; v->ny = c->ny; v->nz = c->nz; v->Nx = c->Nx; v->Ny = c->Ny;
+  v->gh = GH;
   v->es = c->es;
   v->bcs = c->prm.bcs;
   v->dev = c->dev;
@@ -275,10 +289,11 @@ int ensure_encode(gpe_ctx* c) {
   return GPE_OK;
 }
 
-// kind 0: halo box (64+4) x (TY+2R); kind 1: pointwise box 64 x TY.
+// kind 0: halo box (64+4) x (TY+2R); kind 1: pointwise box 64 x TY; kinds 2
+// and 3: the pair kernel's boxes of halo 2R and R.
 int get_map(gpe_ctx* c, int field, int kind, int TY, int R,
             CUtensorMap* out) {
-  auto key = std::make_tuple(field, kind, TY, kind == 0 ? R : 0);
+  auto key = std::make_tuple(field, kind, TY, kind == 1 ? 0 : R);
   auto it = c->maps.find(key);
   if (it != c->maps.end()) {
     *out = it->second;
@@ -295,9 +310,14 @@ int get_map(gpe_ctx* c, int field, int kind, int TY, int R,
   if (kind == 0) {
     box[0] = (cuuint32_t)(W * (TX + 4));
     box[1] = (cuuint32_t)(TY + 2 * R);
-  } else {
+  } else if (kind == 1) {
     box[0] = (cuuint32_t)(W * TX);
     box[1] = (cuuint32_t)TY;
+  } else {
+    const bool f32 = c->es == 8, wide = kind == 2;
+    box[0] = (cuuint32_t)(W * (f32 ? (wide ? PairTile<float>::BW : PairTile<float>::UW)
+                                   : (wide ? PairTile<double>::BW : PairTile<double>::UW)));
+    box[1] = (cuuint32_t)(TY + (wide ? 4 : 2) * R);
   }
   box[2] = 1;
   cuuint32_t estr[3] = {1, 1, 1};
@@ -338,11 +358,11 @@ int exchange_ghosts(gpe_ctx* c, int field, cudaStream_t st = nullptr) {
   if (!st) st = c->stream;
   const size_t plane = (size_t)c->Nx * c->Ny * (size_t)c->es;  // bytes
   unsigned char* f = static_cast<unsigned char*>(c->fld[field]);
-  // padded plane index pz = z + 2
-  unsigned char* bottom = f + 2 * plane;                    // z = 0, 1
-  unsigned char* top = f + (size_t)c->nz * plane;           // z = nz-2, nz-1
-  unsigned char* ghost_lo = f;                              // z = -2, -1
-  unsigned char* ghost_hi = f + (size_t)(c->nz + 2) * plane; // z = nz, nz+1
+  // padded plane index pz = z + GH
+  unsigned char* bottom = f + GH * plane;                        // z = 0, 1
+  unsigned char* top = f + (size_t)(c->nz - 2 + GH) * plane;     // z = nz-2, nz-1
+  unsigned char* ghost_lo = f + (GH - 2) * plane;                // z = -2, -1
+  unsigned char* ghost_hi = f + (size_t)(c->nz + GH) * plane;    // z = nz, nz+1
   const size_t n = 2 * plane;
   NCCL_CHECK(c, g_nccl.GroupStart());
   if (c->exch_hi) NCCL_CHECK(c, g_nccl.Send(top, n, ncclUint8, c->nbr_hi, c->comm, st));
@@ -635,30 +655,26 @@ void recipe_masks(const StageSpec& sp, int* am, int* bm) {
   }
 }
 
-// Per-run part of a stage launch.
+// A grid that a correction network can be attached to (gpe_cnn_create:
+// complex64, periodic, nx a multiple of 16 up to 128).  The network rounds psi
+// to bfloat16, which makes last-bit differences of psi differences of 1e-5, so
+// rk4 keeps on these grids the summation order its weights were trained with,
+// d4, d2, d3 one after another, attached or not; on all others the pointwise
+// increments are summed first, which lets two stages share a launch with one
+// stored sum (pair_kernel.cuh).
+bool network_grid(const gpe_ctx* c) {
+  return c->es == 8 && c->prm.bcs == 1 && c->nx % 16 == 0 && c->nx <= 128;
+}
+
+// Per-run part of a launch that does not depend on its fields: geometry,
+// stencil and right-hand-side coefficients, tables.
 template <typename TS, typename TC>
-int fill_run(gpe_ctx* c, const StageSpec& sp, int R, const LaunchShape& sh,
-             RhsForm f, RunDesc<TS, TC>* rd, int force_full = -1) {
-  if (force_full >= 0) f.full = force_full != 0;
-  memset(rd, 0, sizeof(*rd));
-  int rc = get_map(c, sp.stencil, 0, sh.TY, R, &rd->maps.halo);
-  if (rc) return rc;
-  if (sp.stencil2 >= 0) {
-    rc = get_map(c, sp.stencil2, 0, sh.TY, R, &rd->maps.halo2);
-    if (rc) return rc;
-  }
-  for (int q = 0; q < sp.np; q++) {
-    rc = get_map(c, sp.pt[q], 1, sh.TY, R, &rd->maps.pt[q]);
-    if (rc) return rc;
-  }
+void fill_geometry(const gpe_ctx* c, int R, const RhsForm& f, RunDesc<TS, TC>* rd) {
   rd->nx = c->nx; rd->ny = c->ny; rd->nz = c->nz; rd->Nx = c->Nx; rd->Ny = c->Ny;
-  rd->ntx = sh.ntx; rd->nty = sh.nty; rd->zchunk = sh.zchunk; rd->nchunks = sh.nchunks;
   rd->bcs = c->prm.bcs;
+  rd->acc_first = network_grid(c) ? 0 : 1;
   rd->zg_lo = c->exch_lo ? 0 : 1;
   rd->zg_hi = c->exch_hi ? 0 : 1;
-  rd->stencil = static_cast<const TS*>(c->fld[sp.stencil]);
-  rd->stencil2 = sp.stencil2 >= 0 ? static_cast<const TS*>(c->fld[sp.stencil2]) : nullptr;
-  for (int o = 0; o < sp.nout; o++) rd->out[o] = static_cast<TS*>(c->fld[sp.out[o]]);
   const double h2[3] = {c->dx * c->dx, c->dy * c->dy, c->dz * c->dz};
   double c1[3], c2[3];
   const double r2 = c->prm.fd_match * c->prm.fd_match;
@@ -692,6 +708,29 @@ int fill_run(gpe_ctx* c, const StageSpec& sp, int R, const LaunchShape& sh,
   }
   rd->eg = c->prm.g;
   rd->emu = c->prm.mu;
+}
+
+// Per-run part of a stage launch.
+template <typename TS, typename TC>
+int fill_run(gpe_ctx* c, const StageSpec& sp, int R, const LaunchShape& sh,
+             RhsForm f, RunDesc<TS, TC>* rd, int force_full = -1) {
+  if (force_full >= 0) f.full = force_full != 0;
+  memset(rd, 0, sizeof(*rd));
+  int rc = get_map(c, sp.stencil, 0, sh.TY, R, &rd->maps.halo);
+  if (rc) return rc;
+  if (sp.stencil2 >= 0) {
+    rc = get_map(c, sp.stencil2, 0, sh.TY, R, &rd->maps.halo2);
+    if (rc) return rc;
+  }
+  for (int q = 0; q < sp.np; q++) {
+    rc = get_map(c, sp.pt[q], 1, sh.TY, R, &rd->maps.pt[q]);
+    if (rc) return rc;
+  }
+  rd->ntx = sh.ntx; rd->nty = sh.nty; rd->zchunk = sh.zchunk; rd->nchunks = sh.nchunks;
+  rd->stencil = static_cast<const TS*>(c->fld[sp.stencil]);
+  rd->stencil2 = sp.stencil2 >= 0 ? static_cast<const TS*>(c->fld[sp.stencil2]) : nullptr;
+  for (int o = 0; o < sp.nout; o++) rd->out[o] = static_cast<TS*>(c->fld[sp.out[o]]);
+  fill_geometry<TS, TC>(c, R, f, rd);
   return GPE_OK;
 }
 
@@ -843,14 +882,15 @@ int group_exchange(gpe_group* g, int field, cudaStream_t st = nullptr) {
     if (c->exch_lo) {
       const gpe_ctx* lo = g->m[c->nbr_lo];
       const unsigned char* src = static_cast<const unsigned char*>(lo->fld[field]) +
-                                 (size_t)lo->nz * plane;  // its z = nz-2, nz-1
-      CU_CHECK(c, cudaMemcpyAsync(f, src, 2 * plane, cudaMemcpyDeviceToDevice, st));
+                                 (size_t)(lo->nz - 2 + GH) * plane;  // its z = nz-2, nz-1
+      CU_CHECK(c, cudaMemcpyAsync(f + (GH - 2) * plane, src, 2 * plane,
+                                  cudaMemcpyDeviceToDevice, st));
     }
     if (c->exch_hi) {
       const gpe_ctx* hi = g->m[c->nbr_hi];
       const unsigned char* src = static_cast<const unsigned char*>(hi->fld[field]) +
-                                 2 * plane;  // its z = 0, 1
-      CU_CHECK(c, cudaMemcpyAsync(f + (size_t)(c->nz + 2) * plane, src, 2 * plane,
+                                 GH * plane;  // its z = 0, 1
+      CU_CHECK(c, cudaMemcpyAsync(f + (size_t)(c->nz + GH) * plane, src, 2 * plane,
                                   cudaMemcpyDeviceToDevice, st));
     }
   }
@@ -893,6 +933,7 @@ int ensure_side(gpe_ctx* c, cudaStream_t* xs, cudaEvent_t* ev) {
 int launch_stage(gpe_ctx* c, const StageSpec& sp) {
   bool ghosts = false;
   for (int o = 0; o < sp.nout; o++) ghosts = ghosts || (sp.ghost_mask & (1 << o));
+  if (ghosts) c->wide = false;  // one-stage launches fill the inner ghosts only
   if (c->group) {
     gpe_group* g = c->group;
     bool split = ghosts;
@@ -978,6 +1019,9 @@ int elementwise_blocks(size_t n) {
   return (int)std::min<size_t>(b, 148 * 16);
 }
 
+// Blocks of 8 warps for a kernel that takes one row per warp.
+int row_blocks(size_t rows) { return (int)std::min<size_t>((rows + 7) / 8, 148 * 16); }
+
 void begin_timed(gpe_ctx* c, Launch& L, int family, int64_t sites) {
   if (!c->timing) return;
   L.family = family;
@@ -997,9 +1041,8 @@ int finalize_one(gpe_ctx* c, int nblk, int slot, int op, double scale,
                  int out_index, bool series) {
   Launch L{};
   begin_timed(c, L, GPE_FAM_REDUCE, 0);
-  finalize_kernel<<<1, 1024, 0, c->stream>>>(
-      c->d_partials, nblk, slot, op, scale, c->d_scal + out_index,
-      series ? c->d_series : nullptr, c->d_counter);
+  finalize_kernel<<<1, 1024, 0, c->stream>>>(c->d_partials, nblk, slot, op, scale,
+                                              c->d_scal + out_index, series ? c->step_series : nullptr);
   CU_CHECK(c, cudaGetLastError());
   end_timed(c, L);
   c->launches++;
@@ -1078,10 +1121,268 @@ int step_euler(gpe_ctx* c, cd dt) {
   int rc = launch_stage(c, s);
   if (rc) return rc;
   swap_psi(c);
-  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, false);
+  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, true);
+}
+
+// --------------------------------------------------------------------------
+// Pairs of stages (pair_kernel.cuh).
+
+struct PairSpec {
+  int kind = PAIR_RK4_A;
+  int s = F_PSI, base = -1, acc = -1, comp = -1;  // fields read
+  int out0 = F_ALT, out1 = -1;                    // fields written (out1: no ghosts)
+  cd a[2] = {cd(0), cd(0)};
+  int family = GPE_FAM_OTHER;
+};
+
+// A context steps with pairs unless its z ghosts come from neighbours (two
+// planes are exchanged, a pair needs four), per-launch timing is on, whose
+// families are single stages, the equation has the sphere mask, rk4 keeps the
+// increments apart (network_grid), or the full form, whose terms
+// spill the pair's registers, except in complex64 at order 2 (equation 1 at
+// 150 x 93 x 71, rk4, us a step in pairs and in stages: 54 and 59 there;
+// complex128 95 and 97 at order 2, 182 and 125 at order 4; rk2 at 200 x 193 x
+// 171, complex128, order 2: 223 and 209).
+bool steps_in_pairs(const gpe_ctx* c) {
+  if (c->comm || c->group || c->nzg != c->nz || c->timing || c->prm.eqn_to_solve == 3) return false;
+  if (c->prm.scheme == GPE_SCHEME_RK4 && network_grid(c)) return false;
+  return (c->prm.order == 2 && c->es == 8) || !rhs_form(c).full;
+}
+
+template <typename T>
+int pair_shape(gpe_ctx* c, KernelFn fn, int R, const PairSpec& sp, int tile_y, PairShape* out) {
+  PairShape s;
+  // complex64: 16 rows (the ring's share of the first stage falls from 1.6 to
+  // 1.3 sites per site against 8) unless the grid has no more than 8
+  s.TY = tile_y > 0 ? tile_y : std::min(PairTile<T>::TY_MAX, c->ny <= 8 ? 8 : 16);
+  const unsigned es = 2 * sizeof(T);
+  s.s_bytes = (unsigned)(PairTile<T>::BW * (s.TY + 4 * R)) * es;
+  s.base_bytes = (unsigned)(PairTile<T>::UW * (s.TY + 2 * R)) * es;
+  s.pt_bytes = (unsigned)(TX * s.TY) * es;
+  s.u_stride = (unsigned)round_up(s.base_bytes, 128);
+  size_t at = round_up(s.s_bytes, 128);
+  if (sp.base >= 0) {
+    s.base_off = (unsigned)at;
+    at += round_up(s.base_bytes, 128);
+  }
+  s.slot_stride = (unsigned)at;
+  at = 0;
+  if (sp.acc >= 0) at += round_up(s.pt_bytes, 128);
+  if (sp.comp >= 0) {
+    s.comp_off = (unsigned)at;
+    at += round_up(s.pt_bytes, 128);
+  }
+  s.pt_stride = (unsigned)at;
+  // R + 1 slots are held by the compute warps; the rest are in flight
+  const size_t d_bytes = pair_d_in_smem<T>(R, sp.kind) ? (size_t)(R + 1) * s.pt_bytes : 0;
+  const size_t rest = (size_t)PT_SLOTS * s.pt_stride + (size_t)U_SLOTS * s.u_stride + d_bytes;
+  s.S = (int)std::min<size_t>(8, (231000 - 256 - rest) / s.slot_stride);
+  if (s.S < R + 2) return fail(c, GPE_ERR_INVALID, "pair kernel ring does not fit");
+  s.pt_ring = 256 + (unsigned)s.S * s.slot_stride;
+  s.u_ring = s.pt_ring + PT_SLOTS * s.pt_stride;
+  s.d_ring = s.u_ring + U_SLOTS * s.u_stride;
+  s.smem = s.d_ring + d_bytes;
+  s.threads_y = pair_warps<T>(R, s.TY) + 1;
+  CU_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem));
+  CU_CHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s.occ, fn, 32 * s.threads_y, s.smem));
+  if (s.occ < 1) return fail(c, GPE_ERR_INVALID, "pair kernel cannot be resident");
+  *out = s;
+  return GPE_OK;
+}
+
+// z-planes per item of a single-run launch on `slots` resident CTAs: the
+// count of chunks that minimises (rounds of items) x (planes an item marches,
+// its 3R lead-in planes included).  (Equal shares of all tile planes, cut
+// where they fall, would keep all SMs busy where chunks leave some idle, but
+// their CTAs work at unrelated heights and find no neighbour's halo in L2:
+// 336 against 283 us a step at 256^3, complex64 order 2.)
+int pair_zchunk(int nz, long ntiles, long slots, int R) {
+  int zc = nz;
+  double best = 1e300;
+  for (int n = 1; n <= std::min(nz, 256); n++) {
+    const int z = (nz + n - 1) / n;
+    const long nch = (nz + z - 1) / z;
+    const double cost = (double)((ntiles * nch + slots - 1) / slots) * (double)(z + 3 * R + 1);
+    if (cost < best - 1e-9) {
+      best = cost;
+      zc = z;
+    }
+  }
+  return zc;
+}
+
+template <typename T>
+int pair_run(gpe_ctx* c, const PairSpec& sp, int R, int TY, const RhsForm& f, RunDesc<T, T>* rd) {
+  memset(rd, 0, sizeof(*rd));
+  int rc = get_map(c, sp.s, 2, TY, R, &rd->maps.halo);
+  if (!rc && sp.base >= 0) rc = get_map(c, sp.base, 3, TY, R, &rd->maps.halo2);
+  if (!rc && sp.acc >= 0) rc = get_map(c, sp.acc, 1, TY, R, &rd->maps.pt[0]);
+  if (!rc && sp.comp >= 0) rc = get_map(c, sp.comp, 1, TY, R, &rd->maps.pt[1]);
+  if (rc) return rc;
+  rd->stencil = static_cast<const T*>(c->fld[sp.s]);
+  rd->out[0] = static_cast<T*>(c->fld[sp.out0]);
+  rd->out[1] = sp.out1 >= 0 ? static_cast<T*>(c->fld[sp.out1]) : nullptr;
+  rd->ntx = (c->nx + TX - 1) / TX;
+  rd->nty = (c->ny + TY - 1) / TY;
+  fill_geometry<T, T>(c, R, f, rd);
+  return GPE_OK;
+}
+
+template <typename T>
+void pair_common(const PairSpec& sp, const PairShape& sh, bool fold, PairParams<T>* p) {
+  const cd I(0.0, 1.0);
+  p->TY = sh.TY; p->stages = sh.S;
+  p->s_bytes = sh.s_bytes; p->base_bytes = sh.base_bytes; p->pt_bytes = sh.pt_bytes;
+  p->base_off = sh.base_off; p->comp_off = sh.comp_off;
+  p->slot_stride = sh.slot_stride; p->pt_stride = sh.pt_stride; p->u_stride = sh.u_stride;
+  p->pt_ring = sh.pt_ring; p->u_ring = sh.u_ring; p->d_ring = sh.d_ring;
+  for (int k = 0; k < 2; k++) {
+    const cd a = fold ? I * sp.a[k] : sp.a[k];
+    p->a_r[k] = (T)a.real();
+    p->a_i[k] = (T)a.imag();
+  }
+}
+
+template <typename T>
+int launch_pair_t(gpe_ctx* c, const PairSpec& sp) {
+  const int R = c->prm.order / 2;
+  RhsForm f = rhs_form(c);
+  const int form = form_of(f);
+  KernelFn fn = pair_kernel_fn(c->es, R, sp.kind, sp.comp >= 0, form, false);
+  if (!fn) return fail(c, GPE_ERR_INVALID, "no pair kernel for this step");
+  auto hit = c->pair_shapes.find(fn);
+  if (hit == c->pair_shapes.end()) {
+    PairShape sh;
+    const int rc = pair_shape<T>(c, fn, R, sp, c->prm.tile_y, &sh);
+    if (rc) return rc;
+    hit = c->pair_shapes.emplace(fn, sh).first;
+  }
+  const PairShape& sh = hit->second;
+  PairParams<T> p;
+  memset(&p, 0, sizeof(p));
+  int rc = pair_run<T>(c, sp, R, sh.TY, f, &p.run);
+  if (rc) return rc;
+  pair_common<T>(sp, sh, form != FORM_FULL, &p);
+  const long slots = (long)sh.occ * c->num_sms;
+  const long ntiles = (long)p.run.ntx * p.run.nty;
+  p.run.zchunk = c->prm.zchunk > 0 ? c->prm.zchunk : pair_zchunk(c->nz, ntiles, slots, R);
+  p.run.nchunks = (c->nz + p.run.zchunk - 1) / p.run.zchunk;
+  p.nitems = (int)(ntiles * p.run.nchunks);
+  if ((size_t)p.nitems > c->partials_cap)
+    return fail(c, GPE_ERR_INVALID, "partials buffer too small");
+  p.partials = c->d_partials;
+  p.status = c->d_status;
+  p.wait_limit_ns = c->wait_limit_ns;
+  p.stall_plane = c->stall_plane;
+  void* args[] = {&p};
+  const unsigned grid = (unsigned)std::min<long>(p.nitems, slots);
+  CU_CHECK(c, cudaLaunchKernel(fn, dim3(grid), dim3(32, (unsigned)sh.threads_y), args, sh.smem,
+                               c->stream));
+  c->launches++;
+  c->last_nblk = p.nitems;
+  return GPE_OK;
+}
+
+// Blocks of `warps` warps for the ghost rows of a field (fill_ghost_rows).
+int ghost_blocks(const gpe_ctx* c, int warps) {
+  const int depth = c->prm.order;
+  const int tasks = 2 * depth * (c->ny + 2 * depth + c->nz) + c->ny * c->nz / 4;
+  return std::min(tasks / warps + 1, 148 * 64 / warps);
+}
+
+// Ghosts of a field 2R deep, edges included.
+int fill_ghosts(gpe_ctx* c, int field) {
+  const Geom g = geom(c);
+  const int depth = c->prm.order, nb = ghost_blocks(c, 8);
+  if (c->es == 8)
+    fill_ghosts_kernel<float><<<nb, 256, 0, c->stream>>>((float*)c->fld[field], g, depth);
+  else
+    fill_ghosts_kernel<double><<<nb, 256, 0, c->stream>>>((double*)c->fld[field], g, depth);
+  CU_CHECK(c, cudaGetLastError());
+  c->launches++;
+  return GPE_OK;
+}
+
+// psi's ghosts for a pair, where the last writer filled fewer.
+int widen_ghosts(gpe_ctx* c) {
+  if (c->wide) return GPE_OK;
+  c->wide = true;
+  return fill_ghosts(c, c->psi_id);
+}
+
+int launch_pair(gpe_ctx* c, const PairSpec& sp) {
+  return c->es == 8 ? launch_pair_t<float>(c, sp) : launch_pair_t<double>(c, sp);
+}
+
+// The end of a step in pairs: psi's ghosts and the norm, one launch.
+int finish_pairs(gpe_ctx* c) {
+  const Geom g = geom(c);
+  const int depth = c->prm.order, nb = ghost_blocks(c, 32) + 1;
+  if (c->es == 8)
+    ghosts_norm_kernel<float><<<nb, 1024, 0, c->stream>>>(
+        (float*)c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk, cell_volume(c), c->d_scal,
+        c->step_series);
+  else
+    ghosts_norm_kernel<double><<<nb, 1024, 0, c->stream>>>(
+        (double*)c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk, cell_volume(c), c->d_scal,
+        c->step_series);
+  CU_CHECK(c, cudaGetLastError());
+  c->launches++;
+  return GPE_OK;
+}
+
+// rk4 as two pairs: u3 into F_UB, acc into psi's spare buffer, over which
+// psi' is then written (acc is read at the same site only).
+void rk4_pairs(const gpe_ctx* c, cd dt, PairSpec sp[2]) {
+  sp[0] = PairSpec();
+  sp[0].kind = PAIR_RK4_A;
+  sp[0].s = c->psi_id;
+  sp[0].out0 = F_UB;
+  sp[0].out1 = c->alt_id;
+  sp[0].a[0] = sp[0].a[1] = 0.5 * dt;
+  sp[0].family = GPE_FAM_STAGE_FIRST;
+  sp[1] = PairSpec();
+  sp[1].kind = PAIR_RK4_B;
+  sp[1].s = F_UB;
+  sp[1].base = c->psi_id;
+  sp[1].acc = c->alt_id;
+  sp[1].out0 = c->alt_id;
+  sp[1].a[0] = dt;
+  sp[1].a[1] = dt / 6.0;
+  if (c->prm.kahan) sp[1].comp = sp[1].out1 = c->c_id;
+  sp[1].family = GPE_FAM_STAGE_LAST;
+}
+
+int step_rk4_pairs(gpe_ctx* c, cd dt) {
+  PairSpec sp[2];
+  rk4_pairs(c, dt, sp);
+  int rc = widen_ghosts(c);
+  if (!rc) rc = launch_pair(c, sp[0]);
+  if (!rc) rc = fill_ghosts(c, sp[0].out0);
+  if (!rc) rc = launch_pair(c, sp[1]);
+  if (rc) return rc;
+  swap_psi(c);
+  return finish_pairs(c);
+}
+
+int step_rk2_pair(gpe_ctx* c, cd dt) {
+  PairSpec sp;
+  sp.kind = PAIR_RK2;
+  sp.s = c->psi_id;
+  sp.out0 = c->alt_id;
+  sp.a[0] = 0.5 * dt;
+  sp.a[1] = dt;
+  if (c->prm.kahan) sp.comp = sp.out1 = c->c_id;
+  sp.family = GPE_FAM_STAGE_LAST;
+  int rc = widen_ghosts(c);
+  if (!rc) rc = launch_pair(c, sp);
+  if (rc) return rc;
+  swap_psi(c);
+  return finish_pairs(c);
 }
 
 int step_rk2(gpe_ctx* c, cd dt) {
+  if (steps_in_pairs(c)) return step_rk2_pair(c, dt);
   StageSpec s1;
   s1.stencil = c->psi_id; s1.nout = 1; s1.out[0] = F_UA; s1.ghost_mask = 1;
   s1.alpha[0] = 1.0; s1.a[0] = 0.5 * dt; s1.family = GPE_FAM_STAGE_FIRST;
@@ -1102,7 +1403,7 @@ int step_rk2(gpe_ctx* c, cd dt) {
   }
   rc = launch_stage(c, s2);
   if (rc) return rc;
-  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, false);
+  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, true);
 }
 
 // The four classic RK4 stages (src/solve.f90:109-154) as stage recipes, in
@@ -1158,6 +1459,7 @@ void rk4_specs(const gpe_ctx* c, cd dt, StageSpec sp[4]) {
 }
 
 int step_rk4(gpe_ctx* c, cd dt) {
+  if (steps_in_pairs(c)) return step_rk4_pairs(c, dt);
   StageSpec sp[4];
   rk4_specs(c, dt, sp);
   for (int st = 0; st < 4; st++) {
@@ -1165,7 +1467,7 @@ int step_rk4(gpe_ctx* c, cd dt) {
     if (rc) return rc;
   }
   swap_psi(c);
-  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, false);
+  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, true);
 }
 
 // rkck (src/solve.f90:248-378) with the psi_scal / errmax reduction of rkqs
@@ -1248,7 +1550,7 @@ int attempt_rkck(gpe_ctx* c, cd dt, cd dt0, const double* dyn = nullptr, bool re
   if (!reduce) return GPE_OK;
   rc = finalize(c, c->last_nblk, 1, 1, 1.0 / RK_EPS, 3, false);
   if (rc) return rc;
-  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, false);
+  return finalize(c, c->last_nblk, 0, 0, cell_volume(c), 0, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -1536,37 +1838,22 @@ int build_tables(gpe_ctx* c) {
   const int zoff[3] = {0, 0, c->z_off};
   const std::vector<double>* crd[3] = {&c->x, &c->y, &c->z};
   const double om[3] = {p.omx, p.omy, p.omz};
-  size_t total = 0;
+  // per axis: Vf, Df (float) + Vd, Dd, W, X (double), each with GH entries
+  // before index 0 (and room past the end) for the ghost sites, which hold
+  // the entry of the site they are an image of
+  constexpr int LEAD = 8;
+  static_assert(LEAD >= GH, "lead-in holds the ghost entries");
+  size_t offs[3][6], off = 0;
   for (int a = 0; a < 3; a++) {
     c->tab_n[a] = (int)round_up((size_t)n[a], 64) + 64;
-    total += (size_t)c->tab_n[a];
+    for (int k = 0; k < 6; k++) {
+      offs[a][k] = off + LEAD * (k < 2 ? sizeof(float) : sizeof(double));
+      off += round_up((k < 2 ? sizeof(float) : sizeof(double)) * (size_t)(c->tab_n[a] + LEAD), 256);
+    }
   }
-  // per axis: Vf, Df (float) + Vd, Dd, W, X (double)
-  const size_t bytes = total * (2 * sizeof(float) + 4 * sizeof(double));
-  CU_CHECK(c, cudaMalloc(&c->d_tables, bytes));
-  c->device_bytes += (int64_t)bytes;
-  std::vector<unsigned char> h(bytes, 0);
-  size_t off = 0;
-  auto take = [&](size_t nbytes) {
-    size_t o = off;
-    off += round_up(nbytes, 256);
-    return o;
-  };
-  // recompute offsets with alignment
-  off = 0;
-  size_t offs[3][6];
-  for (int a = 0; a < 3; a++) {
-    offs[a][0] = take(sizeof(float) * c->tab_n[a]);
-    offs[a][1] = take(sizeof(float) * c->tab_n[a]);
-    for (int k = 2; k < 6; k++) offs[a][k] = take(sizeof(double) * c->tab_n[a]);
-  }
-  if (off > bytes) {
-    cudaFree(c->d_tables);
-    c->device_bytes -= (int64_t)bytes;
-    CU_CHECK(c, cudaMalloc(&c->d_tables, off));
-    c->device_bytes += (int64_t)off;
-    h.assign(off, 0);
-  }
+  CU_CHECK(c, cudaMalloc(&c->d_tables, off));
+  c->device_bytes += (int64_t)off;
+  std::vector<unsigned char> h(off, 0);
   for (int a = 0; a < 3; a++) {
     float* vf = reinterpret_cast<float*>(&h[offs[a][0]]);
     float* df = reinterpret_cast<float*>(&h[offs[a][1]]);
@@ -1586,6 +1873,12 @@ int build_tables(gpe_ctx* c) {
       vd[i] = v; vf[i] = (float)v;
       dd[i] = d; df[i] = (float)d;
       xx[i] = X[i];
+    }
+    for (int q = 1; q <= GH; q++) {
+      const int lo = -q, hi = N - 1 + q;
+      const int slo = p.bcs == 1 ? N - q : q, shi = p.bcs == 1 ? q - 1 : N - 1 - q;
+      vd[lo] = vd[slo]; vf[lo] = vf[slo]; dd[lo] = dd[slo]; df[lo] = df[slo]; xx[lo] = xx[slo];
+      vd[hi] = vd[shi]; vf[hi] = vf[shi]; dd[hi] = dd[shi]; df[hi] = df[shi]; xx[hi] = xx[shi];
     }
     // norm weights (src/variables.f90:713-823): x sums every term that
     // names an index, y and z take the last matching assignment.
@@ -1640,7 +1933,7 @@ int load_stage(gpe_ctx* c, int elem_bytes) {
   Launch L{};
   begin_timed(c, L, GPE_FAM_COPY, (int64_t)c->nint);
   const Geom g = geom(c);
-  const int nb = elementwise_blocks(c->nint);
+  const int nb = row_blocks((size_t)c->Ny * c->Nz);
   void* dst = c->fld[c->psi_id];
   if (c->es == 8) {
     if (elem_bytes == 8)
@@ -1664,6 +1957,7 @@ int load_stage(gpe_ctx* c, int elem_bytes) {
     CU_CHECK(c, cudaMemsetAsync(c->fld[c->c_id], 0, c->npad * (size_t)c->es,
                                 c->stream));
   c->norm_valid = false;
+  c->wide = true;
   // a slab-group member's z ghosts come from its neighbours, which may not
   // be loaded yet: the group refreshes them before its next step
   if (c->group) c->ghosts_dirty = true;
@@ -1684,7 +1978,7 @@ int pack_stage(gpe_ctx* c, int field, int elem_bytes) {
   Launch L{};
   begin_timed(c, L, GPE_FAM_COPY, (int64_t)c->nint);
   const Geom g = geom(c);
-  const int nb = elementwise_blocks(c->nint);
+  const int nb = row_blocks((size_t)c->ny * c->nz);
   const void* src = c->fld[field];
   if (c->es == 8) {
     if (elem_bytes == 8)
@@ -1775,7 +2069,7 @@ int gpe_internal_restore_norm(gpe_ctx* c) {
                                                    c->d_partials);
   CU_CHECK(c, cudaGetLastError());
   finalize_kernel<<<1, 1024, 0, c->stream>>>(c->d_partials, nb, 0, 0, cell_volume(c),
-                                              c->d_scal + 8, nullptr, c->d_counter);
+                                              c->d_scal + 8, nullptr);
   const size_t n = c->npad * 2;
   const int sb = elementwise_blocks(n);
   if (c->es == 8)
@@ -1803,6 +2097,9 @@ struct gpe_batch {
   gpe_batch_opts opts;
   int es = 8, R = 1;
   int form = FORM_PLAIN;  // the highest right-hand-side form among the members
+  // two stages per launch (pair_kernel.cuh); not for the full form, of which
+  // no batched pair is built, or where a member keeps its increments apart
+  bool pairs = false;
   int TY = 8;
   WorkItem* d_items = nullptr;
   int* d_item_run = nullptr;
@@ -1819,9 +2116,11 @@ struct gpe_batch {
   // (rk4_specs), so [0] steps from the members' current psi and [1] from the
   // buffer the step after it starts from; steps alternate between them.
   void* d_rundesc[2][4] = {};
+  GhostRun* d_ghosts[2][2] = {};  // pairs: the fields whose ghosts follow each launch
   struct Stage {
     KernelFn fn = nullptr;
-    LaunchShape sh{};
+    int warps = 0;
+    size_t smem = 0;
     int grid = 0;
     std::vector<unsigned char> params;  // StageParams bytes
   } st[2][4];
@@ -1901,7 +2200,56 @@ int batch_prepare_par(gpe_batch* b, cd dt, int par) {
     p.partials = b->d_partials;
     p.status = b->d_status;
     b->st[par][s].fn = fn;
-    b->st[par][s].sh = sh;
+    b->st[par][s].warps = sh.TY / sh.rows + 1;
+    b->st[par][s].smem = sh.smem;
+    b->st[par][s].grid = grid;
+    b->st[par][s].params.assign(reinterpret_cast<unsigned char*>(&p),
+                                reinterpret_cast<unsigned char*>(&p) + sizeof(p));
+  }
+  return GPE_OK;
+}
+
+// The same for the two pairs.
+template <typename T>
+int batch_prepare_pairs(gpe_batch* b, cd dt, int par) {
+  for (int s = 0; s < 2; s++) {
+    PairSpec sp0[2];
+    rk4_pairs(b->runs[0], dt, sp0);
+    KernelFn fn = pair_kernel_fn(b->es, b->R, sp0[s].kind, sp0[s].comp >= 0, b->form, true);
+    if (!fn) return bfail(b, GPE_ERR_INVALID, "no batched pair kernel");
+    PairShape sh;
+    int rc = pair_shape<T>(b->runs[0], fn, b->R, sp0[s], b->TY, &sh);
+    if (rc) return bfail(b, rc, b->runs[0]->err);
+    const int per_sm = b->opts.ctas_per_sm > 0 ? std::min(b->opts.ctas_per_sm, sh.occ) : sh.occ;
+    const int grid = std::min(b->nitems, per_sm * b->runs[0]->num_sms);
+    std::vector<RunDesc<T, T>> rds(b->runs.size());
+    std::vector<GhostRun> gr(b->runs.size());
+    for (size_t r = 0; r < b->runs.size(); r++) {
+      gpe_ctx* c = b->runs[r];
+      PairSpec spr[2];
+      rk4_pairs(c, dt, spr);
+      rc = pair_run<T>(c, spr[s], b->R, sh.TY, rhs_form(c), &rds[r]);
+      if (rc) return bfail(b, rc, c->err);
+      gr[r].field = c->fld[spr[s].out0];
+      gr[r].g = geom(c);
+    }
+    BCU(b, cudaMemcpy(b->d_ghosts[par][s], gr.data(), sizeof(GhostRun) * gr.size(),
+                      cudaMemcpyHostToDevice));
+    BCU(b, cudaMemcpy(b->d_rundesc[par][s], rds.data(), sizeof(RunDesc<T, T>) * rds.size(),
+                      cudaMemcpyHostToDevice));
+    PairParams<T> p;
+    memset(&p, 0, sizeof(p));
+    pair_common<T>(sp0[s], sh, true, &p);
+    p.runs = static_cast<const RunDesc<T, T>*>(b->d_rundesc[par][s]);
+    p.items = b->d_items;
+    p.nitems = b->nitems;
+    p.partials = b->d_partials;
+    p.status = b->d_status;
+    p.wait_limit_ns = WAIT_LIMIT_NS;
+    p.stall_plane = -1;
+    b->st[par][s].fn = fn;
+    b->st[par][s].warps = sh.threads_y;
+    b->st[par][s].smem = sh.smem;
     b->st[par][s].grid = grid;
     b->st[par][s].params.assign(reinterpret_cast<unsigned char*>(&p),
                                 reinterpret_cast<unsigned char*>(&p) + sizeof(p));
@@ -1913,12 +2261,19 @@ void batch_swap_members(gpe_batch* b) {
   for (auto* c : b->runs) std::swap(c->psi_id, c->alt_id);
 }
 
-template <typename TS, typename TC>
-int batch_prepare_t(gpe_batch* b, cd dt) {
-  int rc = batch_prepare_par<TS, TC>(b, dt, 0);
+int batch_prepare_form(gpe_batch* b, cd dt, int par) {
+  if (b->pairs)
+    return b->es == 8 ? batch_prepare_pairs<float>(b, dt, par)
+                      : batch_prepare_pairs<double>(b, dt, par);
+  if (b->es == 8) return batch_prepare_par<float, float>(b, dt, par);
+  return batch_prepare_par<double, double>(b, dt, par);
+}
+
+int batch_prepare(gpe_batch* b, cd dt) {
+  int rc = batch_prepare_form(b, dt, 0);
   if (rc) return rc;
   batch_swap_members(b);
-  rc = batch_prepare_par<TS, TC>(b, dt, 1);
+  rc = batch_prepare_form(b, dt, 1);
   batch_swap_members(b);
   if (rc) return rc;
   b->prepared_dt = dt;
@@ -1928,19 +2283,21 @@ int batch_prepare_t(gpe_batch* b, cd dt) {
   return GPE_OK;
 }
 
-int batch_prepare(gpe_batch* b, cd dt) {
-  if (b->es == 8) return batch_prepare_t<float, float>(b, dt);
-  return batch_prepare_t<double, double>(b, dt);
-}
-
-// One RK4 step of every member: 4 persistent stage launches, per-run norm
+// One RK4 step of every member: the persistent stage (or pair) launches, per-run norm
 // into d_norm and the series, step counter bump.
 int batch_enqueue_step(gpe_batch* b, int par) {
-  for (int s = 0; s < 4; s++) {
+  for (int s = 0; s < (b->pairs ? 2 : 4); s++) {
     auto& S = b->st[par][s];
     void* args[] = {S.params.data()};
-    BCU(b, cudaLaunchKernel(S.fn, dim3((unsigned)S.grid), dim3(32, (unsigned)(S.sh.TY / S.sh.rows) + 1),
-                            args, S.sh.smem, b->stream));
+    BCU(b, cudaLaunchKernel(S.fn, dim3((unsigned)S.grid), dim3(32, (unsigned)S.warps), args, S.smem,
+                            b->stream));
+    if (b->pairs) {
+      const dim3 grid(16, (unsigned)b->runs.size());
+      if (b->es == 8)
+        batch_ghosts_kernel<float><<<grid, 256, 0, b->stream>>>(b->d_ghosts[par][s], 2 * b->R);
+      else
+        batch_ghosts_kernel<double><<<grid, 256, 0, b->stream>>>(b->d_ghosts[par][s], 2 * b->R);
+    }
   }
   batch_finalize_kernel<<<(unsigned)b->runs.size(), 256, 0, b->stream>>>(
       b->d_partials, b->d_item_run, b->nitems, b->d_scale, b->d_norm, b->d_series,
@@ -1956,12 +2313,17 @@ const char* bad_opts(const gpe_batch_opts& o) {
   return nullptr;
 }
 
+// Rows per tile: 16 for complex64 pairs (pair_shape), else 8.
+int batch_tile_y(const gpe_batch* b) {
+  return b->opts.tile_y > 0 ? b->opts.tile_y : b->pairs && b->es == 8 ? PairTile<float>::TY_MAX : 8;
+}
+
 // The work list of b->opts: every member's (tile, z-range) items, sorted by
 // the sites they touch (warm-up planes included), largest first, so the
 // persistent CTAs' round-robin walk ends on the small items.
 int batch_plan(gpe_batch* b) {
   const gpe_batch_opts& o = b->opts;
-  b->TY = o.tile_y > 0 ? o.tile_y : 8;
+  b->TY = batch_tile_y(b);
   std::vector<WorkItem> items;
   std::vector<long> work;
   for (int r = 0; r < (int)b->runs.size(); r++) {
@@ -1973,7 +2335,7 @@ int batch_plan(gpe_batch* b) {
         const int tx = t % ntx, tyy = t / ntx;
         const int z1 = std::min(z0 + zc, c->nz);
         items.push_back(WorkItem{r, t, z0, z1});
-        work.push_back((long)(z1 - z0 + 2 * b->R) * std::min(TX, c->nx - tx * TX) *
+        work.push_back((long)(z1 - z0 + (b->pairs ? 3 : 2) * b->R) * std::min(TX, c->nx - tx * TX) *
                        std::min(b->TY, c->ny - tyy * b->TY));
       }
   }
@@ -2030,6 +2392,7 @@ void batch_flip(gpe_batch* b) {
   for (int s = 0; s < 4; s++) {
     std::swap(b->st[0][s], b->st[1][s]);
     std::swap(b->d_rundesc[0][s], b->d_rundesc[1][s]);
+    if (s < 2) std::swap(b->d_ghosts[0][s], b->d_ghosts[1][s]);
   }
   std::swap(b->graph[0], b->graph[1]);
   std::swap(b->exec[0], b->exec[1]);
@@ -2113,9 +2476,9 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
     return bail(GPE_ERR_CUDA);
   }
   c->nx = p.nx; c->ny = p.ny; c->nz = p.nz;
-  c->Nx = (int)round_up((size_t)p.nx + 4, 4);
-  c->Ny = p.ny + 4;
-  c->Nz = p.nz + 4;
+  c->Nx = (int)round_up((size_t)p.nx + 2 * GH, 4);
+  c->Ny = p.ny + 2 * GH;
+  c->Nz = p.nz + 2 * GH;
   c->npad = (size_t)c->Nx * c->Ny * c->Nz;
   c->nint = (size_t)p.nx * p.ny * p.nz;
   c->es = p.precision;
@@ -2156,7 +2519,6 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
   c->partials_cap = std::max<size_t>(ntiles_max * (size_t)p.nz, 148 * 16);
   if (cudaMalloc(&c->d_partials, 2 * sizeof(double) * c->partials_cap) != cudaSuccess ||
       cudaMalloc(&c->d_scal, 16 * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c->d_counter, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&c->d_stage, c->nint * 16) != cudaSuccess) {
     cudaGetLastError();
@@ -2164,7 +2526,7 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
     return bail(GPE_ERR_OOM);
   }
   c->device_bytes += (int64_t)(2 * sizeof(double) * c->partials_cap +
-                               16 * sizeof(double) + 2 * sizeof(int) + c->nint * 16);
+                               16 * sizeof(double) + sizeof(int) + c->nint * 16);
   if (p.scheme == GPE_SCHEME_RK45) {
     if (cudaMalloc(&c->d_time, sizeof(DevTime)) != cudaSuccess) {
       cudaGetLastError();
@@ -2176,7 +2538,6 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
   }
   cudaMemset(c->d_scal, 0, 16 * sizeof(double));
   cudaMemset(c->d_status, 0, sizeof(int));
-  cudaMemset(c->d_counter, 0, sizeof(int));
   if (cudaDeviceSynchronize() != cudaSuccess) {
     c->err = "device synchronisation failed during create";
     return bail(GPE_ERR_CUDA);
@@ -2207,7 +2568,6 @@ void gpe_gpu_destroy(gpe_ctx* c) {
   if (c->d_partials) cudaFree(c->d_partials);
   if (c->d_scal) cudaFree(c->d_scal);
   if (c->d_series) cudaFree(c->d_series);
-  if (c->d_counter) cudaFree(c->d_counter);
   if (c->d_status) cudaFree(c->d_status);
   if (c->d_stage) cudaFree(c->d_stage);
   rk45_drop_graphs(c);
@@ -2286,7 +2646,7 @@ int gpe_gpu_get_site(gpe_ctx* c, int32_t i, int32_t j, int32_t k, double* re_im)
   if (!re_im) return fail(c, GPE_ERR_INVALID, "null output");
   if (i < 0 || i >= c->nx || j < 0 || j >= c->ny || k < 0 || k >= c->nz)
     return fail(c, GPE_ERR_INVALID, "site outside the grid");
-  const size_t q = ((size_t)(k + 2) * c->Ny + (size_t)(j + 2)) * c->Nx + (size_t)(i + 2);
+  const size_t q = ((size_t)(k + GH) * c->Ny + (size_t)(j + GH)) * c->Nx + (size_t)(i + GH);
   unsigned char buf[16];
   CU_CHECK(c, cudaMemcpyAsync(buf, static_cast<const unsigned char*>(c->fld[c->psi_id]) +
                                        q * (size_t)c->es,
@@ -2309,7 +2669,7 @@ int gpe_gpu_get_plane(gpe_ctx* c, int32_t k, void* out, int32_t elem_bytes) {
   rc = check_elem(c, elem_bytes, out);
   if (rc) return rc;
   if (k < 0 || k >= c->nz) return fail(c, GPE_ERR_INVALID, "plane outside the grid");
-  const size_t first = ((size_t)(k + 2) * c->Ny + 2) * c->Nx + 2;
+  const size_t first = ((size_t)(k + GH) * c->Ny + GH) * c->Nx + GH;
   const unsigned char* src = static_cast<const unsigned char*>(c->fld[c->psi_id]) +
                              first * (size_t)c->es;
   const size_t n = (size_t)c->nx * c->ny;
@@ -2420,13 +2780,17 @@ int gpe_gpu_advance(gpe_ctx* c, int64_t nsteps, gpe_time* tm, double* norms) {
     c->norm_valid = true;
     return GPE_OK;
   }
-  CU_CHECK(c, cudaMemsetAsync(c->d_counter, 0, sizeof(int), c->stream));
   for (int64_t s = 0; s < nsteps; s++) {
+    // the step's norm reduction writes the series too; a reduction that ends in
+    // an all-reduce (communicator) or on the rk45 control is copied there
+    const bool direct = !c->comm && c->prm.scheme != GPE_SCHEME_RK45;
+    c->step_series = direct ? c->d_series + s : nullptr;
     rc = do_step(c, tm, nullptr);
+    c->step_series = nullptr;
     if (rc) return rc;
-    // copy the fused norm into the per-step series
-    CU_CHECK(c, cudaMemcpyAsync(c->d_series + s, c->d_scal, sizeof(double),
-                                cudaMemcpyDeviceToDevice, c->stream));
+    if (!direct)
+      CU_CHECK(c, cudaMemcpyAsync(c->d_series + s, c->d_scal, sizeof(double),
+                                  cudaMemcpyDeviceToDevice, c->stream));
     tm->p += 1;
   }
   if (norms && nsteps > 0)
@@ -2672,6 +3036,7 @@ int gpe_gpu_set_slab(gpe_ctx* c, int32_t nz_global, int32_t z_offset) {
   }
   rc = build_tables(c);
   if (rc) return rc;
+  c->wide = false;
   c->norm_valid = false;
   return GPE_OK;
 }
@@ -2791,6 +3156,7 @@ int gpe_group_create(gpe_ctx* const* members, int32_t n, gpe_group** out) {
     c->exch_lo = periodic || r > 0;
     c->exch_hi = periodic || r < n - 1;
     c->ghosts_dirty = true;
+    c->wide = false;
     c->norm_valid = false;
     c->maps.clear();
     c->shapes.clear();
@@ -2811,6 +3177,7 @@ void gpe_group_destroy(gpe_group* g) {
     c->rank = 0;
     c->nranks = 1;
     c->exch_lo = c->exch_hi = false;
+    c->wide = false;
     c->maps.clear();
     c->shapes.clear();
     rk45_drop_graphs(c);
@@ -2952,7 +3319,6 @@ int gpe_batch_create(const gpe_params* prms, int32_t nruns, const gpe_batch_opts
   b->dev = p0.device;
   b->es = p0.precision;
   b->R = p0.order / 2;
-  b->TY = o.tile_y > 0 ? o.tile_y : 8;
   auto bail = [&](int rc) {
     g_last_create_error = b->err;
     gpe_batch_destroy(b);
@@ -2961,7 +3327,7 @@ int gpe_batch_create(const gpe_params* prms, int32_t nruns, const gpe_batch_opts
   for (int r = 0; r < nruns; r++) {
     gpe_ctx* c = nullptr;
     gpe_params pr = prms[r];
-    pr.tile_y = b->TY;
+    pr.tile_y = o.tile_y;
     const int rc = gpe_gpu_create(&pr, &c);
     if (rc) {
       b->err = std::string("member ") + std::to_string(r) + ": " + g_last_create_error;
@@ -2971,6 +3337,8 @@ int gpe_batch_create(const gpe_params* prms, int32_t nruns, const gpe_batch_opts
     b->form = std::max(b->form, form_of(rhs_form(c)));
     b->sites += (int64_t)c->nint;
   }
+  b->pairs = b->form != FORM_FULL;
+  for (auto* c : b->runs) b->pairs = b->pairs && !network_grid(c);
   if (cudaSetDevice(b->dev) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
     b->err = "stream creation failed";
@@ -2998,6 +3366,13 @@ int gpe_batch_create(const gpe_params* prms, int32_t nruns, const gpe_batch_opts
         b->err = "cudaMalloc of run descriptors failed";
         return bail(GPE_ERR_OOM);
       }
+  for (int k = 0; k < 2; k++)
+    for (int s = 0; s < 2; s++)
+      if (cudaMalloc(&b->d_ghosts[k][s], sizeof(GhostRun) * nruns) != cudaSuccess) {
+        cudaGetLastError();
+        b->err = "cudaMalloc of ghost descriptors failed";
+        return bail(GPE_ERR_OOM);
+      }
   cudaMemcpy(b->d_scale, scale.data(), sizeof(double) * nruns, cudaMemcpyHostToDevice);
   cudaMemset(b->d_counter, 0, sizeof(int));
   cudaMemset(b->d_status, 0, sizeof(int));
@@ -3018,6 +3393,9 @@ void gpe_batch_destroy(gpe_batch* b) {
   for (int k = 0; k < 2; k++)
     for (int s = 0; s < 4; s++)
       if (b->d_rundesc[k][s]) cudaFree(b->d_rundesc[k][s]);
+  for (int k = 0; k < 2; k++)
+    for (int s = 0; s < 2; s++)
+      if (b->d_ghosts[k][s]) cudaFree(b->d_ghosts[k][s]);
   if (b->d_items) cudaFree(b->d_items);
   if (b->d_item_run) cudaFree(b->d_item_run);
   if (b->d_partials) cudaFree(b->d_partials);
@@ -3064,6 +3442,11 @@ int gpe_batch_advance(gpe_batch* b, int64_t nsteps, double dt_re, double dt_im,
     const int rc = batch_prepare(b, dt);
     if (rc) return rc;
   }
+  if (b->pairs && nsteps > 0)
+    for (auto* c : b->runs) {
+      const int rc = widen_ghosts(c);
+      if (rc) return bfail(b, rc, c->err);
+    }
   // members' own kernels (state loads) must be done before the batch runs
   for (auto* c : b->runs) BCU(b, cudaStreamSynchronize(c->stream));
   BCU(b, cudaMemsetAsync(b->d_counter, 0, sizeof(int), b->stream));
@@ -3089,10 +3472,13 @@ int gpe_batch_advance(gpe_batch* b, int64_t nsteps, double dt_re, double dt_im,
       const int rc = batch_enqueue_step(b, par);
       if (rc) return rc;
     }
-    b->launches += 6;
+    b->launches += 6;  // 4 stages, or 2 pairs with their ghosts; finalize, counter
   }
   if (nsteps & 1) batch_flip(b);
-  for (auto* c : b->runs) c->norm_valid = false;
+  for (auto* c : b->runs) {
+    c->norm_valid = false;
+    if (!b->pairs && nsteps > 0) c->wide = false;
+  }
   if (norms && nsteps > 0) {
     // series is [run][cap]: copy the first nsteps of each run
     BCU(b, cudaMemcpy2DAsync(norms, sizeof(double) * nsteps, b->d_series,

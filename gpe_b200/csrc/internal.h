@@ -11,11 +11,12 @@
 
 namespace gpe {
 
-// The resident psi of a context: padded field (2 ghosts per side, pitches
-// Nx >= nx + 4, Ny = ny + 4), complex of es bytes.
+// The resident psi of a context: padded field (gh ghosts per side, pitches
+// Nx >= nx + 2 gh, Ny = ny + 2 gh), complex of es bytes.
 struct FieldView {
   void* psi;
   int nx, ny, nz, Nx, Ny;
+  int gh;
   int es;
   int bcs;
   int dev;

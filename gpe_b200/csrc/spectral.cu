@@ -134,9 +134,9 @@ int prepare(gpe_ctx* c, FieldView* v, Spectral** out) {
   if (!s->has_plan_psi) {
     // reads the interior of the padded field (row pitch Nx, plane pitch Nx Ny)
     int n[3] = {v->nz, v->ny, v->nx};
-    int inembed[3] = {v->nz + 4, v->Ny, v->Nx};
+    int inembed[3] = {v->nz + 2 * v->gh, v->Ny, v->Nx};
     int onembed[3] = {v->nz, v->ny, v->nx};
-    SP_FFT(c, g_fft.PlanMany(&s->plan_psi, 3, n, inembed, 1, (v->nz + 4) * v->Ny * v->Nx, onembed,
+    SP_FFT(c, g_fft.PlanMany(&s->plan_psi, 3, n, inembed, 1, (v->nz + 2 * v->gh) * v->Ny * v->Nx, onembed,
                              1, v->nz * v->ny * v->nx, v->es == 16 ? CUFFT_Z2Z : CUFFT_C2C, 1));
     s->has_plan_psi = true;
     SP_FFT(c, g_fft.SetStream(s->plan_psi, v->stream));
@@ -223,7 +223,7 @@ int launch_spectrum(gpe_ctx* c, Spectral* s, const FieldView& v, const SpecArgs&
 int backward_from_psi(gpe_ctx* c, Spectral* s, const FieldView& v) {
   TimedRegion t;
   gpe_internal_time_begin(c, &t, GPE_FAM_OTHER, (int64_t)v.nx * v.ny * v.nz);
-  const size_t origin = ((size_t)2 * v.Ny + 2) * v.Nx + 2;
+  const size_t origin = ((size_t)v.gh * v.Ny + v.gh) * v.Nx + v.gh;
   if (v.es == 16) {
     auto* in = static_cast<cufftDoubleComplex*>(v.psi) + origin;
     SP_FFT(c, g_fft.ExecZ2Z(s->plan_psi, in, static_cast<cufftDoubleComplex*>(v.stage),

@@ -47,12 +47,12 @@
 #include <type_traits>
 
 #include "device_utils.cuh"
+#include "rhs.cuh"
 #include "vec2.cuh"
 
 namespace gpe {
 
 constexpr int TX = 64;   // x sites per tile: one warp row, two per lane
-constexpr int GH = 2;    // ghost width of every stored field
 constexpr int MAXP = 6;  // maximum pointwise inputs of one stage
 
 enum : int {
@@ -62,9 +62,6 @@ enum : int {
   EPI_ENERGY = 8,  // no outputs; reduce E (slot 0) and H4 (slot 1)
   EPI_LAP = 16,    // K is the Laplacian itself
 };
-
-// Right-hand-side forms of a recipe (see the top of this file).
-enum : int { FORM_PLAIN = 0, FORM_TRAP = 1, FORM_FULL = 2 };
 
 // Rows of the tile each compute warp owns.  Two for the complex64 recipes
 // that stage two stencil fields and nothing else (rk4 stages 2 and 3, in
@@ -115,6 +112,7 @@ struct alignas(64) RunDesc {
   // plain: K = cL*L + (c0 + cn*|u|^2) u   (the factor i is folded into a[o])
   TC ar0, ard, ai, cL, c0, cV, cn, U;
   int use_diss, use_V, use_sphere, use_grad;
+  int acc_first;          // rk4's last stage: sum d2/3 + 2 d3/3 first
   const TC* tabV[3];      // per-axis trap terms, V = Vx[i]+Vy[j]+Vz[k]
   const TC* tabD[3];      // per-axis sponge terms (times diss_amp)
   const double* tabW[3];  // per-axis norm weights
@@ -263,10 +261,10 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
           const bool with_pt = (NP > 0) && (u >= R);
           mbar_arrive_expect_tx(&full[slot],
                                 NS * p.halo_box_bytes + (with_pt ? NP * p.pt_box_bytes : 0u));
-          tma_load_3d(st, &rd.maps.halo, &full[slot], W * tile_x * TX,
+          tma_load_3d(st, &rd.maps.halo, &full[slot], W * (tile_x * TX + GH - 2),
                       tile_y * TY + GH - R, w.z0 + u + GH);
           if (NS == 2)
-            tma_load_3d(st + p.halo_smem_bytes, &rd.maps.halo2, &full[slot], W * tile_x * TX,
+            tma_load_3d(st + p.halo_smem_bytes, &rd.maps.halo2, &full[slot], W * (tile_x * TX + GH - 2),
                         tile_y * TY + GH - R, w.z0 + u + GH);
           if (with_pt) {
 #pragma unroll
@@ -353,16 +351,17 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
   }
   const size_t Nx = (size_t)rd.Nx, NxNy = (size_t)rd.Nx * (size_t)rd.Ny;
   TS* const outp[2] = {rd.out[0], rd.out[1]};
-  const TC c0s = rd.c0, cns = rd.cn, cVs = rd.cV, ar0 = rd.ar0, ard = rd.ard, ais = rd.ai;
-  const TC Us = rd.U, gx1 = rd.gx1, gx2 = rd.gx2;
+  const TC c0s = rd.c0, cns = rd.cn, cVs = rd.cV, Us = rd.U;
+  const FullTerms<TC> ft = {rd.c0, rd.cV, rd.cn, rd.ar0, rd.ard, rd.ai, rd.gx1, rd.gx2};
   const int useV = rd.use_V, useD = rd.use_diss, useS = rd.use_sphere, useG = rd.use_grad;
   const TC* const tabVz = rd.tabV[2];
   const TC* const tabDz = rd.tabD[2];
   const double* const tabWz = rd.tabW[2];
   const double eg = rd.eg, emu = rd.emu;
-  const V cx1 = vsplat(rd.cx1), cx2 = vsplat(rd.cx2), cy1 = vsplat(rd.cy1),
-          cy2 = vsplat(rd.cy2), cz1 = vsplat(rd.cz1), cz2 = vsplat(rd.cz2),
-          c0l = vsplat(rd.c0lap), cLv = vsplat(rd.cL);
+  const bool accf = rd.acc_first != 0;
+  const LapCoef<V> lc = {vsplat(rd.cx1), vsplat(rd.cx2), vsplat(rd.cy1), vsplat(rd.cy2),
+                         vsplat(rd.cz1), vsplat(rd.cz2), vsplat(rd.c0lap)};
+  const V cLv = vsplat(rd.cL);
   double red0 = 0.0, red1 = 0.0;
 
   // Per-thread constants of this item, per row.
@@ -375,7 +374,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
   {
     int a, b;
     for (int e = 0; e < 2; e++) {
-      ghost_targets(i0 + e, nx, bcs, a, b);
+      ghost_targets(i0 + e, nx, bcs, 2, a, b);
       gxo[e][0] = (a != NO_GHOST) ? a - (i0 + e) : 0;
       gxo[e][1] = (b != NO_GHOST) ? b - (i0 + e) : 0;
     }
@@ -396,7 +395,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
         Wxy[rr][0] = rd.tabW[0][i0] * rd.tabW[1][j];
         Wxy[rr][1] = rd.tabW[0][i0 + 1] * rd.tabW[1][j];
       }
-      ghost_targets(j, ny, bcs, a, b);
+      ghost_targets(j, ny, bcs, 2, a, b);
       gyo[rr][0] = (a != NO_GHOST) ? (a - j) * rd.Nx : 0;
       gyo[rr][1] = (b != NO_GHOST) ? (b - j) * rd.Nx : 0;
       edge_xy[rr] = (gxo[0][0] | gxo[0][1] | gxo[1][0] | gxo[1][1] | gyo[rr][0] | gyo[rr][1]) != 0;
@@ -489,7 +488,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
         gzo[0] = gzo[1] = 0;
         if (near_edge(z, nz)) {
           int a, b;
-          ghost_targets(z, nz, bcs, a, b);
+          ghost_targets(z, nz, bcs, 2, a, b);
           if (a != NO_GHOST && !((a < 0) ? zg_lo : zg_hi)) a = NO_GHOST;
           if (b != NO_GHOST && !((b < 0) ? zg_lo : zg_hi)) b = NO_GHOST;
           gzo[0] = (a != NO_GHOST) ? (long)(a - z) * (long)NxNy : 0;
@@ -528,18 +527,22 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
 #pragma unroll
         for (int e = 0; e < 2; e++) {
           const CPair<TC>& ctr = zq(rr, 0);
-          const V f0 = e ? ctr.b : ctr.a;
-          const V xm1 = e ? ctr.a : xa.b, xp1 = e ? xc.a : ctr.b;
-          const V xm2 = e ? xa.b : xa.a, xp2 = e ? xc.b : xc.a;
-          V L = vmul(cx1, vadd(xp1, xm1));
-          L = vfma(cy1, vadd(e ? yp1.b : yp1.a, e ? ym1.b : ym1.a), L);
-          L = vfma(cz1, vadd(e ? zq(rr, 1).b : zq(rr, 1).a, e ? zq(rr, -1).b : zq(rr, -1).a), L);
-          if (R == 2) {
-            L = vfma(cx2, vadd(xp2, xm2), L);
-            L = vfma(cy2, vadd(e ? yp2.b : yp2.a, e ? ym2.b : ym2.a), L);
-            L = vfma(cz2, vadd(e ? zq(rr, 2).b : zq(rr, 2).a, e ? zq(rr, -2).b : zq(rr, -2).a), L);
-          }
-          L = vfma(c0l, f0, L);
+          Star<V> st;
+          st.f0 = e ? ctr.b : ctr.a;
+          st.xm1 = e ? ctr.a : xa.b;
+          st.xp1 = e ? xc.a : ctr.b;
+          st.xm2 = e ? xa.b : xa.a;
+          st.xp2 = e ? xc.b : xc.a;
+          st.ym1 = e ? ym1.b : ym1.a;
+          st.yp1 = e ? yp1.b : yp1.a;
+          st.zm1 = e ? zq(rr, -1).b : zq(rr, -1).a;
+          st.zp1 = e ? zq(rr, 1).b : zq(rr, 1).a;
+          st.ym2 = e ? ym2.b : ym2.a;
+          st.yp2 = e ? yp2.b : yp2.a;
+          st.zm2 = R == 2 ? (e ? zq(rr, -2).b : zq(rr, -2).a) : st.zm1;
+          st.zp2 = R == 2 ? (e ? zq(rr, 2).b : zq(rr, 2).a) : st.zp1;
+          const V f0 = st.f0;
+          const V L = star_laplacian<R>(st, lc);
           const bool ok = e ? ok1[rr] : ok0[rr];
 
           if (EPI & EPI_ENERGY) {
@@ -555,27 +558,16 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
             continue;
           }
 
-          const TC a2 = fma(f0.y, f0.y, f0.x * f0.x);
           V Kv;
           if (EPI & EPI_LAP) {
             Kv = L;
           } else if (!FULL) {
-            const TC s = TRAP ? fma(cns, a2, fma(cVs, Vxy[rr][e] + Vz, c0s)) : fma(cns, a2, c0s);
-            Kv = vfma(vsplat(s), f0, vmul(cLv, L));
+            Kv = rhs_plain<TRAP>(L, f0, TRAP ? Vxy[rr][e] + Vz : TC(0), c0s, cVs, cns, cLv);
           } else {
-            const TC Vs = useV ? Vxy[rr][e] + Vz : TC(0);
-            const TC s = c0s + cVs * Vs + cns * a2;
-            const V B = vfma(vsplat(s), f0, vmul(cLv, L));
-            const TC arr = useD ? ar0 + ard * (Dxy[rr][e] + Dz) : ar0;
-            Kv = vfma(vsplat(arr), B, vmul(vpair(-ais, ais), vswap(B)));
-            if (useG) {
-              V gx = vmul(vsplat(gx1), vfma(xm1, mone, xp1));
-              if (R == 2) gx = vfma(vsplat(gx2), vfma(xm2, mone, xp2), gx);
-              Kv = vfma(vsplat(Us), gx, Kv);
-            }
+            Kv = rhs_full<R>(st, L, cLv, ft, useV ? Vxy[rr][e] + Vz : TC(0), useD != 0,
+                             Dxy[rr][e] + Dz, useG != 0, Us);
             if (useS) {
-              const double X = rd.tabX[0][i0 + e], Y = rd.tabX[1][j0 + rr], Z = rd.tabX[2][z];
-              const TC m = (TC)(0.5 * (1.0 + tanh(sqrt(X * X + Y * Y + Z * Z) - 10.0 - 2.0)));
+              const TC m = (TC)sphere_mask(rd.tabX[0][i0 + e], rd.tabX[1][j0 + rr], rd.tabX[2][z]);
               Kv = vmul(vsplat(m), Kv);
             }
           }
@@ -586,9 +578,17 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
             // smallest terms first: a (x) K, field 1, pointwise, field 0
             V v = vfma(ar[o], Kv, vmul(aix[o], Ks));
             if (NS == 2 && (AMASK & (4 << o))) v = vfma(alv2[o], e ? sc1.b : sc1.a, v);
+            if (NS == 2 && (BMASK & 3) == 3 && accf) {
+              // rk4's last stage: the two increments among themselves first,
+              // the sum pair_kernel.cuh stores for this stage
+              const V acc = vfma(bev[o][NP > 1 ? 1 : 0], e ? P[NP > 1 ? 1 : 0].b : P[NP > 1 ? 1 : 0].a,
+                                 vmul(bev[o][0], e ? P[0].b : P[0].a));
+              v = vadd(v, acc);
+            } else {
 #pragma unroll
-            for (int qq = 0; qq < NP; qq++)
-              if (BMASK & (1 << (o * 8 + qq))) v = vfma(bev[o][qq], e ? P[qq].b : P[qq].a, v);
+              for (int qq = 0; qq < NP; qq++)
+                if (BMASK & (1 << (o * 8 + qq))) v = vfma(bev[o][qq], e ? P[qq].b : P[qq].a, v);
+            }
             if (AMASK & (1 << o)) v = vfma(alv[o], NS == 2 ? (e ? sc0.b : sc0.a) : f0, v);
             res[o][e] = v;
           }

@@ -30,11 +30,12 @@ __device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) {
 __device__ __forceinline__ float2 vsplat(float s) { return make_float2(s, s); }
 __device__ __forceinline__ float2 vpair(float a, float b) { return make_float2(a, b); }
 
+// (intrinsics: a sum of a product is only ever fused where vfma says so)
 __device__ __forceinline__ double2 vadd(double2 a, double2 b) {
-  return make_double2(a.x + b.x, a.y + b.y);
+  return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
 }
 __device__ __forceinline__ double2 vmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x, a.y * b.y);
+  return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
 }
 __device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) {
   return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
@@ -48,6 +49,14 @@ __device__ __forceinline__ V vswap(V a) {
   V r;
   r.x = a.y;
   r.y = a.x;
+  return r;
+}
+
+template <typename V>
+__device__ __forceinline__ V vsel(bool c, V a, V b) {
+  V r;
+  r.x = c ? a.x : b.x;
+  r.y = c ? a.y : b.y;
   return r;
 }
 
@@ -100,8 +109,7 @@ __device__ __forceinline__ typename VT<TS>::T cvt_v(V a) {
 
 template <typename TS, typename V>
 __device__ __forceinline__ void st_c1(TS* p, V a) {
-  p[0] = (TS)a.x;
-  p[1] = (TS)a.y;
+  *reinterpret_cast<typename VT<TS>::T*>(p) = cvt_v<TS>(a);
 }
 
 }  // namespace gpe

@@ -55,7 +55,7 @@ int run(gpe_ctx* c, const FieldView& v, const void* field, bool dense, double* l
   p.nz = v.nz;
   p.Nx = dense ? v.nx : v.Nx;
   p.Ny = dense ? v.ny : v.Ny;
-  p.ghost = dense ? 0 : 2;
+  p.ghost = dense ? 0 : v.gh;
   p.cx = v.nx - 2;
   const long long rows = (long long)(v.ny - 2) * (v.nz - 2);
   p.ncell = rows * p.cx;
@@ -118,6 +118,7 @@ int run_zeros(gpe_ctx* c, const FieldView& v, int64_t* counts, double* points, i
   p.nz = v.nz;
   p.Nx = v.Nx;
   p.Ny = v.Ny;
+  p.ghost = v.gh;
   p.cx = v.nx - 2;
   const long long rows = (long long)(v.ny - 2) * (v.nz - 2);
   p.ncell = rows * p.cx;

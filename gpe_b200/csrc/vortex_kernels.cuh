@@ -218,7 +218,7 @@ __device__ __forceinline__ double segment(const Pt& p1, const Pt& p2) {
 struct LineArgs {
   const void* psi;        // the resident padded field, or a dense interior array
   int nx, ny, nz, Nx, Ny;
-  int ghost;              // 2 for the padded field, 0 for a dense array
+  int ghost;              // ghost layers of the padded field, 0 for a dense array
   int cx;               // cells per row, nx - 2
   long long ncell;      // (nx-2)(ny-2)(nz-2)
   long long per_block;  // cells per block (whole rows)
@@ -595,6 +595,7 @@ constexpr int Z_SECTIONS = 12;
 struct ZeroArgs {
   const void* psi;
   int nx, ny, nz, Nx, Ny;
+  int ghost;              // ghost layers of the padded field
   int cx;
   long long ncell, per_block;
   const double* x;  // grid coordinates (src/ic.f90:53-66)
@@ -620,8 +621,8 @@ __device__ __forceinline__ void load_zero_corners(const ZeroArgs& p, long long c
             dk[7] = {0, 0, 0, 1, 0, 1, 1};
 #pragma unroll
   for (int q = 0; q < 7; q++) {
-    const size_t at = ((size_t)(k + dk[q] + 2) * p.Ny + (size_t)(j + dj[q] + 2)) * p.Nx +
-                      (size_t)(i + di[q] + 2);
+    const size_t at = ((size_t)(k + dk[q] + p.ghost) * p.Ny + (size_t)(j + dj[q] + p.ghost)) * p.Nx +
+                      (size_t)(i + di[q] + p.ghost);
     const V w = f[at];
     re[q] = (double)w.x;
     im[q] = (double)w.y;

@@ -413,7 +413,9 @@ int64_t gpe_batch_launch_count(const gpe_batch* batch);
 int gpe_batch_info(const gpe_batch* batch, int64_t* sites, int32_t* nitems,
                    int32_t* grid, int32_t* tile_y);
 
-/* Per-kernel-family CUDA-event timing (off by default). */
+/* Per-kernel-family CUDA-event timing (off by default).  The families are
+ * single stages: while it is on, rk2 and rk4 step one stage per launch where
+ * they otherwise run two (the states are the same bit for bit). */
 int gpe_gpu_set_timing(gpe_ctx* ctx, int32_t on);
 int gpe_gpu_get_timing(gpe_ctx* ctx, gpe_timing* out);
 /* Number of kernels this context has launched (graph replays count their
