@@ -1,8 +1,8 @@
 """Launch-shape autotuner for batched ensembles.
 
 A batch's stage launches have three free knobs (include/gpe_gpu.h,
-gpe_batch_opts): the tile height (4 or 8 rows of 64 sites), the z-planes per
-work item, and the resident CTAs per SM.  Small grids want short items (more
+gpe_batch_opts): the tile height (the library's own, 4 or 8 rows of 64 sites),
+the z-planes per work item, and the resident CTAs per SM.  Small grids want short items (more
 items to balance 148 SMs), large grids want long ones (fewer warm-up planes
 per item: an item of zc planes reads zc + 2R planes of its stencil field).
 The best point depends on the ensemble's size mix, so it is measured: every
@@ -11,8 +11,8 @@ and timed with CUDA events on the batch's stream; the fastest wins.  Results
 are cached in a JSON file keyed by the ensemble's signature (member shapes,
 order, boundary, precision, device name), so a repeated scan pays once.
 
-The candidate set is small and explicit on purpose: 2 x 4 x 3 = 24 shapes,
-each timed over a few steps, costs well under a second for ensembles of tens
+The candidate set is small and explicit on purpose: 3 x 5 x 2 = 30 shapes (0 =
+the library's own choice, 16 rows for complex64 pairs of stages), each timed over a few steps, costs well under a second for ensembles of tens
 of millions of sites.
 """
 from __future__ import annotations
@@ -26,9 +26,9 @@ from typing import Iterable
 
 from .batch import BatchOpts, GpeBatch
 
-TILE_Y = (8, 4)
-ZCHUNK = (8, 16, 32, 64)
-CTAS_PER_SM = (0, 1, 2)
+TILE_Y = (0, 8, 4)
+ZCHUNK = (0, 8, 16, 32, 64)
+CTAS_PER_SM = (0, 2)
 
 
 def candidates() -> list[BatchOpts]:

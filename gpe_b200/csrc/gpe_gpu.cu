@@ -16,6 +16,7 @@
 #include <complex>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <string>
 #include <tuple>
@@ -2103,6 +2104,8 @@ struct gpe_batch {
   int TY = 8;
   WorkItem* d_items = nullptr;
   int* d_item_run = nullptr;
+  int* d_starts = nullptr;  // pairs: first item of every CTA's list, and the end
+  int lists = 0;
   int nitems = 0;
   double* d_partials = nullptr;
   double* d_scale = nullptr;
@@ -2116,6 +2119,7 @@ struct gpe_batch {
   // (rk4_specs), so [0] steps from the members' current psi and [1] from the
   // buffer the step after it starts from; steps alternate between them.
   void* d_rundesc[2][4] = {};
+  int ghost_blocks = 1;           // per member, for the largest
   GhostRun* d_ghosts[2][2] = {};  // pairs: the fields whose ghosts follow each launch
   struct Stage {
     KernelFn fn = nullptr;
@@ -2220,8 +2224,7 @@ int batch_prepare_pairs(gpe_batch* b, cd dt, int par) {
     PairShape sh;
     int rc = pair_shape<T>(b->runs[0], fn, b->R, sp0[s], b->TY, &sh);
     if (rc) return bfail(b, rc, b->runs[0]->err);
-    const int per_sm = b->opts.ctas_per_sm > 0 ? std::min(b->opts.ctas_per_sm, sh.occ) : sh.occ;
-    const int grid = std::min(b->nitems, per_sm * b->runs[0]->num_sms);
+    const int grid = b->lists;
     std::vector<RunDesc<T, T>> rds(b->runs.size());
     std::vector<GhostRun> gr(b->runs.size());
     for (size_t r = 0; r < b->runs.size(); r++) {
@@ -2242,6 +2245,7 @@ int batch_prepare_pairs(gpe_batch* b, cd dt, int par) {
     pair_common<T>(sp0[s], sh, true, &p);
     p.runs = static_cast<const RunDesc<T, T>*>(b->d_rundesc[par][s]);
     p.items = b->d_items;
+    p.starts = b->d_starts;
     p.nitems = b->nitems;
     p.partials = b->d_partials;
     p.status = b->d_status;
@@ -2292,7 +2296,7 @@ int batch_enqueue_step(gpe_batch* b, int par) {
     BCU(b, cudaLaunchKernel(S.fn, dim3((unsigned)S.grid), dim3(32, (unsigned)S.warps), args, S.smem,
                             b->stream));
     if (b->pairs) {
-      const dim3 grid(16, (unsigned)b->runs.size());
+      const dim3 grid((unsigned)b->ghost_blocks, (unsigned)b->runs.size());
       if (b->es == 8)
         batch_ghosts_kernel<float><<<grid, 256, 0, b->stream>>>(b->d_ghosts[par][s], 2 * b->R);
       else
@@ -2318,37 +2322,103 @@ int batch_tile_y(const gpe_batch* b) {
   return b->opts.tile_y > 0 ? b->opts.tile_y : b->pairs && b->es == 8 ? PairTile<float>::TY_MAX : 8;
 }
 
-// The work list of b->opts: every member's (tile, z-range) items, sorted by
-// the sites they touch (warm-up planes included), largest first, so the
-// persistent CTAs' round-robin walk ends on the small items.
-int batch_plan(gpe_batch* b) {
-  const gpe_batch_opts& o = b->opts;
-  b->TY = batch_tile_y(b);
-  std::vector<WorkItem> items;
-  std::vector<long> work;
+// Every member's (tile, z-range) items with zc planes each (a member's chunks
+// evened out when `even`).
+void batch_items(const gpe_batch* b, int zc, bool even, std::vector<WorkItem>* items) {
+  items->clear();
   for (int r = 0; r < (int)b->runs.size(); r++) {
     const gpe_ctx* c = b->runs[r];
     const int ntx = (c->nx + TX - 1) / TX, nty = (c->ny + b->TY - 1) / b->TY;
-    const int zc = o.zchunk > 0 ? std::min(o.zchunk, c->nz) : std::min(c->nz, 64);
-    for (int z0 = 0; z0 < c->nz; z0 += zc)
-      for (int t = 0; t < ntx * nty; t++) {
-        const int tx = t % ntx, tyy = t / ntx;
-        const int z1 = std::min(z0 + zc, c->nz);
-        items.push_back(WorkItem{r, t, z0, z1});
-        work.push_back((long)(z1 - z0 + (b->pairs ? 3 : 2) * b->R) * std::min(TX, c->nx - tx * TX) *
-                       std::min(b->TY, c->ny - tyy * b->TY));
+    int z = std::min(zc, c->nz);
+    if (even) {
+      const int n = std::max(1, (c->nz + zc / 2) / zc);
+      z = (c->nz + n - 1) / n;
+    }
+    for (int z0 = 0; z0 < c->nz; z0 += z)
+      for (int t = 0; t < ntx * nty; t++)
+        items->push_back(WorkItem{r, t, z0, std::min(z0 + z, c->nz)});
+  }
+}
+
+// Pairs: items dealt to `ctas` lists, longest first, each to the list that is
+// shortest so far (an item costs the planes it marches, whatever part of its
+// tile the member covers).  Returns the longest list.
+long batch_deal(const gpe_batch* b, const std::vector<WorkItem>& items, int ctas,
+                std::vector<std::vector<int>>* lists) {
+  std::vector<int> order(items.size());
+  for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    return items[x].z1 - items[x].z0 > items[y].z1 - items[y].z0;
+  });
+  std::vector<std::pair<long, int>> heap;  // (load, list), smallest first
+  for (int k = 0; k < ctas; k++) heap.push_back({0, k});
+  const auto later = std::greater<std::pair<long, int>>();
+  if (lists) lists->assign(ctas, {});
+  long longest = 0;
+  for (int i : order) {
+    std::pop_heap(heap.begin(), heap.end(), later);
+    auto& h = heap.back();
+    h.first += items[i].z1 - items[i].z0 + 3 * b->R + 1;
+    longest = std::max(longest, h.first);
+    if (lists) (*lists)[h.second].push_back(i);
+    std::push_heap(heap.begin(), heap.end(), later);
+  }
+  return longest;
+}
+
+// The work list of b->opts: one stage per launch, the members' items by the
+// sites they touch (warm-up planes included), largest first, walked round-robin
+// by the persistent CTAs; pairs, a list per CTA (batch_deal), with the chunk
+// length that makes the longest list shortest.
+int batch_plan(gpe_batch* b) {
+  const gpe_batch_opts& o = b->opts;
+  b->TY = batch_tile_y(b);
+  std::vector<WorkItem> items, sorted;
+  std::vector<int> starts;
+  if (b->pairs) {
+    const int per_sm = o.ctas_per_sm > 0 ? o.ctas_per_sm : b->TY <= 4 ? 2 : 1;
+    const int ctas = per_sm * b->runs[0]->num_sms;
+    int zc = o.zchunk;
+    if (zc <= 0) {
+      long best = -1;
+      for (int z : {8, 12, 16, 24, 32, 48, 64, 96, 128, 256}) {
+        batch_items(b, z, true, &items);
+        if (items.size() > 200000) continue;
+        const long cost = batch_deal(b, items, ctas, nullptr);
+        if (best < 0 || cost < best) {
+          best = cost;
+          zc = z;
+        }
       }
+      if (zc <= 0) zc = 256;
+    }
+    batch_items(b, zc, o.zchunk <= 0, &items);
+    std::vector<std::vector<int>> lists;
+    batch_deal(b, items, ctas, &lists);
+    for (const auto& l : lists) {
+      if (l.empty()) continue;
+      starts.push_back((int)sorted.size());
+      for (int i : l) sorted.push_back(items[i]);
+    }
+    starts.push_back((int)sorted.size());
+  } else {
+    batch_items(b, o.zchunk > 0 ? o.zchunk : 64, false, &items);
+    auto work = [&](const WorkItem& w) {
+      const gpe_ctx* c = b->runs[w.run];
+      const int ntx = (c->nx + TX - 1) / TX;
+      return (long)(w.z1 - w.z0 + 2 * b->R) * std::min(TX, c->nx - w.tile % ntx * TX) *
+             std::min(b->TY, c->ny - w.tile / ntx * b->TY);
+    };
+    sorted = items;
+    std::stable_sort(sorted.begin(), sorted.end(),
+                     [&](const WorkItem& x, const WorkItem& y) { return work(x) > work(y); });
+    starts.push_back(0);
   }
-  std::vector<size_t> order(items.size());
-  for (size_t i = 0; i < order.size(); i++) order[i] = i;
-  std::stable_sort(order.begin(), order.end(),
-                   [&](size_t x, size_t y) { return work[x] > work[y]; });
-  std::vector<WorkItem> sorted;
+  b->lists = (int)starts.size() - 1;
   std::vector<int> item_run;
-  for (size_t i : order) {
-    sorted.push_back(items[i]);
-    item_run.push_back(items[i].run);
-  }
+  for (const WorkItem& w : sorted) item_run.push_back(w.run);
+  if (b->d_starts) cudaFree(b->d_starts);
+  b->d_starts = nullptr;
   if (b->d_items) cudaFree(b->d_items);
   if (b->d_item_run) cudaFree(b->d_item_run);
   if (b->d_partials) cudaFree(b->d_partials);
@@ -2358,12 +2428,15 @@ int batch_plan(gpe_batch* b) {
   b->nitems = (int)sorted.size();
   if (cudaMalloc(&b->d_items, sizeof(WorkItem) * sorted.size()) != cudaSuccess ||
       cudaMalloc(&b->d_item_run, sizeof(int) * item_run.size()) != cudaSuccess ||
+      cudaMalloc(&b->d_starts, sizeof(int) * starts.size()) != cudaSuccess ||
       cudaMalloc(&b->d_partials, 2 * sizeof(double) * sorted.size()) != cudaSuccess) {
     cudaGetLastError();
     b->err = "cudaMalloc of the batch work list failed";
     return GPE_ERR_OOM;
   }
   if (cudaMemcpy(b->d_items, sorted.data(), sizeof(WorkItem) * sorted.size(),
+                 cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(b->d_starts, starts.data(), sizeof(int) * starts.size(),
                  cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(b->d_item_run, item_run.data(), sizeof(int) * item_run.size(),
                  cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -3338,7 +3411,10 @@ int gpe_batch_create(const gpe_params* prms, int32_t nruns, const gpe_batch_opts
     b->sites += (int64_t)c->nint;
   }
   b->pairs = b->form != FORM_FULL;
-  for (auto* c : b->runs) b->pairs = b->pairs && !network_grid(c);
+  for (auto* c : b->runs) {
+    b->pairs = b->pairs && !network_grid(c);
+    b->ghost_blocks = std::max(b->ghost_blocks, std::min(ghost_blocks(c, 16), 256));
+  }
   if (cudaSetDevice(b->dev) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
     b->err = "stream creation failed";
@@ -3398,6 +3474,7 @@ void gpe_batch_destroy(gpe_batch* b) {
       if (b->d_ghosts[k][s]) cudaFree(b->d_ghosts[k][s]);
   if (b->d_items) cudaFree(b->d_items);
   if (b->d_item_run) cudaFree(b->d_item_run);
+  if (b->d_starts) cudaFree(b->d_starts);
   if (b->d_partials) cudaFree(b->d_partials);
   if (b->d_scale) cudaFree(b->d_scale);
   if (b->d_norm) cudaFree(b->d_norm);

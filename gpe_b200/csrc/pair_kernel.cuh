@@ -98,7 +98,8 @@ struct PairParams {
   // (UW x (TY+2R), PAIR_RK4_B), pt[0] = acc (PAIR_RK4_B), pt[1] = compensation
   RunDesc<T, T> run;         // single-run launch
   const RunDesc<T, T>* runs;  // batched launch: per-run descriptors
-  const WorkItem* items;      // batched launch: the work list
+  const WorkItem* items;      // batched launch: the work list,
+  const int* starts;          // and where in it each CTA's items start
   int nitems;
   int TY, stages;
   // bytes a box delivers, offsets in a slot, strides of the three rings
@@ -143,6 +144,9 @@ __device__ __forceinline__ void pair_body(const PairParams<T>& p) {
     const int z0 = ch * p.run.zchunk;
     return WorkItem{0, it - ch * ntiles, z0, min(z0 + p.run.zchunk, p.run.nz)};
   };
+  const int it0 = BATCH ? p.starts[blockIdx.x] : (int)blockIdx.x;
+  const int it1 = BATCH ? p.starts[blockIdx.x + 1] : p.nitems;
+  const int its = BATCH ? 1 : (int)gridDim.x;
   auto run_of = [&](const WorkItem& w) -> const RD& {
     if (BATCH) return p.runs[w.run];
     return p.run;
@@ -182,7 +186,7 @@ __device__ __forceinline__ void pair_body(const PairParams<T>& p) {
       int slot = 0, issued = 0, pissued = 0;
       uint32_t cyc = 0;  // completed passes over the ring
       bool stop = false;
-      for (int it = blockIdx.x; it < p.nitems && !stop; it += gridDim.x) {
+      for (int it = it0; it < it1 && !stop; it += its) {
         const WorkItem w = item_of(it);
         const RD& rd = run_of(w);
         const int tile_x = w.tile % rd.ntx, tile_y = w.tile / rd.ntx;
@@ -301,7 +305,7 @@ __device__ __forceinline__ void pair_body(const PairParams<T>& p) {
     unsigned so = s_first, fo = s_first, uo = p.u_ring,
              zo = p.u_ring + (U_SLOTS - R) * p.u_stride;
 
-    for (int it = blockIdx.x; it < p.nitems; it += gridDim.x) {
+    for (int it = it0; it < it1; it += its) {
       const WorkItem w = item_of(it);
       const RD& rd = run_of(w);
       const int nx = rd.nx, ny = rd.ny, bcs = rd.bcs;
