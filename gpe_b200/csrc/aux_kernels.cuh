@@ -1,6 +1,8 @@
 // aux_kernels.cuh -- state transfer, scaling and reduction kernels.
 #pragma once
 
+#include <type_traits>
+
 #include "device_utils.cuh"
 #include "vec2.cuh"
 
@@ -23,12 +25,36 @@ __device__ __forceinline__ size_t padded_index(const Geom& g, int i, int j,
   for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   \
        r < (nrows); r += gridDim.x * (blockDim.x >> 5))
 
+// Row copies with conversion: a pair of sites per lane where both rows start on
+// a pair's alignment and the types agree (16-byte accesses for complex64), one
+// site otherwise; four accesses in flight per lane.
+template <typename TO, typename TI>
+__device__ __forceinline__ void copy_row(TO* __restrict__ d, const TI* __restrict__ s, int n,
+                                         int lane) {
+  using VI = typename VT<TI>::T;
+  int first = 0;
+  if (std::is_same<TO, float>::value && std::is_same<TI, float>::value &&
+      ((reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(s)) & 15) == 0) {
+    const float4* s4 = reinterpret_cast<const float4*>(s);
+    float4* d4 = reinterpret_cast<float4*>(d);
+#pragma unroll 4
+    for (int i = lane; i < n / 2; i += 32) d4[i] = s4[i];
+    first = n & ~1;
+  }
+#pragma unroll 4
+  for (int i = first + lane; i < n; i += 32) {
+    const VI v = reinterpret_cast<const VI*>(s)[i];
+    st_one<TO>(d + 2 * i, (TO)v.x, (TO)v.y);
+  }
+}
+
 // Dense interior array (any complex type TI) -> padded field of TS, with the
 // boundary ghosts filled, edges included (the caller's halo exchange,
 // src/gpe.f90:165-174).  One warp per padded row, which it gathers from the
 // interior row it is an image of: every store is in row order.  HBM-bound.
 template <typename TS, typename TI>
 __global__ void unpack_kernel(const TI* __restrict__ src, TS* __restrict__ dst, Geom g) {
+  using VI = typename VT<TI>::T;
   const int lane = threadIdx.x & 31;
   const int Nz = g.nz + 2 * GH;
   GPE_FOR_ROWS(r, g.Ny * Nz) {
@@ -38,15 +64,10 @@ __global__ void unpack_kernel(const TI* __restrict__ src, TS* __restrict__ dst, 
     const int ks = ghost_source(k, g.nz, g.bcs), js = ghost_source(j, g.ny, g.bcs);
     const TI* s = src + 2 * ((size_t)ks * g.ny + js) * (size_t)g.nx;
     TS* d = dst + 2 * ((size_t)r * g.Nx + GH);
-#pragma unroll 4
-    for (int i = lane; i < g.nx; i += 32) {
-      const typename VT<TI>::T v = reinterpret_cast<const typename VT<TI>::T*>(s)[i];
-      st_one<TS>(d + 2 * i, (TS)v.x, (TS)v.y);
-    }
+    copy_row<TS, TI>(d, s, g.nx, lane);
     if (lane < 2 * GH) {
       const int i = lane < GH ? lane - GH : g.nx + lane - GH;
-      const typename VT<TI>::T v =
-          reinterpret_cast<const typename VT<TI>::T*>(s)[ghost_source(i, g.nx, g.bcs)];
+      const VI v = reinterpret_cast<const VI*>(s)[ghost_source(i, g.nx, g.bcs)];
       st_one<TS>(d + 2 * i, (TS)v.x, (TS)v.y);
     }
   }
@@ -170,14 +191,7 @@ __global__ void pack_kernel(const TS* __restrict__ src, TO* __restrict__ dst, Ge
   const int lane = threadIdx.x & 31;
   GPE_FOR_ROWS(r, g.ny * g.nz) {
     const int k = r / g.ny, j = r - k * g.ny;
-    const typename VT<TS>::T* s =
-        reinterpret_cast<const typename VT<TS>::T*>(src) + padded_index(g, 0, j, k);
-    TO* d = dst + 2 * (size_t)r * g.nx;
-#pragma unroll 4
-    for (int i = lane; i < g.nx; i += 32) {
-      const typename VT<TS>::T v = s[i];
-      st_one<TO>(d + 2 * i, (TO)v.x, (TO)v.y);
-    }
+    copy_row<TO, TS>(dst + 2 * (size_t)r * g.nx, src + 2 * padded_index(g, 0, j, k), g.nx, lane);
   }
 }
 

@@ -1929,8 +1929,22 @@ int alloc_field(gpe_ctx* c, int id) {
   return GPE_OK;
 }
 
-// d_stage (dense, elements of elem_bytes) -> psi with ghosts.
-int load_stage(gpe_ctx* c, int elem_bytes) {
+// Whether a caller's device array can be read or written by this context's
+// kernels directly: memory of the context's own device, aligned to its
+// elements.  Anything else goes through the staging buffer by cudaMemcpyAsync.
+bool direct_array(const gpe_ctx* c, const void* p, int elem_bytes) {
+  if (reinterpret_cast<uintptr_t>(p) % (uintptr_t)elem_bytes != 0) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == c->dev;
+}
+
+// A dense array (elements of elem_bytes, the staging buffer or a caller's
+// device array) -> psi with ghosts.
+int load_dense(gpe_ctx* c, const void* src, int elem_bytes) {
   Launch L{};
   begin_timed(c, L, GPE_FAM_COPY, (int64_t)c->nint);
   const Geom g = geom(c);
@@ -1939,17 +1953,17 @@ int load_stage(gpe_ctx* c, int elem_bytes) {
   if (c->es == 8) {
     if (elem_bytes == 8)
       unpack_kernel<float, float><<<nb, 256, 0, c->stream>>>(
-          (const float*)c->d_stage, (float*)dst, g);
+          (const float*)src, (float*)dst, g);
     else
       unpack_kernel<float, double><<<nb, 256, 0, c->stream>>>(
-          (const double*)c->d_stage, (float*)dst, g);
+          (const double*)src, (float*)dst, g);
   } else {
     if (elem_bytes == 8)
       unpack_kernel<double, float><<<nb, 256, 0, c->stream>>>(
-          (const float*)c->d_stage, (double*)dst, g);
+          (const float*)src, (double*)dst, g);
     else
       unpack_kernel<double, double><<<nb, 256, 0, c->stream>>>(
-          (const double*)c->d_stage, (double*)dst, g);
+          (const double*)src, (double*)dst, g);
   }
   CU_CHECK(c, cudaGetLastError());
   end_timed(c, L);
@@ -1966,16 +1980,17 @@ int load_stage(gpe_ctx* c, int elem_bytes) {
 }
 
 int stage_in(gpe_ctx* c, const void* src, int elem_bytes, bool device) {
+  if (device && direct_array(c, src, elem_bytes)) return load_dense(c, src, elem_bytes);
   const size_t bytes = c->nint * (size_t)elem_bytes;
   CU_CHECK(c, cudaMemcpyAsync(c->d_stage, src, bytes,
                               device ? cudaMemcpyDeviceToDevice
                                      : cudaMemcpyHostToDevice,
                               c->stream));
-  return load_stage(c, elem_bytes);
+  return load_dense(c, c->d_stage, elem_bytes);
 }
 
-// field -> d_stage (dense, elements of elem_bytes).
-int pack_stage(gpe_ctx* c, int field, int elem_bytes) {
+// field -> dense array (elements of elem_bytes).
+int pack_dense(gpe_ctx* c, int field, void* dst, int elem_bytes) {
   Launch L{};
   begin_timed(c, L, GPE_FAM_COPY, (int64_t)c->nint);
   const Geom g = geom(c);
@@ -1984,17 +1999,17 @@ int pack_stage(gpe_ctx* c, int field, int elem_bytes) {
   if (c->es == 8) {
     if (elem_bytes == 8)
       pack_kernel<float, float><<<nb, 256, 0, c->stream>>>(
-          (const float*)src, (float*)c->d_stage, g);
+          (const float*)src, (float*)dst, g);
     else
       pack_kernel<float, double><<<nb, 256, 0, c->stream>>>(
-          (const float*)src, (double*)c->d_stage, g);
+          (const float*)src, (double*)dst, g);
   } else {
     if (elem_bytes == 8)
       pack_kernel<double, float><<<nb, 256, 0, c->stream>>>(
-          (const double*)src, (float*)c->d_stage, g);
+          (const double*)src, (float*)dst, g);
     else
       pack_kernel<double, double><<<nb, 256, 0, c->stream>>>(
-          (const double*)src, (double*)c->d_stage, g);
+          (const double*)src, (double*)dst, g);
   }
   CU_CHECK(c, cudaGetLastError());
   end_timed(c, L);
@@ -2003,7 +2018,13 @@ int pack_stage(gpe_ctx* c, int field, int elem_bytes) {
 }
 
 int stage_out(gpe_ctx* c, int field, void* dst, int elem_bytes, bool device) {
-  int rc = pack_stage(c, field, elem_bytes);
+  if (device && direct_array(c, dst, elem_bytes)) {
+    const int rc = pack_dense(c, field, dst, elem_bytes);
+    if (rc) return rc;
+    CU_CHECK(c, cudaStreamSynchronize(c->stream));
+    return GPE_OK;
+  }
+  int rc = pack_dense(c, field, c->d_stage, elem_bytes);
   if (rc) return rc;
   CU_CHECK(c, cudaMemcpyAsync(dst, c->d_stage, c->nint * (size_t)elem_bytes,
                               device ? cudaMemcpyDeviceToDevice
@@ -2052,7 +2073,7 @@ void gpe_internal_time_end(gpe_ctx* c, gpe::TimedRegion* r) {
   Launch L{r->family, r->a, r->b, r->sites};
   end_timed(c, L);
 }
-int gpe_internal_load_stage(gpe_ctx* c) { return load_stage(c, c->es); }
+int gpe_internal_load_stage(gpe_ctx* c) { return load_dense(c, c->d_stage, c->es); }
 
 // psi rescaled on the context's stream so that its norm equals the norm the
 // last step fused into d_scal[0] (before any post-step correction); the
