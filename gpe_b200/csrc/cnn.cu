@@ -138,6 +138,11 @@ int launch_conv(gpe_cnn* n, cudaStream_t st, const Act& in, int layer, bool dgra
   return GPE_OK;
 }
 
+// CTAs that take the first W_TAPS0 of the 9 (dz, dx) taps: by the MMAs they issue.
+int wgrad_role0(const gpe_cnn* n) {
+  return std::max(1, std::min(n->wgrad_grid - 1, (n->wgrad_grid * W_TAPS0 + 4) / 9));
+}
+
 int launch_wgrad(gpe_cnn* n, cudaStream_t st, const Act& x, const Act& dy) {
   WgradParams p;
   memset(&p, 0, sizeof(p));
@@ -146,19 +151,17 @@ int launch_wgrad(gpe_cnn* n, cudaStream_t st, const Act& x, const Act& dy) {
   p.nx = n->nx; p.ny = n->ny; p.nz = n->nz;
   p.Xp = n->Xp; p.Yp = n->Yp; p.Zp = n->Zp;
   p.nslab = (n->ny + TYW - 1) / TYW;
-  const int want = std::min(n->nz, std::max(1, (2 * n->num_sms + p.nslab - 1) / p.nslab));
-  p.zchunk = (n->nz + want - 1) / want;
-  p.nzc = (n->nz + p.zchunk - 1) / p.zchunk;
-  p.nitems = p.nslab * p.nzc;
-  p.xbox_bytes = (uint32_t)(XROWS * 2 * n->Xp * 16);
-  p.xslot_bytes = round1k(p.xbox_bytes);
-  p.dbox_bytes = (uint32_t)(TYW * 2 * n->Xp * 16);
-  p.dslot_bytes = round1k(p.dbox_bytes);
+  p.role0 = wgrad_role0(n);
+  p.xslot_bytes = round1k((uint32_t)(XROWS * 2 * n->Xp * 16));
+  p.dslot_bytes = round1k((uint32_t)(TYW * 2 * n->Xp * 16));
   p.partials = n->d_wpart;
+  p.bpartials = n->d_bpart;
   p.status = n->d_status;
   p.wait_limit_ns = CNN_WAIT_LIMIT_NS;
-  const size_t smem = 1024 + (size_t)WSLOTS * p.xslot_bytes + (size_t)DSLOTS * p.dslot_bytes +
-                      16 * 8 + 16;
+  // the epilogue reuses the X ring for 8 x 3 x 256 floats
+  const size_t ring = std::max((size_t)WSLOTS * p.xslot_bytes, (size_t)XROWS * 3 * 256 * 4);
+  const size_t smem = 1024 + ring + (size_t)DSLOTS * p.dslot_bytes +
+                      (2 * WSLOTS + 2 * DSLOTS + 1) * 8 + 16 + 4 * 8 * 4 + 16;
   CNN_CU(n, cudaFuncSetAttribute(conv_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
   conv_wgrad_kernel<<<n->wgrad_grid, W_THREADS, smem, st>>>(p);
@@ -269,13 +272,11 @@ int enqueue_backward(gpe_cnn* n, const FieldView& v, const void* target, int eb)
   for (int l = 3; l >= 0; l--) {
     int rc = launch_wgrad(n, v.stream, n->T[l], *g);
     if (rc) return rc;
-    channel_sum_kernel<<<nb, 256, 0, v.stream>>>(g->p, n->nx, n->ny, n->nz, n->d_bpart);
-    CNN_CU(n, cudaGetLastError());
-    grad_finalize_kernel<<<(NTAP * 256 + 16 + 255) / 256, 256, 0, v.stream>>>(
-        n->d_wpart, n->wgrad_grid, n->d_bpart, nb, n->d_grad + (size_t)l * NTAP * 256,
+    grad_finalize_kernel<<<NTAP + 1, 1024, 0, v.stream>>>(
+        n->d_wpart, n->wgrad_grid, wgrad_role0(n), n->d_bpart, n->d_grad + (size_t)l * NTAP * 256,
         n->d_grad + GPE_CNN_WEIGHTS + l * 16);
     CNN_CU(n, cudaGetLastError());
-    n->launches += 2;
+    n->launches++;
     if (l > 0) {
       ConvParams p;
       memset(&p, 0, sizeof(p));
@@ -409,8 +410,8 @@ int gpe_cnn_create(const gpe_cnn_params* p, gpe_cnn** out) {
             mask[((size_t)(l * NTAP + t) * 16 + co) * 16 + ci] = real_weight(l, co, ci);
     for (int co = 2; co < 16; co++) mask[GPE_CNN_WEIGHTS + 3 * 16 + co] = 0;
     if (cudaMalloc(&n->d_delta, sizeof(float) * 2 * n->nint) != cudaSuccess ||
-        cudaMalloc(&n->d_wpart, sizeof(float) * n->wgrad_grid * NACC * 128 * 16) != cudaSuccess ||
-        cudaMalloc(&n->d_bpart, sizeof(float) * n->ew_blocks * 16) != cudaSuccess ||
+        cudaMalloc(&n->d_wpart, sizeof(float) * n->wgrad_grid * W_PART) != cudaSuccess ||
+        cudaMalloc(&n->d_bpart, sizeof(float) * n->wgrad_grid * 16) != cudaSuccess ||
         cudaMalloc(&n->d_lpart, sizeof(double) * n->ew_blocks) != cudaSuccess ||
         cudaMalloc(&n->d_grad, sizeof(float) * np) != cudaSuccess ||
         cudaMalloc(&n->d_m, sizeof(float) * np) != cudaSuccess ||

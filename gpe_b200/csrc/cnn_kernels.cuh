@@ -28,11 +28,18 @@
 // epilogue and the stores, which overlap the next plane's MMAs.  Every MMA
 // accumulates; slots are zero when a plane first receives data.
 //
-// Weight-gradient kernel: D[(dy, ci), co] += X[(row y + dy), ci, x + dx] *
-// dY[row y, co, x] summed over x in 16-site K steps; A (X) and B (dY) are
-// MN-major operands read in place (8 consecutive rows x 2 halves form the
-// 16 M-groups of an M = 128 operand, three of which are the dy taps), one
-// accumulator per (dz, dx).  All waits are bounded; a timeout sets *status.
+// Weight-gradient kernel: D[(xrow, ci), (yrow, co)] += X[xrow, ci, x + dx] *
+// dY[yrow, co, x] summed over x in 16-site K steps; A (X) and B (dY) are
+// MN-major operands read in place: 8 consecutive X rows x 2 halves form the 16
+// M-groups of an M = 128 operand, 6 dY rows x 2 halves the 12 N-groups of an
+// N = 96 one, and the blocks with xrow - yrow = 0, 1, 2 are the dy taps of all
+// six rows.  An MMA costs about 50 issue cycles whatever its N up to 96, so
+// this does in one what took six with N = 16 (one dY row): 578 -> 71 us a
+// layer at 128^3.  One accumulator of 96 TMEM columns per (dz, dx), so a CTA
+// takes five of the nine (dz, dx) taps or the other four (5 x 96 = 480 of 512
+// columns), over an equal share of all (slab, plane) positions.  The epilogue
+// warps sum dY's channels (the bias gradient) from the same tiles meanwhile.
+// All waits are bounded; a timeout sets *status.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -95,14 +102,18 @@ constexpr int F_TAIL_BYTES = 256;
 static_assert((2 * FSLOTS + 5) * 8 + 16 + 64 <= F_TAIL_BYTES, "tail fits");
 
 // weight gradient
-constexpr int TYW = 2;
-constexpr int XROWS = TYW + 7;
-constexpr int WSLOTS = 4;
-constexpr int DSLOTS = 2;
+constexpr int TYW = 6;            // dY rows of a slab
+constexpr int XROWS = TYW + 2;    // X rows they need: M = 128 = 8 rows x 16 channels
+constexpr int WSLOTS = 4;         // X planes in the ring (two in use)
+constexpr int DSLOTS = 3;         // dY planes
 constexpr int W_EPI_WARPS = 4;
 constexpr int W_THREADS = 32 * (2 + W_EPI_WARPS);
-constexpr uint32_t W_TMEM_COLS = 256;
-constexpr int NACC = 9;  // (dz, dx) accumulators
+constexpr uint32_t W_TMEM_COLS = 512;
+constexpr int W_NCOL = TYW * CH;  // 96 columns per accumulator
+constexpr int W_TAPS0 = 5;        // (dz, dx) taps 0-4 in one role, 5-8 in the other
+constexpr int W_PART = W_TAPS0 * 3 * CH * CH;  // floats of one CTA's partial sums
+static_assert(XROWS * CH == 128, "X rows fill M");
+static_assert(W_TAPS0 * W_NCOL <= (int)W_TMEM_COLS, "accumulators fit TMEM");
 
 enum Epi { EPI_GELU = 0, EPI_GELU_PRE = 1, EPI_DELTA = 2, EPI_RESID = 3, EPI_DGELU = 4 };
 
@@ -128,9 +139,11 @@ struct WgradParams {
   const __nv_bfloat16* x;           // layer input [Zp][Yp][2][Xp][8]
   const __nv_bfloat16* dy;          // gradient of the layer output, same layout
   int nx, ny, nz, Xp, Yp, Zp;
-  int nslab, nzc, zchunk, nitems;
-  uint32_t xslot_bytes, xbox_bytes, dslot_bytes, dbox_bytes;
-  float* partials;                  // [gridDim.x][NACC][128][16]
+  int nslab;                        // slabs of TYW rows
+  int role0;                        // CTAs that take taps 0..W_TAPS0-1
+  uint32_t xslot_bytes, dslot_bytes;
+  float* partials;                  // [gridDim.x][W_TAPS0][3 dy][16 co][16 ci]
+  float* bpartials;                 // [role0][16]
   int* status;
   unsigned long long wait_limit_ns;
 };
@@ -543,6 +556,27 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
 // --------------------------------------------------------------------------
 // Weight gradient.
 
+// The role and the share of (slab, plane) positions, planes running fastest, of
+// one CTA.
+struct WShare {
+  int t0, nt;      // first (dz, dx) tap and their number
+  int dz0;         // its taps need X planes z + dz0 and z + dz0 + 1 (padded)
+  int pos, end;
+};
+__device__ __forceinline__ WShare wgrad_share(const WgradParams& p) {
+  const bool r0 = (int)blockIdx.x < p.role0;
+  const int n = r0 ? p.role0 : (int)gridDim.x - p.role0;
+  const int i = r0 ? (int)blockIdx.x : (int)blockIdx.x - p.role0;
+  const long long total = (long long)p.nslab * p.nz;
+  WShare s;
+  s.t0 = r0 ? 0 : W_TAPS0;
+  s.nt = r0 ? W_TAPS0 : 9 - W_TAPS0;
+  s.dz0 = s.t0 / 3;
+  s.pos = (int)(i * total / n);
+  s.end = (int)((i + 1) * total / n);
+  return s;
+}
+
 __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_constant__ WgradParams p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* xring = reinterpret_cast<unsigned char*>(
@@ -555,15 +589,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
   uint64_t* drain = dempty + DSLOTS;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
-  volatile int* any_flag = abort_flag + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  {  // rings start at zero: rows a copy leaves untouched stay finite
-    uint4* z = reinterpret_cast<uint4*>(xring);
-    const int n16 = (int)(WSLOTS * p.xslot_bytes + DSLOTS * p.dslot_bytes) / 16;
-    for (int i = threadIdx.x; i < n16; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
-  }
-  fence_proxy_async();
+  const WShare sh = wgrad_share(p);
+  const bool bias = (int)blockIdx.x < p.role0;  // this role sums the bias gradient
   if (threadIdx.x == 0) {
     for (int s = 0; s < WSLOTS; s++) {
       mbar_init(&xfull[s], 1);
@@ -571,11 +600,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
     }
     for (int s = 0; s < DSLOTS; s++) {
       mbar_init(&dfull[s], 1);
-      mbar_init(&dempty[s], 1);
+      mbar_init(&dempty[s], bias ? 1 + W_EPI_WARPS : 1);
     }
     mbar_init(drain, 1);
     *abort_flag = 0;
-    *any_flag = 0;
     fence_mbar_init();
   }
   if (warp == 1) tc::tmem_alloc(smem_u32(tmem_holder), W_TMEM_COLS);
@@ -585,6 +613,14 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
   const uint32_t tmem = *tmem_holder;
   const uint64_t lim = p.wait_limit_ns;
   const uint32_t row_bytes = (uint32_t)p.Xp * 16;
+  if (warp >= 2) {  // the accumulators start at zero (every MMA accumulates)
+    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    for (int a = 0; a < W_TAPS0 * W_NCOL / 16; a++) tc::st_32x32b_x16_zero(tq + a * 16);
+    tc::wait_st();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -602,10 +638,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
         gx++;
         return true;
       };
-      auto load_d = [&](int y0, int zpad) -> bool {
+      auto load_d = [&](int y0, int nrows, int zpad) -> bool {
         const uint32_t slot = gd % DSLOTS, cyc = gd / DSLOTS;
         if (cyc > 0 && !mbar_wait_bounded(&dempty[slot], (cyc - 1) & 1, lim)) return false;
-        const uint32_t bytes = (uint32_t)min(TYW, p.Yp - (y0 + 1)) * (uint32_t)(row_elems * 2);
+        const uint32_t bytes = (uint32_t)nrows * (uint32_t)(row_elems * 2);
         mbar_arrive_expect_tx(&dfull[slot], bytes);
         tc::bulk_load(smem_u32(dring + slot * p.dslot_bytes),
                       p.dy + (size_t)zpad * plane_elems + (size_t)(y0 + 1) * row_elems, bytes,
@@ -614,12 +650,14 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
         return true;
       };
       bool ok = true;
-      for (int it = blockIdx.x; it < p.nitems && ok && !*abort_flag; it += gridDim.x) {
-        const int slab = it % p.nslab, zc = it / p.nslab;
-        const int y0 = slab * TYW, z0 = zc * p.zchunk;
-        const int nout = min(z0 + p.zchunk, p.nz) - z0;
-        ok = load_x(y0, z0) && load_x(y0, z0 + 1);
-        for (int o = 0; o < nout && ok; o++) ok = load_x(y0, z0 + o + 2) && load_d(y0, z0 + o + 1);
+      for (int pos = sh.pos; pos < sh.end && ok && !*abort_flag;) {
+        const int slab = pos / p.nz, z0 = pos - slab * p.nz;
+        const int len = min(p.nz - z0, sh.end - pos);
+        const int y0 = slab * TYW, nrows = min(TYW, p.ny - y0);
+        ok = load_x(y0, z0 + sh.dz0);
+        for (int o = 0; o < len && ok && !*abort_flag; o++)
+          ok = load_x(y0, z0 + o + sh.dz0 + 1) && load_d(y0, nrows, z0 + o + 1);
+        pos += len;
       }
       if (!ok) set_abort(p.status, abort_flag, 1);
       const uint32_t fx = gx > WSLOTS ? gx - WSLOTS : 0;
@@ -637,83 +675,132 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = tc::idesc_bf16_f32(128, 16, true, true);
       const uint32_t xring_s = smem_u32(xring), dring_s = smem_u32(dring);
-      uint32_t gx0 = 0, gd0 = 0, xw = 0, dw = 0;
-      bool started = false;
+      uint32_t gx0 = 0, gd = 0, xw = 0;
       const int nxc = p.nx / 16;
-      for (int it = blockIdx.x; it < p.nitems && !*abort_flag; it += gridDim.x) {
-        const int slab = it % p.nslab, zc = it / p.nslab;
-        const int y0 = slab * TYW, z0 = zc * p.zchunk;
-        const int nout = min(z0 + p.zchunk, p.nz) - z0;
-        const int nrows = min(TYW, p.ny - y0);
-        for (int o = 0; o < nout && !*abort_flag; o++) {
+      for (int pos = sh.pos; pos < sh.end && !*abort_flag;) {
+        const int slab = pos / p.nz, z0 = pos - slab * p.nz;
+        const int len = min(p.nz - z0, sh.end - pos);
+        const int nrows = min(TYW, p.ny - slab * TYW);
+        const uint32_t idesc = tc::idesc_bf16_f32(128, 16 * nrows, true, true);
+        for (int o = 0; o < len && !*abort_flag; o++, gd++) {
           bool ok = true;
-          while (ok && xw < gx0 + o + 3) {
+          while (ok && xw < gx0 + o + 2) {
             ok = mbar_wait_bounded(&xfull[xw % WSLOTS], (xw / WSLOTS) & 1, lim);
             if (ok) xw++;
           }
-          while (ok && dw < gd0 + o + 1) {
-            ok = mbar_wait_bounded(&dfull[dw % DSLOTS], (dw / DSLOTS) & 1, lim);
-            if (ok) dw++;
-          }
+          ok = ok && mbar_wait_bounded(&dfull[gd % DSLOTS], (gd / DSLOTS) & 1, lim);
           if (!ok) {
             set_abort(p.status, abort_flag, 1);
             break;
           }
           tc::fence_after_sync();
-          uint32_t xb[3];
+          const uint32_t xb0 = xring_s + ((gx0 + o) % WSLOTS) * p.xslot_bytes;
+          const uint32_t xb1 = xring_s + ((gx0 + o + 1) % WSLOTS) * p.xslot_bytes;
+          const uint32_t db = dring_s + (gd % DSLOTS) * p.dslot_bytes;
+          for (int xc = 0; xc < nxc; xc++) {
+            const uint64_t bdesc =
+                tc::smem_desc(db + (uint32_t)(1 + 16 * xc) * 16, 128, row_bytes);
 #pragma unroll
-          for (int dz = 0; dz < 3; dz++) xb[dz] = xring_s + ((gx0 + o + dz) % WSLOTS) * p.xslot_bytes;
-          const uint32_t db = dring_s + ((gd0 + o) % DSLOTS) * p.dslot_bytes;
-          for (int r = 0; r < nrows; r++) {
-            for (int xc = 0; xc < nxc; xc++) {
-              const uint64_t bdesc = tc::smem_desc(db + (uint32_t)(r * 2) * row_bytes +
-                                                       (uint32_t)(1 + 16 * xc) * 16,
-                                                   128, row_bytes);
-#pragma unroll
-              for (int dz = 0; dz < 3; dz++)
-#pragma unroll
-                for (int dx = 0; dx < 3; dx++) {
-                  const uint64_t adesc = tc::smem_desc(
-                      xb[dz] + (uint32_t)(r * 2) * row_bytes + (uint32_t)(16 * xc + dx) * 16, 128,
-                      row_bytes);
-                  tc::mma_bf16(tmem + (dz * 3 + dx) * 16, adesc, bdesc, idesc, started ? 1u : 0u);
-                }
-              started = true;
+            for (int a = 0; a < W_TAPS0; a++) {
+              if (a >= sh.nt) break;
+              const int t = sh.t0 + a, dz = t / 3, dx = t - 3 * dz;
+              const uint32_t xb = dz == sh.dz0 ? xb0 : xb1;
+              const uint64_t adesc =
+                  tc::smem_desc(xb + (uint32_t)(16 * xc + dx) * 16, 128, row_bytes);
+              tc::mma_bf16(tmem + a * W_NCOL, adesc, bdesc, idesc, 1u);
             }
           }
           tc::commit(smem_u32(&xempty[(gx0 + o) % WSLOTS]));
-          tc::commit(smem_u32(&dempty[(gd0 + o) % DSLOTS]));
+          tc::commit(smem_u32(&dempty[gd % DSLOTS]));
         }
         if (*abort_flag) break;
-        tc::commit(smem_u32(&xempty[(gx0 + nout) % WSLOTS]));
-        tc::commit(smem_u32(&xempty[(gx0 + nout + 1) % WSLOTS]));
-        gx0 += nout + 2;
-        gd0 += nout;
+        tc::commit(smem_u32(&xempty[(gx0 + len) % WSLOTS]));
+        gx0 += len + 1;
+        pos += len;
       }
-      if (started) *any_flag = 1;
       tc::commit(smem_u32(drain));
       if (!mbar_wait_bounded(drain, 0, lim)) set_abort(p.status, abort_flag, 1);
     }
+  } else if (bias) {
+    // bias gradient: warp w sums the (row, half) runs 4 k + w of every dY tile
+    // (its half is w & 1), lanes along x
+    const int w = warp - 2;
+    float acc[8] = {};
+    uint32_t gd = 0;
+    for (int pos = sh.pos; pos < sh.end && !*abort_flag;) {
+      const int slab = pos / p.nz, z0 = pos - slab * p.nz;
+      const int len = min(p.nz - z0, sh.end - pos);
+      const int nrows = min(TYW, p.ny - slab * TYW);
+      for (int o = 0; o < len && !*abort_flag; o++, gd++) {
+        if (!mbar_wait_bounded(&dfull[gd % DSLOTS], (gd / DSLOTS) & 1, lim)) {
+          set_abort(p.status, abort_flag, 1);
+          break;
+        }
+        const unsigned char* d = dring + (gd % DSLOTS) * p.dslot_bytes;
+        for (int q = w; q < 2 * nrows; q += 4)
+          for (int x = lane; x < p.nx; x += 32) {
+            const uint4 v = *reinterpret_cast<const uint4*>(d + (size_t)q * row_bytes + (x + 1) * 16);
+            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[c]));
+              acc[2 * c] += f.x;
+              acc[2 * c + 1] += f.y;
+            }
+          }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&dempty[gd % DSLOTS]);
+      }
+      pos += len;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    }
+    // (through the holder's spare words: 4 warps x 8 floats)
+    float* bs = reinterpret_cast<float*>(tmem_holder + 4);
+    if (lane == 0)
+#pragma unroll
+      for (int c = 0; c < 8; c++) bs[8 * w + c] = acc[c];
   }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  if (warp >= 2) {
-    const int q = warp & 3;
-    const int m = 32 * q + lane;
-    float* out = p.partials + (size_t)blockIdx.x * NACC * 128 * 16;
-    const bool any = *any_flag && !*abort_flag;
-    for (int a = 0; a < NACC; a++) {
-      float v[16];
-      tc::ld_32x32b_x16(tmem + ((uint32_t)(32 * q) << 16) + a * 16, v);
-      float4* o4 = reinterpret_cast<float4*>(out + ((size_t)a * 128 + m) * 16);
+  const bool good = !*abort_flag;
+  float* red = reinterpret_cast<float*>(xring);  // [8 xrow][3 dy][16 co][16 ci], the ring is idle
+  for (int a = 0; a < sh.nt; a++) {
+    if (warp >= 2) {
+      const int q = warp & 3, xrow = 2 * q + (lane >> 4), ci = lane & 15;
+      const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16) + a * W_NCOL;
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        o4[i] = any ? make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3])
-                    : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int jj = -2; jj < 2; jj++) {  // dY rows this warp's two X rows meet
+        const int j = 2 * q + jj;
+        if (j < 0 || j >= TYW) continue;
+        float v[16];
+        tc::ld_32x32b_x16(tq + j * CH, v);
+        const int dy = xrow - j;
+        if (dy >= 0 && dy < 3)
+#pragma unroll
+          for (int co = 0; co < CH; co++) red[((xrow * 3 + dy) * CH + co) * CH + ci] = v[co];
+      }
     }
+    __syncthreads();
+    float* out = p.partials + (size_t)blockIdx.x * W_PART + a * 3 * CH * CH;
+    for (int i = threadIdx.x; i < 3 * CH * CH; i += W_THREADS) {
+      const int dy = i / (CH * CH);
+      float t = 0.f;
+#pragma unroll
+      for (int j = 0; j < TYW; j++) t += red[(j + dy) * 3 * CH * CH + i];
+      out[i] = good ? t : 0.f;
+    }
+    __syncthreads();
+  }
+  if (bias && threadIdx.x < CH) {
+    const float* bs = reinterpret_cast<const float*>(tmem_holder + 4);
+    const int h = threadIdx.x >> 3, c = threadIdx.x & 7;
+    p.bpartials[blockIdx.x * CH + threadIdx.x] = good ? bs[8 * h + c] + bs[8 * (h + 2) + c] : 0.f;
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -788,52 +875,34 @@ __global__ void loss_kernel(const float* __restrict__ delta, const TS* __restric
   }
 }
 
-// Per-block channel sums of a gradient buffer's interior (bias gradient).
-__global__ void channel_sum_kernel(const __nv_bfloat16* __restrict__ g, int nx, int ny, int nz,
-                                   float* __restrict__ partials) {
-  __shared__ float red[256][17];
-  const int Xp = nx + 2, Yp = ny + 2;
-  const size_t n = (size_t)nx * ny * nz;
-  float acc[16] = {};
-  for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n;
-       s += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(s % nx);
-    const size_t t = s / nx;
-    const int y = (int)(t % ny), z = (int)(t / ny);
-    float a[16];
-    load_act16(g, Xp, Yp, x, y, z, a);
-#pragma unroll
-    for (int c = 0; c < 16; c++) acc[c] += a[c];
+// dW[tap][co][ci] (fp32) of one layer from the wgrad partials (one block per
+// tap; four groups of threads take every fourth CTA of the tap's role, added in
+// a fixed order), and db from the channel sums (the last block).
+__global__ void __launch_bounds__(1024) grad_finalize_kernel(const float* __restrict__ wpart, int nblk,
+                                                              int role0,
+                                                              const float* __restrict__ bpart,
+                                                              float* __restrict__ dw,
+                                                              float* __restrict__ db) {
+  __shared__ float s[4][256];
+  const int c = threadIdx.x & 255, g = threadIdx.x >> 8;
+  if (blockIdx.x == NTAP) {
+    if (threadIdx.x < 16) {
+      float t = 0.f;
+      for (int b = 0; b < role0; b++) t += bpart[b * 16 + threadIdx.x];
+      db[threadIdx.x] = t;
+    }
+    return;
   }
-#pragma unroll
-  for (int c = 0; c < 16; c++) red[threadIdx.x][c] = acc[c];
+  const int tap = blockIdx.x, dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+  const int zx = dz * 3 + dx;
+  const int a = zx < W_TAPS0 ? zx : zx - W_TAPS0;
+  const int b0 = zx < W_TAPS0 ? 0 : role0, b1 = zx < W_TAPS0 ? role0 : nblk;
+  float t = 0.f;
+#pragma unroll 8
+  for (int b = b0 + g; b < b1; b += 4) t += wpart[(size_t)b * W_PART + (a * 3 + dy) * 256 + c];
+  s[g][c] = t;
   __syncthreads();
-  if (threadIdx.x < 16) {
-    float t = 0.f;
-    for (int i = 0; i < (int)blockDim.x; i++) t += red[i][threadIdx.x];
-    partials[blockIdx.x * 16 + threadIdx.x] = t;
-  }
-}
-
-// dW[tap][co][ci] (fp32) of one layer from the wgrad partials, and db from
-// the channel sums.  One thread per weight; fixed summation order.
-__global__ void grad_finalize_kernel(const float* __restrict__ wpart, int nwblk,
-                                     const float* __restrict__ bpart, int nbblk,
-                                     float* __restrict__ dw, float* __restrict__ db) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < NTAP * 16 * 16) {
-    const int ci = i % 16, co = (i / 16) % 16, tap = i / 256;
-    const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-    const int a = dz * 3 + dx, m = dy * 16 + ci;
-    float t = 0.f;
-    for (int b = 0; b < nwblk; b++) t += wpart[(((size_t)b * NACC + a) * 128 + m) * 16 + co];
-    dw[i] = t;
-  } else if (i < NTAP * 16 * 16 + 16) {
-    const int c = i - NTAP * 16 * 16;
-    float t = 0.f;
-    for (int b = 0; b < nbblk; b++) t += bpart[b * 16 + c];
-    db[c] = t;
-  }
+  if (g == 0) dw[tap * 256 + c] = (s[0][c] + s[1][c]) + (s[2][c] + s[3][c]);
 }
 
 // Adam (Kingma & Ba) on the masked parameters of all layers.
