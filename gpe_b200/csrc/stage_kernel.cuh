@@ -289,9 +289,21 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
   // ------------------------------ compute warps ------------------------------
   int slot = 0, cslot = 0;
   uint32_t phase = 0;
+  // complex128 pairs are two 16-byte accesses, lanes 32 bytes apart: the upper
+  // four of each eight lanes take their second site first (e = 0 is site x +
+  // sel), so that the eight cover all banks (in order, half of them twice)
+  constexpr bool D = sizeof(TS) == 8;
+  const int sel = D ? (lane >> 2) & 1 : 0;
+  const int oth = 16 - 32 * sel;  // bytes from a pair's first access to the other
   // the warp's first row; row rr of the warp sits rr rows further on
-  const unsigned row_off = ES * (unsigned)((ty * ROWS + R) * HW + 2 * lane + 2);
-  const unsigned pt_off = ES * (unsigned)(ty * ROWS * TX + 2 * lane);
+  const unsigned row_off = ES * (unsigned)((ty * ROWS + R) * HW + 2 * lane + 2 + sel);
+  const unsigned pt_off = ES * (unsigned)(ty * ROWS * TX + 2 * lane + sel);
+  auto ld = [&](const unsigned char* a) -> CPair<TC> {
+    if constexpr (D)
+      return {*reinterpret_cast<const V*>(a), *reinterpret_cast<const V*>(a + oth)};
+    else
+      return ld_cpair<TS, TC>(reinterpret_cast<const TS*>(a));
+  };
   V ar[2], aix[2], alv[2], alv2[2], bev[2][NP > 0 ? NP : 1];
   TC a_re[2] = {p.a_r[0], p.a_r[1]}, a_im[2] = {p.a_i[0], p.a_i[1]};
   double cek_r = p.cek_r, cek_i = p.cek_i, dt0_r = p.dt0_r, dt0_i = p.dt0_i,
@@ -342,12 +354,13 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
   const int z0 = w.z0;
   const int niters = (w.z1 - w.z0) + R;
   const int i0 = tile_x * TX + 2 * lane;
+  const int ie[2] = {i0 + sel, i0 + (1 ^ sel)};  // x of sites e = 0, 1
   const int j0 = tile_y * TY + ty * ROWS;  // the warp's first row
   bool ok0[ROWS], ok1[ROWS];
 #pragma unroll
   for (int rr = 0; rr < ROWS; rr++) {
-    ok0[rr] = (i0 < nx) && (j0 + rr < ny);
-    ok1[rr] = (i0 + 1 < nx) && (j0 + rr < ny);
+    ok0[rr] = (ie[0] < nx) && (j0 + rr < ny);
+    ok1[rr] = (ie[1] < nx) && (j0 + rr < ny);
   }
   const size_t Nx = (size_t)rd.Nx, NxNy = (size_t)rd.Nx * (size_t)rd.Ny;
   TS* const outp[2] = {rd.out[0], rd.out[1]};
@@ -374,9 +387,9 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
   {
     int a, b;
     for (int e = 0; e < 2; e++) {
-      ghost_targets(i0 + e, nx, bcs, 2, a, b);
-      gxo[e][0] = (a != NO_GHOST) ? a - (i0 + e) : 0;
-      gxo[e][1] = (b != NO_GHOST) ? b - (i0 + e) : 0;
+      ghost_targets(ie[e], nx, bcs, 2, a, b);
+      gxo[e][0] = (a != NO_GHOST) ? a - ie[e] : 0;
+      gxo[e][1] = (b != NO_GHOST) ? b - ie[e] : 0;
     }
 #pragma unroll
     for (int rr = 0; rr < ROWS; rr++) {
@@ -384,16 +397,16 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
       Vxy[rr][0] = Vxy[rr][1] = Dxy[rr][0] = Dxy[rr][1] = TC(0);
       Wxy[rr][0] = Wxy[rr][1] = 0.0;
       if (TRAP || ((FULL || (EPI & EPI_ENERGY)) && useV)) {
-        Vxy[rr][0] = rd.tabV[0][i0] + rd.tabV[1][j];
-        Vxy[rr][1] = rd.tabV[0][i0 + 1] + rd.tabV[1][j];
+        Vxy[rr][0] = rd.tabV[0][ie[0]] + rd.tabV[1][j];
+        Vxy[rr][1] = rd.tabV[0][ie[1]] + rd.tabV[1][j];
       }
       if (FULL && useD) {
-        Dxy[rr][0] = rd.tabD[0][i0] + rd.tabD[1][j];
-        Dxy[rr][1] = rd.tabD[0][i0 + 1] + rd.tabD[1][j];
+        Dxy[rr][0] = rd.tabD[0][ie[0]] + rd.tabD[1][j];
+        Dxy[rr][1] = rd.tabD[0][ie[1]] + rd.tabD[1][j];
       }
       if (EPI & EPI_NORM) {
-        Wxy[rr][0] = rd.tabW[0][i0] * rd.tabW[1][j];
-        Wxy[rr][1] = rd.tabW[0][i0 + 1] * rd.tabW[1][j];
+        Wxy[rr][0] = rd.tabW[0][ie[0]] * rd.tabW[1][j];
+        Wxy[rr][1] = rd.tabW[0][ie[1]] * rd.tabW[1][j];
       }
       ghost_targets(j, ny, bcs, 2, a, b);
       gyo[rr][0] = (a != NO_GHOST) ? (a - j) * rd.Nx : 0;
@@ -413,13 +426,14 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
 #pragma unroll
     for (int w = 0; w < R; w++) {
       CPair<TC> v = {vsplat(TC(0)), vsplat(TC(0))};
-      if (ok0[rr]) {
+      if (ok0[rr] || ok1[rr]) {
         const size_t off = 2 * (base + rr * Nx - (size_t)(R - w) * NxNy);
         v = ld_cpair<TS, TC>(rd.stencil + off);
         if (NS == 2) {
           const CPair<TC> v2 = ld_cpair<TS, TC>(rd.stencil2 + off);
           v = {vadd(v.a, v2.a), vadd(v.b, v2.b)};
         }
+        if (D && sel) v = {v.b, v.a};
       }
       q[rr][w] = v;
     }
@@ -441,10 +455,9 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
     for (int rr = 0; rr < ROWS; rr++) {
       // the stencil value is the sum of the NS stencil fields
       const unsigned char* sp = sbase + (size_t)slot * stride + row_off + ES * rr * HW;
-      CPair<TC> v = ld_cpair<TS, TC>(reinterpret_cast<const TS*>(sp));
+      CPair<TC> v = ld(sp);
       if (NS == 2) {
-        const CPair<TC> v2 =
-            ld_cpair<TS, TC>(reinterpret_cast<const TS*>(sp + p.halo_smem_bytes));
+        const CPair<TC> v2 = ld(sp + p.halo_smem_bytes);
         v = {vadd(v.a, v2.a), vadd(v.b, v2.b)};
       }
       q[rr][(R + KK) % QN] = v;
@@ -454,9 +467,9 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
       const unsigned char* hc = sbase + (size_t)cslot * stride + row_off;
       auto lds = [&](int drow, int dcol) {
         const unsigned char* a = hc + (int)ES * (drow * HW + dcol);
-        CPair<TC> v = ld_cpair<TS, TC>(reinterpret_cast<const TS*>(a));
+        CPair<TC> v = ld(a);
         if (NS == 2) {
-          const CPair<TC> v2 = ld_cpair<TS, TC>(reinterpret_cast<const TS*>(a + p.halo_smem_bytes));
+          const CPair<TC> v2 = ld(a + p.halo_smem_bytes);
           v = {vadd(v.a, v2.a), vadd(v.b, v2.b)};
         }
         return v;
@@ -505,8 +518,8 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
         // pointwise part of the recipe
         CPair<TC> sc0, sc1;
         if (NS == 2) {
-          sc0 = ld_cpair<TS, TC>(reinterpret_cast<const TS*>(hr));
-          sc1 = ld_cpair<TS, TC>(reinterpret_cast<const TS*>(hr + p.halo_smem_bytes));
+          sc0 = ld(hr);
+          sc1 = ld(hr + p.halo_smem_bytes);
         }
         const CPair<TC> xa = lds(rr, -2);
         const CPair<TC> xc = lds(rr, 2);
@@ -520,7 +533,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
               sbase + (size_t)slot * stride + hstride + pt_off + ES * rr * TX;
 #pragma unroll
           for (int qq = 0; qq < NP; qq++)
-            P[qq] = ld_cpair<TS, TC>(reinterpret_cast<const TS*>(pb + (size_t)qq * p.pt_smem_bytes));
+            P[qq] = ld(pb + (size_t)qq * p.pt_smem_bytes);
         }
 
         V res[2][2];  // [output][site]
@@ -529,8 +542,17 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
           const CPair<TC>& ctr = zq(rr, 0);
           Star<V> st;
           st.f0 = e ? ctr.b : ctr.a;
-          st.xm1 = e ? ctr.a : xa.b;
-          st.xp1 = e ? xc.a : ctr.b;
+          if (D) {
+            // the pair's other site, and the one chosen from the pairs beside it
+            const V own = e ? ctr.a : ctr.b;
+            const V far = e ? vsel(sel, xa.a, xc.a) : vsel(sel, xc.b, xa.b);
+            const bool up = (e != 0) == (sel != 0);  // the other site is x + 1 of this one
+            st.xp1 = FULL ? vsel(up, own, far) : own;
+            st.xm1 = FULL ? vsel(up, far, own) : far;
+          } else {
+            st.xm1 = e ? ctr.a : xa.b;
+            st.xp1 = e ? xc.a : ctr.b;
+          }
           st.xm2 = e ? xa.b : xa.a;
           st.xp2 = e ? xc.b : xc.a;
           st.ym1 = e ? ym1.b : ym1.a;
@@ -567,7 +589,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
             Kv = rhs_full<R>(st, L, cLv, ft, useV ? Vxy[rr][e] + Vz : TC(0), useD != 0,
                              Dxy[rr][e] + Dz, useG != 0, Us);
             if (useS) {
-              const TC m = (TC)sphere_mask(rd.tabX[0][i0 + e], rd.tabX[1][j0 + rr], rd.tabX[2][z]);
+              const TC m = (TC)sphere_mask(rd.tabX[0][ie[e]], rd.tabX[1][j0 + rr], rd.tabX[2][z]);
               Kv = vmul(vsplat(m), Kv);
             }
           }
@@ -638,7 +660,10 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
 #pragma unroll
           for (int o = 0; o < NOUT; o++) {
             TS* out = outp[o] + 2 * (base + rr * Nx);
-            if (ok1[rr]) {
+            if constexpr (D) {
+              if (ok0[rr]) st_c1<TS>(out + 2 * sel, res[o][0]);
+              if (ok1[rr]) st_c1<TS>(out + 2 * (1 ^ sel), res[o][1]);
+            } else if (ok1[rr]) {
               st_cpair<TS, typename VT<TS>::T>(out, cvt_v<TS>(res[o][0]),
                                                 cvt_v<TS>(res[o][1]));
             } else if (ok0[rr]) {
@@ -648,7 +673,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
 #pragma unroll
               for (int e = 0; e < 2; e++) {
                 if (!(e ? ok1[rr] : ok0[rr])) continue;
-                TS* o1 = out + 2 * e;
+                TS* o1 = out + 2 * (e ^ sel);
                 const V v = res[o][e];
                 if (gxo[e][0]) st_c1<TS>(o1 + 2 * (ptrdiff_t)gxo[e][0], v);
                 if (gxo[e][1]) st_c1<TS>(o1 + 2 * (ptrdiff_t)gxo[e][1], v);
