@@ -451,71 +451,99 @@ __global__ void wait_probe_kernel(unsigned long long limit_ns, int* status) {
 // per block, [4] partials = { sum |psi|^2, and for d = x, y, z the weighted
 // sum of (Re psi - 1) Im(d conj psi) - Im psi Re(d psi) }.  First
 // derivatives use the face ghosts: c1 (f+1 - f-1) + c2 (f+2 - f-2).
-template <typename TS>
-__global__ void diag_kernel(const TS* __restrict__ f, Geom g, double c1x, double c2x,
-                            double c1y, double c2y, double c1z, double c2z,
-                            const double* __restrict__ wx, const double* __restrict__ wy,
-                            const double* __restrict__ wz, double* __restrict__ partials) {
-  __shared__ double red[4][32];
-  const size_t n = (size_t)g.nx * g.ny * g.nz;
-  const size_t sx = 1, sy = (size_t)g.Nx, sz = (size_t)g.Nx * g.Ny;
+// A block owns 32 x 8 sites in (x, y) and marches a chunk of z: the z
+// neighbours come from a register queue, the x and y ones from L1, so DRAM is
+// read about once.  Bound by FP64 and L1 (256^3 complex128: 296 us with every
+// neighbour fetched by its own 64-bit index).
+struct DiagArgs {
+  Geom g;
+  double c1[3], c2[3];
+  const double* w[3];
+  int tx, ty, zchunk;  // tiles in x and y, planes per block
+};
+template <typename TS, bool FOURTH>
+__global__ void __launch_bounds__(256) diag_kernel(const TS* __restrict__ f, DiagArgs p,
+                                                    double* __restrict__ partials) {
+  using V = typename VT<TS>::T;
+  __shared__ double red[4][8];
+  constexpr int R = FOURTH ? 2 : 1;
+  const V* F = reinterpret_cast<const V*>(f);
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int tile = blockIdx.x % (p.tx * p.ty), chunk = blockIdx.x / (p.tx * p.ty);
+  const int i = (tile % p.tx) * 32 + lane, j = (tile / p.tx) * 8 + row;
+  const int z0 = chunk * p.zchunk, z1 = min(z0 + p.zchunk, p.g.nz);
+  const int sy = p.g.Nx;
+  const size_t sz = (size_t)p.g.Nx * p.g.Ny;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-       q += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(q % g.nx);
-    const size_t r = q / g.nx;
-    const int j = (int)(r % g.ny);
-    const int k = (int)(r / g.ny);
-    const size_t pi = padded_index(g, i, j, k);
-    const double re = (double)f[2 * pi], im = (double)f[2 * pi + 1];
-    acc[0] += re * re + im * im;
-    const size_t st[3] = {sx, sy, sz};
-    const double c1[3] = {c1x, c1y, c1z}, c2[3] = {c2x, c2y, c2z};
-    const double w = (wx[i] * wy[j]) * wz[k];
+  if (i < p.g.nx && j < p.g.ny) {
+    const double wxy = p.w[0][i] * p.w[1][j];
+    const V* c = F + padded_index(p.g, i, j, z0);
+    V q[2 * R + 1];  // planes z - R .. z + R
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const size_t p1 = pi + st[a], m1 = pi - st[a], p2 = pi + 2 * st[a], m2 = pi - 2 * st[a];
-      double dr = c1[a] * ((double)f[2 * p1] - (double)f[2 * m1]);
-      double di = c1[a] * ((double)f[2 * p1 + 1] - (double)f[2 * m1 + 1]);
-      if (c2[a] != 0.0) {
-        dr += c2[a] * ((double)f[2 * p2] - (double)f[2 * m2]);
-        di += c2[a] * ((double)f[2 * p2 + 1] - (double)f[2 * m2 + 1]);
+    for (int d = 0; d < 2 * R; d++) q[d] = *(c + (ptrdiff_t)(d - R) * (ptrdiff_t)sz);
+#pragma unroll 2
+    for (int z = z0; z < z1; z++, c += sz) {
+      q[2 * R] = c[(size_t)R * sz];
+      const double re = (double)q[R].x, im = (double)q[R].y;
+      acc[0] += re * re + im * im;
+      const double w = wxy * p.w[2][z];
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        V p1, m1, p2, m2;
+        if (a == 2) {
+          p1 = q[R + 1];
+          m1 = q[R - 1];
+          p2 = q[2 * R];
+          m2 = q[0];
+        } else {
+          const int s = a == 0 ? 1 : sy;
+          p1 = c[s];
+          m1 = c[-s];
+          p2 = FOURTH ? c[2 * s] : p1;
+          m2 = FOURTH ? c[-2 * s] : m1;
+        }
+        double dr = p.c1[a] * ((double)p1.x - (double)m1.x);
+        double di = p.c1[a] * ((double)p1.y - (double)m1.y);
+        if (FOURTH) {
+          dr += p.c2[a] * ((double)p2.x - (double)m2.x);
+          di += p.c2[a] * ((double)p2.y - (double)m2.y);
+        }
+        // Im(d conj psi) = -Im(d psi)
+        acc[1 + a] += w * (-(re - 1.0) * di - im * dr);
       }
-      // Im(d conj psi) = -Im(d psi)
-      acc[1 + a] += w * (-(re - 1.0) * di - im * dr);
+#pragma unroll
+      for (int d = 0; d < 2 * R; d++) q[d] = q[d + 1];
     }
   }
 #pragma unroll
   for (int v = 0; v < 4; v++) {
     const double t = warp_sum(acc[v]);
-    if ((threadIdx.x & 31) == 0) red[v][threadIdx.x >> 5] = t;
+    if (lane == 0) red[v][row] = t;
   }
   __syncthreads();
   if (threadIdx.x < 4) {
     double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[threadIdx.x][w];
+    for (int w = 0; w < 8; w++) t += red[threadIdx.x][w];
     partials[4 * (size_t)blockIdx.x + threadIdx.x] = t;
   }
 }
 
-// [nblk][4] partials -> out[0..3] * scale, fixed order (one CTA of 256).
-__global__ void diag_finalize_kernel(const double* __restrict__ partials, int nblk, double scale,
-                                     double* __restrict__ out) {
-  __shared__ double s[4][256];
-  double a[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-#pragma unroll
-    for (int v = 0; v < 4; v++) a[v] += partials[4 * (size_t)b + v];
-#pragma unroll
-  for (int v = 0; v < 4; v++) s[v][threadIdx.x] = a[v];
+// [nblk][4] partials -> out[0..3] * scale, fixed order (one CTA of 1024).
+__global__ void __launch_bounds__(1024) diag_finalize_kernel(const double* __restrict__ partials,
+                                                              int nblk, double scale,
+                                                              double* __restrict__ out) {
+  __shared__ double s[1024];
+  // value v of blocks b, b + 256, ...: thread 4 b + v, so loads are contiguous
+  double a = 0.0;
+#pragma unroll 4
+  for (int q = threadIdx.x; q < 4 * nblk; q += 1024) a += partials[q];
+  s[threadIdx.x] = a;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-#pragma unroll
-      for (int v = 0; v < 4; v++) s[v][threadIdx.x] += s[v][threadIdx.x + w];
+  for (int w = 512; w >= 4; w >>= 1) {
+    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x < 4) out[threadIdx.x] = s[threadIdx.x][0] * scale;
+  if (threadIdx.x < 4) out[threadIdx.x] = s[threadIdx.x] * scale;
 }
 
 }  // namespace gpe

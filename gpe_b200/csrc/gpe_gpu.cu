@@ -2969,24 +2969,33 @@ int gpe_gpu_diagnostics(gpe_ctx* c, double* mass, double* mom) {
   int rc = check_solo(c);
   if (rc) return rc;
   if (!mass || !mom) return fail(c, GPE_ERR_INVALID, "null output");
-  const Geom g = geom(c);
-  const int nb = (int)std::min<size_t>((size_t)elementwise_blocks(c->nint), c->partials_cap / 2);
-  double c1[3], c2[3];
+  DiagArgs d;
+  d.g = geom(c);
   const double h[3] = {c->dx, c->dy, c->dz};
   for (int a = 0; a < 3; a++) {
-    if (c->prm.order == 2) { c1[a] = 1.0 / (2.0 * h[a]); c2[a] = 0.0; }
-    else { c1[a] = 8.0 / (12.0 * h[a]); c2[a] = -1.0 / (12.0 * h[a]); }
+    if (c->prm.order == 2) { d.c1[a] = 1.0 / (2.0 * h[a]); d.c2[a] = 0.0; }
+    else { d.c1[a] = 8.0 / (12.0 * h[a]); d.c2[a] = -1.0 / (12.0 * h[a]); }
+    d.w[a] = c->tabW[a];
   }
-  if (c->es == 8)
-    diag_kernel<float><<<nb, 256, 0, c->stream>>>((const float*)c->fld[c->psi_id], g, c1[0], c2[0],
-                                                  c1[1], c2[1], c1[2], c2[2], c->tabW[0],
-                                                  c->tabW[1], c->tabW[2], c->d_partials);
-  else
-    diag_kernel<double><<<nb, 256, 0, c->stream>>>((const double*)c->fld[c->psi_id], g, c1[0],
-                                                   c2[0], c1[1], c2[1], c1[2], c2[2], c->tabW[0],
-                                                   c->tabW[1], c->tabW[2], c->d_partials);
+  d.tx = (c->nx + 31) / 32;
+  d.ty = (c->ny + 7) / 8;
+  // about eight blocks of 256 per SM, four partials each
+  const int tiles = d.tx * d.ty;
+  const int room = (int)std::min<size_t>(c->partials_cap / 2 / tiles, (size_t)c->nz);
+  const int chunks = std::max(1, std::min(room, (8 * c->num_sms + tiles - 1) / tiles));
+  d.zchunk = (c->nz + chunks - 1) / chunks;
+  const int nb = tiles * ((c->nz + d.zchunk - 1) / d.zchunk);
+  if ((size_t)nb * 2 > c->partials_cap) return fail(c, GPE_ERR_INVALID, "partials buffer too small");
+  const bool fourth = c->prm.order == 4;
+  if (c->es == 8) {
+    if (fourth) diag_kernel<float, true><<<nb, 256, 0, c->stream>>>((const float*)c->fld[c->psi_id], d, c->d_partials);
+    else diag_kernel<float, false><<<nb, 256, 0, c->stream>>>((const float*)c->fld[c->psi_id], d, c->d_partials);
+  } else {
+    if (fourth) diag_kernel<double, true><<<nb, 256, 0, c->stream>>>((const double*)c->fld[c->psi_id], d, c->d_partials);
+    else diag_kernel<double, false><<<nb, 256, 0, c->stream>>>((const double*)c->fld[c->psi_id], d, c->d_partials);
+  }
   CU_CHECK(c, cudaGetLastError());
-  diag_finalize_kernel<<<1, 256, 0, c->stream>>>(c->d_partials, nb, cell_volume(c), c->d_scal + 4);
+  diag_finalize_kernel<<<1, 1024, 0, c->stream>>>(c->d_partials, nb, cell_volume(c), c->d_scal + 4);
   CU_CHECK(c, cudaGetLastError());
   c->launches += 2;
   rc = allreduce_scalars(c, 4, 4, 0);

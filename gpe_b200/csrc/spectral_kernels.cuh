@@ -352,24 +352,39 @@ struct SpecFinal {
 
 constexpr int F_FIN_THREADS = 1024;
 
-// Sums the block partials (each column by one warp, lanes over blocks, then
-// a fixed shuffle tree), then the mass.dat row (src/io.f90:369-382), eta =
+// Sums of the block partials per column: a block takes 32 columns, its lanes
+// lie over them and its warps over the blocks' rows, then a fixed order over
+// the warps.  (One block for all columns, lanes over rows, read every value
+// from its own sector: 51 us for 592 rows of 144.)
+__global__ void __launch_bounds__(F_FIN_THREADS) spectrum_columns_kernel(
+    const double* __restrict__ partials, int nblk, int ncol, double* __restrict__ cols) {
+  __shared__ double s[32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
+  double x = 0.0;
+  if (c < ncol)
+#pragma unroll 4
+    for (int b = warp; b < nblk; b += 32) x += partials[(size_t)b * ncol + c];
+  s[warp][lane] = x;
+  __syncthreads();
+  if (warp == 0 && c < ncol) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < 32; w++) t += s[w][lane];
+    cols[c] = t;
+  }
+}
+
+// From the column sums the mass.dat row (src/io.f90:369-382), eta =
 // shell sum / count (:701-704) and F(kk) as the running sum of the bins
 // (:673-677).
 template <typename T>
 __global__ void __launch_bounds__(F_FIN_THREADS) spectrum_finalize_kernel(
-    const T* __restrict__ a, const double* __restrict__ partials, SpecFinal f) {
+    const T* __restrict__ a, const double* __restrict__ cols, SpecFinal f) {
   extern __shared__ double col[];  // [HEAD + nf]
   using V2 = typename Vec2<T>::type;
   const int ncol = HEAD + f.nf;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int c = warp; c < ncol; c += F_FIN_THREADS / 32) {
-    double x = 0.0;
-    for (int b = lane; b < f.nblk; b += 32) x += partials[(size_t)b * ncol + c];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(0xffffffffu, x, d);
-    if (lane == 0) col[c] = x;
-  }
+  for (int c = threadIdx.x; c < ncol; c += F_FIN_THREADS) col[c] = cols[c];
   __syncthreads();
   if (threadIdx.x != 0) return;
   const V2 a0 = reinterpret_cast<const V2*>(a)[0];
