@@ -2,6 +2,7 @@
 // length of the resident state; kernels in vortex_kernels.cuh.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -59,10 +60,18 @@ int run(gpe_ctx* c, const FieldView& v, const void* field, bool dense, double* l
   p.cx = v.nx - 2;
   const long long rows = (long long)(v.ny - 2) * (v.nz - 2);
   p.ncell = rows * p.cx;
+  p.scan_rows = std::max(1, L_THREADS / p.cx);
+  size_t smem = (size_t)(p.scan_rows + 1) * v.nx;
+  if (smem > 64 * 1024) {
+    p.scan_rows = 0;
+    smem = 0;
+  }
   int sms = 148, per_sm = 1;
   VX_CU(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, v.dev));
+  VX_CU(c, cudaFuncSetAttribute(line_cells_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)smem));
   VX_CU(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_cells_kernel<T>,
-                                                         L_THREADS, 0));
+                                                         L_THREADS, smem));
   // two waves of resident blocks, each block whole rows in loop order
   const long long want = (long long)sms * (per_sm > 0 ? per_sm : 1) * 2;
   const long long rows_per_block = (rows + want - 1) / want;
@@ -95,7 +104,7 @@ int run(gpe_ctx* c, const FieldView& v, const void* field, bool dense, double* l
   p.bunres = reinterpret_cast<int*>(p.bfirst + nblk);
   TimedRegion t;
   gpe_internal_time_begin(c, &t, GPE_FAM_OTHER, (int64_t)p.ncell);
-  line_cells_kernel<T><<<nblk, L_THREADS, 0, v.stream>>>(p);
+  line_cells_kernel<T><<<nblk, L_THREADS, smem, v.stream>>>(p);
   VX_CU(c, cudaGetLastError());
   gpe_internal_time_end(c, &t);
   line_resolve_kernel<T><<<nblk, L_THREADS, 0, v.stream>>>(p);
@@ -143,7 +152,8 @@ int run_zeros(gpe_ctx* c, const FieldView& v, int64_t* counts, double* points, i
     cudaFree(x->zcount);
     x->zcount = nullptr;
     x->znblk = 0;
-    VX_CU(c, cudaMalloc(&x->zcount, sizeof(long long) * 2 * Z_SECTIONS * (size_t)nblk));
+    VX_CU(c, cudaMalloc(&x->zcount,
+                        sizeof(long long) * Z_SECTIONS * (2 * (size_t)nblk + 1)));
     x->znblk = nblk;
   }
   p.bcount = x->zcount;
@@ -151,21 +161,18 @@ int run_zeros(gpe_ctx* c, const FieldView& v, int64_t* counts, double* points, i
   p.pts = nullptr;
   zeros_count_kernel<T><<<nblk, L_THREADS, 0, v.stream>>>(p);
   VX_CU(c, cudaGetLastError());
-  std::vector<long long> cnt((size_t)Z_SECTIONS * nblk), off((size_t)Z_SECTIONS * nblk);
-  VX_CU(c, cudaMemcpyAsync(cnt.data(), p.bcount, sizeof(long long) * cnt.size(),
-                           cudaMemcpyDeviceToHost, v.stream));
+  long long* d_totals = x->zcount + (size_t)2 * Z_SECTIONS * nblk;
+  zeros_scan_kernel<<<1, Z_SCAN_THREADS, 0, v.stream>>>(p.bcount, nblk,
+                                                        const_cast<long long*>(p.boff), d_totals);
+  VX_CU(c, cudaGetLastError());
+  long long tot[Z_SECTIONS];
+  VX_CU(c, cudaMemcpyAsync(tot, d_totals, sizeof(tot), cudaMemcpyDeviceToHost, v.stream));
   VX_CU(c, cudaStreamSynchronize(v.stream));
-  gpe_internal_count_launches(c, 1);
-  // slots: section by section, blocks in order within a section
+  gpe_internal_count_launches(c, 2);
   long long total = 0;
   for (int s = 0; s < Z_SECTIONS; s++) {
-    long long sec = 0;
-    for (int b = 0; b < nblk; b++) {
-      off[(size_t)b * Z_SECTIONS + s] = total;
-      total += cnt[(size_t)b * Z_SECTIONS + s];
-      sec += cnt[(size_t)b * Z_SECTIONS + s];
-    }
-    if (counts) counts[s] = sec;
+    total += tot[s];
+    if (counts) counts[s] = tot[s];
   }
   if (!points) return GPE_OK;
   if (total > cap)
@@ -181,8 +188,6 @@ int run_zeros(gpe_ctx* c, const FieldView& v, int64_t* counts, double* points, i
     x->zcap = total;
   }
   p.pts = x->zpts;
-  VX_CU(c, cudaMemcpyAsync(const_cast<long long*>(p.boff), off.data(),
-                           sizeof(long long) * off.size(), cudaMemcpyHostToDevice, v.stream));
   zeros_write_kernel<T><<<nblk, L_THREADS, 0, v.stream>>>(p);
   VX_CU(c, cudaGetLastError());
   gpe_internal_count_launches(c, 1);

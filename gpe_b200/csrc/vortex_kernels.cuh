@@ -41,44 +41,37 @@ template <> struct C2<double> { using type = double2; };
 template <> struct C2<float> { using type = float2; };
 
 // Accepted zero points of one component along the 4 edges of a face: the
-// first two (the only ones used) and their count.  An exact zero at a
-// corner writes the reference's xu(lu) without advancing lu and is always
-// overwritten before it is read, so it has no effect here.
+// first two, and how many there are of them (only "two or more" matters).  An
+// exact zero at a corner writes the reference's xu(lu) without advancing lu
+// and is always overwritten before it is read, so it has no effect here.  The
+// crossed edges are taken one after another, so that the lanes of a warp,
+// whose edges differ, divide together.
 __device__ __forceinline__ int edge_zeros(const double w[5], double& x1, double& y1, double& x2,
                                           double& y2) {
+  unsigned rem = 0;
+#pragma unroll
+  for (int q = 0; q < 4; q++) rem |= (w[q] != 0.0 && w[q] * w[q + 1] < 0.0) ? 1u << q : 0u;
   int cnt = 0;
   double px = 0.0, py = 0.0;
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const double a = w[q], b = w[q + 1];
-    if (a != 0.0 && a * b < 0.0) {
-      double cx, cy;
-      if (q == 0) {
-        cx = fabs(a / (a - b));
-        cy = 0.0;
-      } else if (q == 1) {
-        cx = 1.0;
-        cy = fabs(a / (a - b));
-      } else if (q == 2) {
-        cx = fabs(b / (a - b));
-        cy = 1.0;
+  while (rem && cnt < 2) {
+    const int q = __ffs(rem) - 1;
+    rem &= rem - 1;
+    const double a = q == 0 ? w[0] : q == 1 ? w[1] : q == 2 ? w[2] : w[3];
+    const double b = q == 0 ? w[1] : q == 1 ? w[2] : q == 2 ? w[3] : w[4];
+    const double t = fabs((q < 2 ? a : b) / (a - b));
+    const double cx = q == 1 ? 1.0 : q == 3 ? 0.0 : t;
+    const double cy = q == 0 ? 0.0 : q == 2 ? 1.0 : t;
+    if (cnt == 0 || cx != px || cy != py) {
+      if (cnt == 0) {
+        x1 = cx;
+        y1 = cy;
       } else {
-        cx = 0.0;
-        cy = fabs(b / (a - b));
+        x2 = cx;
+        y2 = cy;
       }
-      if (cnt == 0 || cx != px || cy != py) {
-        if (cnt == 0) {
-          x1 = cx;
-          y1 = cy;
-        }
-        if (cnt == 1) {
-          x2 = cx;
-          y2 = cy;
-        }
-        px = cx;
-        py = cy;
-        cnt++;
-      }
+      px = cx;
+      py = cy;
+      cnt++;
     }
   }
   return cnt;
@@ -215,6 +208,14 @@ __device__ __forceinline__ double segment(const Pt& p1, const Pt& p2) {
   return a * sqrt(dx * dx + dy * dy + dz * dz);
 }
 
+// Which components keep one strict sign at a point: bits re > 0, re < 0, im > 0,
+// im < 0.  The AND over the corners of a cell or a face is zero exactly where
+// neither component keeps one sign on all of them.
+template <typename V>
+__device__ __forceinline__ unsigned sign_bits(const V& w) {
+  return (w.x > 0 ? 1u : 0u) | (w.x < 0 ? 2u : 0u) | (w.y > 0 ? 4u : 0u) | (w.y < 0 ? 8u : 0u);
+}
+
 struct LineArgs {
   const void* psi;        // the resident padded field, or a dense interior array
   int nx, ny, nz, Nx, Ny;
@@ -222,6 +223,8 @@ struct LineArgs {
   int cx;               // cells per row, nx - 2
   long long ncell;      // (nx-2)(ny-2)(nz-2)
   long long per_block;  // cells per block (whole rows)
+  int scan_rows;        // rows of cells a scan step takes (max(1, 256 / cx)); 0: rows too
+                        // long for shared memory, cells load their corners
   double* bsum;         // [nblk] sums of the cells resolved in the block
   double* blast;        // [nblk][4] has-writer flag, last x(2) written
   int* bunres;          // [nblk] one-point cells before the block's first writer
@@ -351,22 +354,26 @@ __device__ __forceinline__ int flag_position(bool flag, int* s_cnt, int& total) 
   return pos;
 }
 
-// Pass 1: the block's cells in loop order.  Cells that may hold a line
-// (most do not) are queued in order and processed 256 at a time; their
+// Pass 1: the block's cells in loop order.  A scan step forms, for one more
+// row of points than rows of cells it takes, the sign bits ANDed over the
+// planes k and k + 1 (a row of points is shared with the next step), from
+// which every cell's test is four bytes of shared memory.  Cells that may hold
+// a line (most do not) are queued in order and processed 256 at a time; their
 // faces on which neither component keeps one sign are queued again and
 // evaluated one per thread, so the warps doing the face arithmetic are
 // dense; one-point cells are resolved inside the block wherever an earlier
-// queued cell of the block wrote x(2).
-// Resident blocks per SM the cell pass is compiled for (registers per thread
-// 65536 / (256 x this)).
-#ifndef GPE_LINE_MIN_BLOCKS
-#define GPE_LINE_MIN_BLOCKS 2
-#endif
+// queued cell of the block wrote x(2).  (Loading all eight corners of every
+// cell for its test: 425 us at 256^3 complex128.)
+// Three resident blocks per SM (80 registers, a few spilled): 448 us with two,
+// 359 with three, 357 with four.
 
 template <typename T>
-__global__ void __launch_bounds__(L_THREADS, GPE_LINE_MIN_BLOCKS) line_cells_kernel(LineArgs p) {
+__global__ void __launch_bounds__(L_THREADS, 3) line_cells_kernel(LineArgs p) {
+  using V = typename C2<T>::type;
+  extern __shared__ unsigned char s_bits[];  // [scan_rows + 1][nx]
   __shared__ double s_p2[L_THREADS][3];
-  __shared__ long long s_q[2 * L_THREADS];
+  __shared__ int s_q[2 * L_THREADS];          // queued cells, offsets from the block's first
+  __shared__ long long s_at[L_THREADS];       // field index of a batch cell's corner 0
   __shared__ double s_fx[6 * L_THREADS], s_fy[6 * L_THREADS];
   __shared__ unsigned char s_fc[6 * L_THREADS];
   __shared__ unsigned short s_face[6 * L_THREADS];
@@ -374,47 +381,102 @@ __global__ void __launch_bounds__(L_THREADS, GPE_LINE_MIN_BLOCKS) line_cells_ker
   __shared__ int s_cnt[L_WARPS];
   __shared__ double s_red[L_WARPS];
   const int tid = threadIdx.x;
+  const V* f = static_cast<const V*>(p.psi);
   const long long c0 = (long long)blockIdx.x * p.per_block;
-  const long long c1 = min(c0 + p.per_block, p.ncell);
+  const int ncell = (int)(min(c0 + p.per_block, p.ncell) - c0);  // whole rows
+  const int nrow = ncell / p.cx;
+  const int row0 = (int)(c0 / p.cx), nj = p.ny - 2;
+  const long long plane = (long long)p.Nx * p.Ny;
   double acc = 0.0;
   bool carry_ok = false;
   Pt carry = {0.0, 0.0, 0.0};
-  long long first_writer = c1 - c0;
+  long long first_writer = ncell;
   int unresolved = 0;
   int qn = 0;
-  long long scan = c0;
-  while (scan < c1 || qn > 0) {
+  int row = 0;                     // next row of the block to scan
+  int have_k = -1, have_j = -1;    // the last row of points in s_bits
+  int cell = 0, step_cells = 0;    // cells of the running scan step: done, all
+  int step_row = 0, step_slot = 0;  // its first row, and that row's place in s_bits
+  // this thread's place in a scan step: rows of points, then rows of cells
+  const int pt_rows = max(1, L_THREADS / p.nx), pt_row = p.nx < L_THREADS ? tid / p.nx : 0;
+  const int pt_i = tid - pt_row * p.nx;
+  const int my_jr = p.scan_rows > 1 ? tid / p.cx : 0;
+  while (row < nrow || cell < step_cells || qn > 0) {
     // fill the queue with candidate cells, in order
-    while (qn < L_THREADS && scan < c1) {
-      const long long c = scan + tid;
+    while (qn < L_THREADS && (row < nrow || cell < step_cells)) {
+      if (cell >= step_cells) {  // the next scan step
+        const int r = row0 + row, k = 1 + r / nj, j = 1 + r % nj;
+        const int rows = min(min(max(p.scan_rows, 1), nrow - row), nj - (j - 1));
+        // rows of points j .. j + rows; those up to have_j are there
+        const int from = have_k == k && have_j >= j ? have_j + 1 : j;
+        if (p.scan_rows) {
+          // (no division per point: the threads lie over pt_rows rows at a time)
+          for (int jj = from + pt_row; jj <= j + rows; jj += pt_rows) {
+            const int sl = jj % (p.scan_rows + 1);
+            const V* a = f + ((long long)(k + p.ghost) * p.Ny + (jj + p.ghost)) * p.Nx + p.ghost;
+            if (pt_row < pt_rows)
+              for (int i = pt_i; i < p.nx; i += L_THREADS)
+                s_bits[sl * p.nx + i] = (unsigned char)(sign_bits(a[i]) & sign_bits(a[i + plane]));
+          }
+          step_slot = j % (p.scan_rows + 1);
+        }
+        have_k = k;
+        have_j = j + rows;
+        step_row = row;
+        step_cells = rows * p.cx;
+        cell = 0;
+        row += rows;
+        __syncthreads();
+      }
+      const int c = cell + tid;
       bool cand = false;
-      if (c < c1) {
-        double cu[8], cv[8];
-        load_cell<T>(p, c, cu, cv);
-        cand = may_hold_line(cu, cv);
+      if (c < step_cells) {
+        const int i = 1 + c - my_jr * p.cx;
+        if (p.scan_rows == 0) {
+          const int j = have_j - 1;
+          const V* a = f + ((long long)(have_k + p.ghost) * p.Ny + (j + p.ghost)) * p.Nx + (i + p.ghost);
+          unsigned m = 15u;
+#pragma unroll
+          for (int q = 0; q < 8; q++) m &= sign_bits(a[(q & 1) + ((q >> 1) & 1) * p.Nx + (q >> 2) * plane]);
+          cand = m == 0;
+        } else {
+          int sl = step_slot + my_jr, sh = sl + 1;
+          if (sl > p.scan_rows) sl -= p.scan_rows + 1;
+          if (sh > p.scan_rows) sh -= p.scan_rows + 1;
+          const unsigned char* lo = s_bits + sl * p.nx + i;
+          const unsigned char* hi = s_bits + sh * p.nx + i;
+          cand = (lo[0] & lo[1] & hi[0] & hi[1]) == 0;
+        }
       }
       int total;
       const int pos = flag_position(cand, s_cnt, total);
-      if (cand) s_q[qn + pos] = c;
+      if (cand) s_q[qn + pos] = step_row * p.cx + c;
       qn += total;
-      scan += L_THREADS;
+      cell += L_THREADS;
       __syncthreads();
     }
     if (qn == 0) break;
     const int nb = min(qn, L_THREADS);
     const bool valid = tid < nb;
-    const long long c = valid ? s_q[tid] : 0;
     // the batch's faces: each active one evaluated by whichever thread takes
     // it from the face queue, outcomes folded per cell in face order
     unsigned amask = 0;
     if (valid) {
-      double cu[8], cv[8];
-      load_cell<T>(p, c, cu, cv);
+      const int off = s_q[tid], rr = off / p.cx, r = row0 + rr;
+      const int i = 1 + off - rr * p.cx, k = 1 + r / nj, j = 1 + r % nj;
+      const long long at =
+          ((long long)(k + p.ghost) * p.Ny + (j + p.ghost)) * p.Nx + (i + p.ghost);
+      s_at[tid] = at;
+      unsigned m[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        m[q] = sign_bits(f[at + (q & 1) + ((q >> 1) & 1) * p.Nx + (q >> 2) * plane]);
+      const unsigned faces[6] = {0x2310u, 0x6754u, 0x3751u, 0x2640u, 0x6732u, 0x4510u};
 #pragma unroll
       for (int n = 0; n < 6; n++) {
-        double u[5], v[5];
-        face_values(cu, cv, n, u, v);
-        if (face_active(u, v)) amask |= 1u << n;
+        const unsigned b = m[faces[n] & 7] & m[(faces[n] >> 4) & 7] & m[(faces[n] >> 8) & 7] &
+                           m[(faces[n] >> 12) & 7];
+        if (b == 0) amask |= 1u << n;
         s_fc[tid * 6 + n] = (unsigned char)F_NONE;
       }
     }
@@ -426,10 +488,17 @@ __global__ void __launch_bounds__(L_THREADS, GPE_LINE_MIN_BLOCKS) line_cells_ker
     __syncthreads();
     for (int q = tid; q < nface; q += L_THREADS) {
       const int t = s_face[q] >> 3, n = s_face[q] & 7;
-      double cu[8], cv[8];
-      load_cell<T>(p, s_q[t], cu, cv);
+      const unsigned tab = kFaceCorners[n];
       double u[5], v[5];
-      face_values(cu, cv, n, u, v);
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const int c = (tab >> (4 * e)) & 7;
+        const V w = f[s_at[t] + (c & 1) + ((c >> 1) & 1) * p.Nx + (c >> 2) * plane];
+        u[e] = (double)w.x;
+        v[e] = (double)w.y;
+      }
+      u[4] = u[0];
+      v[4] = v[0];
       double xx = 0.0, yy = 0.0;
       const int code = face_eval(u, v, xx, yy);
       s_fc[t * 6 + n] = (unsigned char)code;
@@ -481,14 +550,14 @@ __global__ void __launch_bounds__(L_THREADS, GPE_LINE_MIN_BLOCKS) line_cells_ker
       b[2] = o.p1.z;
     }
     unresolved += total;
-    if (first >= 0 && !carry_ok) first_writer = s_q[first] - c0;
+    if (first >= 0 && !carry_ok) first_writer = s_q[first];
     if (last >= 0) {
       carry = Pt{s_p2[last][0], s_p2[last][1], s_p2[last][2]};
       carry_ok = true;
     }
     // drop the processed entries
     __syncthreads();
-    const long long keep = (tid < qn - nb) ? s_q[nb + tid] : 0;
+    const int keep = (tid < qn - nb) ? s_q[nb + tid] : 0;
     __syncthreads();
     if (tid < qn - nb) s_q[tid] = keep;
     qn -= nb;
@@ -609,14 +678,16 @@ struct ZeroArgs {
 // Corners of a cell used by the sections: 0 (i,j,k), 1 (i+1,j,k), 2 (i,j+1,k),
 // 3 (i,j,k+1), 4 (i+1,j+1,k), 5 (i+1,j,k+1), 6 (i,j+1,k+1).
 template <typename T>
-__device__ __forceinline__ void load_zero_corners(const ZeroArgs& p, long long c, double re[7],
-                                                  double im[7], int& i, int& j, int& k) {
+__device__ __forceinline__ void load_zero_corners(const ZeroArgs& p, long long c0, int off,
+                                                  double re[7], double im[7], int& i, int& j,
+                                                  int& k) {
+  // cell `off` of a block that starts at c0 (a whole row)
   using V = typename C2<T>::type;
   const V* f = static_cast<const V*>(p.psi);
-  const long long row = c / p.cx;
-  i = 1 + (int)(c - row * p.cx);
-  j = 1 + (int)(row % (p.ny - 2));
-  k = 1 + (int)(row / (p.ny - 2));
+  const int rr = off / p.cx, row = (int)(c0 / p.cx) + rr;
+  i = 1 + off - rr * p.cx;
+  k = 1 + row / (p.ny - 2);
+  j = 1 + row - (k - 1) * (p.ny - 2);
   const int di[7] = {0, 1, 0, 0, 1, 1, 0}, dj[7] = {0, 0, 1, 0, 1, 0, 1},
             dk[7] = {0, 0, 0, 1, 0, 1, 1};
 #pragma unroll
@@ -724,10 +795,11 @@ __global__ void __launch_bounds__(L_THREADS) zeros_count_kernel(ZeroArgs p) {
   int cnt[Z_SECTIONS];
 #pragma unroll
   for (int s = 0; s < Z_SECTIONS; s++) cnt[s] = 0;
-  for (long long c = c0 + threadIdx.x; c < c1; c += L_THREADS) {
+  const int n = (int)(c1 - c0);
+  for (int c = threadIdx.x; c < n; c += L_THREADS) {
     double re[7], im[7];
     int i, j, k;
-    load_zero_corners<T>(p, c, re, im, i, j, k);
+    load_zero_corners<T>(p, c0, c, re, im, i, j, k);
     Pt o;
 #pragma unroll
     for (int s = 0; s < Z_SECTIONS; s++) cnt[s] += zero_section(s, re, im, i, j, k, p, o) ? 1 : 0;
@@ -744,6 +816,40 @@ __global__ void __launch_bounds__(L_THREADS) zeros_count_kernel(ZeroArgs p) {
     long long t = 0;
     for (int w = 0; w < L_WARPS; w++) t += s_cnt[w][threadIdx.x];
     p.bcount[(size_t)blockIdx.x * Z_SECTIONS + threadIdx.x] = t;
+  }
+}
+
+// Output slots: section by section, blocks in order within a section.  Warp s
+// sums section s over the blocks, then scans it from where the sections before
+// it end; totals[s] is the section's number of points.
+constexpr int Z_SCAN_THREADS = 32 * Z_SECTIONS;
+__global__ void __launch_bounds__(Z_SCAN_THREADS) zeros_scan_kernel(
+    const long long* __restrict__ bcount, int nblk, long long* __restrict__ boff,
+    long long* __restrict__ totals) {
+  __shared__ long long s_tot[Z_SECTIONS];
+  const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
+  long long t = 0;
+  for (int b = lane; b < nblk; b += 32) t += bcount[(size_t)b * Z_SECTIONS + s];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+  if (lane == 0) {
+    s_tot[s] = t;
+    totals[s] = t;
+  }
+  __syncthreads();
+  long long at = 0;
+  for (int q = 0; q < s; q++) at += s_tot[q];
+  for (int b0 = 0; b0 < nblk; b0 += 32) {
+    const int b = b0 + lane;
+    const long long c = b < nblk ? bcount[(size_t)b * Z_SECTIONS + s] : 0;
+    long long inc = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const long long o = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += o;
+    }
+    if (b < nblk) boff[(size_t)b * Z_SECTIONS + s] = at + inc - c;
+    at += __shfl_sync(0xffffffffu, inc, 31);
   }
 }
 
@@ -771,7 +877,7 @@ __global__ void __launch_bounds__(L_THREADS) zeros_write_kernel(ZeroArgs p) {
     if (valid) {
       double re[7], im[7];
       int i, j, k;
-      load_zero_corners<T>(p, c, re, im, i, j, k);
+      load_zero_corners<T>(p, c0, (int)(c - c0), re, im, i, j, k);
       Pt o;
 #pragma unroll
       for (int s = 0; s < Z_SECTIONS; s++)
@@ -805,7 +911,7 @@ __global__ void __launch_bounds__(L_THREADS) zeros_write_kernel(ZeroArgs p) {
       const int t = s_qts[q] >> 4, sec = s_qts[q] & 15;
       double re[7], im[7];
       int i, j, k;
-      load_zero_corners<T>(p, base + t, re, im, i, j, k);
+      load_zero_corners<T>(p, c0, (int)(base - c0) + t, re, im, i, j, k);
       Pt o = {0.0, 0.0, 0.0};
       zero_section(sec, re, im, i, j, k, p, o);
       double* out = p.pts + 3 * s_qat[q];
