@@ -17,7 +17,7 @@ from typing import Sequence
 
 import numpy as np
 
-from ._lib import GpeBatchOptsC, GpeParamsC, check_batch, lib
+from ._lib import GpeBatchOptsC, GpeParamsC, check_batch, device_field, lib, torch_ready
 from .solver import GpeParams, GpeSolver
 
 
@@ -107,8 +107,19 @@ class GpeBatch:
         self.opts = opts
 
     def set_states(self, states) -> None:
-        for m, s in zip(self.members, states):
-            m.set_state(s)
+        pairs = list(zip(self.members, states))
+        tensors = [s.contiguous() for _, s in pairs if getattr(s, "is_cuda", False)]
+        if len(tensors) != len(self) or len({t.element_size() for t in tensors}) != 1:
+            for m, s in pairs:
+                m.set_state(s)
+            return
+        # device states of one type for every run: one call, the loads overlap
+        # (24 runs of 25..70 sites a side, loads, 10 steps and reads: 4.88 -> 4.47 ms)
+        for m, t in zip(self.members, tensors):
+            eb = device_field(t, m.shape, m.prm.device, "set_state")
+        torch_ready(tensors[0])
+        ptrs = (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+        check_batch(lib().gpe_batch_set_states_device(self._b, ptrs, eb), self._b)
 
     def advance(self, nsteps: int, want_norms: bool = True) -> np.ndarray | None:
         """nsteps rk4 steps of every run; returns the (nruns, nsteps) norms."""

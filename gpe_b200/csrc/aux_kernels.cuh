@@ -8,6 +8,12 @@
 
 namespace gpe {
 
+// What a step hands back to the host (page-locked memory).
+struct StepResult {
+  double norm;
+  int status;
+};
+
 struct Geom {
   int nx, ny, nz;  // interior
   int Nx, Ny;      // padded pitches
@@ -160,7 +166,9 @@ __global__ void __launch_bounds__(1024) ghosts_norm_kernel(TS* __restrict__ f, G
                                                             const double* __restrict__ partials,
                                                             int nblk, double scale,
                                                             double* __restrict__ out,
-                                                            double* __restrict__ series) {
+                                                            double* __restrict__ series,
+                                                            StepResult* res,
+                                                            const int* __restrict__ status) {
   __shared__ double s[1024];
   if (blockIdx.x > 0) {
     fill_ghost_rows<TS>(f, g, depth, blockIdx.x - 1, gridDim.x - 1);
@@ -171,6 +179,10 @@ __global__ void __launch_bounds__(1024) ghosts_norm_kernel(TS* __restrict__ f, G
     const double r = s[0] * scale;
     out[0] = r;
     if (series) *series = r;
+    if (res) {
+      res->norm = r;
+      res->status = *status;
+    }
   }
 }
 
@@ -254,17 +266,22 @@ __global__ void norm_kernel(const TS* __restrict__ f, Geom g,
 
 // Fixed-order reduction of partials[2*b + slot], b < nblk, by one CTA of
 // 1024 threads.  op 0 = sum, 1 = max.  out[0] = result * scale, written to
-// *series too when it is non-null.
+// *series too when it is non-null, and with the status word to *res.
 __global__ void finalize_kernel(const double* __restrict__ partials, int nblk,
                                 int slot, int op, double scale,
                                 double* __restrict__ out,
-                                double* __restrict__ series) {
+                                double* __restrict__ series, StepResult* res,
+                                const int* __restrict__ status) {
   __shared__ double s[1024];
   reduce_partials(partials, nblk, slot, op, s);
   if (threadIdx.x == 0) {
     const double r = s[0] * scale;
     out[0] = r;
     if (series) *series = r;
+    if (res) {
+      res->norm = r;
+      res->status = *status;
+    }
   }
 }
 

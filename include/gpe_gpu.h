@@ -401,6 +401,11 @@ const char* gpe_batch_last_error(const gpe_batch* batch);
 /* Member context of run `run` (for set_state / get_state / norm / energy;
  * owned by the batch). */
 int gpe_batch_member(gpe_batch* batch, int32_t run, gpe_ctx** ctx);
+/* gpe_gpu_set_state_device for every member at once: psi[run] is a DEVICE array
+ * of that member's grid, finished on the caller's streams; the loads overlap
+ * and the call returns when all are complete. */
+int gpe_batch_set_states_device(gpe_batch* batch, const void* const* psi,
+                                int32_t elem_bytes);
 /* nsteps rk4 steps of every member with time step dt; norms (HOST, may be
  * NULL) receives nruns x nsteps values, run-major. */
 int gpe_batch_advance(gpe_batch* batch, int64_t nsteps, double dt_re,
