@@ -114,7 +114,7 @@ class GpeBatch:
                 m.set_state(s)
             return
         # device states of one type for every run: one call, the loads overlap
-        # (24 runs of 25..70 sites a side, loads, 10 steps and reads: 4.88 -> 4.47 ms)
+        # (24 runs of up to 128 sites a side, loads, 10 steps and reads: 4.88 -> 4.47 ms)
         for m, t in zip(self.members, tensors):
             eb = device_field(t, m.shape, m.prm.device, "set_state")
         torch_ready(tensors[0])

@@ -103,7 +103,7 @@ uint32_t round1k(uint32_t b) { return (b + 1023u) & ~1023u; }
 // Items of a conv launch: y-slabs of TYF rows x z-chunks, about one per SM.
 void conv_items(const gpe_cnn* n, int rows, int* nslab, int* nzc, int* zchunk) {
   *nslab = (n->ny + rows - 1) / rows;
-  int want = std::max(1, F_CTAS_PER_SM * n->num_sms / *nslab);
+  int want = std::max(1, n->num_sms / *nslab);
   want = std::min(want, n->nz);
   *zchunk = (n->nz + want - 1) / want;
   *nzc = (n->nz + *zchunk - 1) / *zchunk;
@@ -131,7 +131,7 @@ int launch_conv(gpe_cnn* n, cudaStream_t st, const Act& in, int layer, bool dgra
                       W_TILES * OutShape<CO>::WTB + F_TAIL_BYTES;
   auto fn = conv_fwd_kernel<EPI, CO>;
   CNN_CU(n, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = std::min(p.nitems, F_CTAS_PER_SM * n->num_sms);
+  const int grid = std::min(p.nitems, n->num_sms);
   fn<<<grid, F_THREADS, smem, st>>>(p);
   CNN_CU(n, cudaGetLastError());
   n->launches++;

@@ -12,33 +12,44 @@
 // operand of tap (dz, dy, dx) for 128 consecutive sites of a row is the row's
 // address + 16 * dx, with LBO = the half stride.  No im2col copy exists.
 //
-// Forward / dgrad kernel: one CTA per (y-slab of 6 rows, z-chunk) item;
-// warp 0 streams input planes (6 + 2 rows, both halves, the full padded x
-// extent) into a 3-slot ring -- in this layout those rows are one contiguous
+// Forward / dgrad kernel: one CTA per (y-slab of 8 rows, z-chunk) item;
+// warp 0 streams input planes (8 + 2 rows, both halves, the full padded x
+// extent) into a 4-slot ring -- in this layout those rows are one contiguous
 // range, fetched by a single 1-D bulk copy (a tensor-map tile with its
-// 16-byte innermost extent moved the same bytes several times slower); warp 1 issues, per input plane and
-// per (input row, dx), ONE tcgen05.mma (M = 128 sites, N = 144, K = 16)
-// whose D block covers every output site that input row feeds: 3 output
-// rows x 3 output planes x 16 channels.  A small MMA costs about 50 issue
-// cycles whatever its N, so 24 MMAs of N = 144 per plane (near the tensor
-// pipe's rate) replace 162 of N = 16.  The accumulators of three output
-// planes rotate in TMEM; when an input plane's MMAs complete, one output
-// plane is finished: warps 2-9 copy its rows to registers (tcgen05.ld
-// 32x32b), zero its slot, release it to the MMA warp, and only then run the
-// epilogue and the stores, which overlap the next plane's MMAs.  Every MMA
-// accumulates; slots are zero when a plane first receives data.
+// 16-byte innermost extent moved the same bytes several times slower); warp 1
+// issues, per input plane and per (input row, dx), ONE tcgen05.mma (M = 128
+// sites, N = 144, K = 16) whose D block covers every output site that input row
+// feeds: 3 output rows x 3 output planes x 16 channels.  The accumulators of
+// three output planes rotate in TMEM; when an input plane's MMAs complete, one
+// output plane is finished.  Its rows are handed over in two halves of four:
+// the 8 epilogue warps of a half copy its rows to registers (tcgen05.ld
+// 32x32b), zero their slots, release them to the MMA warp, and only then run
+// the epilogue and the stores, which overlap the other half's MMAs and the next
+// plane's.  Every MMA accumulates; slots are zero when a plane first receives
+// data.
+//
+// What bounds it: instruction issue of the epilogue (GELU, packing, stores;
+// about 75% of all issue slots) and then the bytes, 134 MB a layer forward, 201
+// where the pre-activation is written or read too.  At 128^3, a layer forward
+// 50.3 -> 33.8 us, with pre-activation 52 -> 42, dgrad 71 -> 46.8, the last
+// layer 35.6 -> 27.9 (of these the elected lane, see tc::elect_one, took an MMA
+// from 110 to 45 cycles of the issuing thread; stores whose ghost images are
+// predicated rather than searched for, and the halves, the rest).  One CTA of 8
+// rows per SM in place of two of 4 reads 1.25 instead of 1.5 times the input and
+// keeps four planes in flight in the same shared memory.
 //
 // Weight-gradient kernel: D[(xrow, ci), (yrow, co)] += X[xrow, ci, x + dx] *
 // dY[yrow, co, x] summed over x in 16-site K steps; A (X) and B (dY) are
 // MN-major operands read in place: 8 consecutive X rows x 2 halves form the 16
 // M-groups of an M = 128 operand, 6 dY rows x 2 halves the 12 N-groups of an
 // N = 96 one, and the blocks with xrow - yrow = 0, 1, 2 are the dy taps of all
-// six rows.  An MMA costs about 50 issue cycles whatever its N up to 96, so
-// this does in one what took six with N = 16 (one dY row): 578 -> 71 us a
-// layer at 128^3.  One accumulator of 96 TMEM columns per (dz, dx), so a CTA
-// takes five of the nine (dz, dx) taps or the other four (5 x 96 = 480 of 512
-// columns), over an equal share of all (slab, plane) positions.  The epilogue
-// warps sum dY's channels (the bias gradient) from the same tiles meanwhile.
+// six rows.  An MMA takes about 90 cycles whatever its N up to 96 (both
+// operands come out of shared memory across the grain), so this does in one
+// what took six with N = 16 (one dY row): 578 -> 66 us a layer at 128^3.  One
+// accumulator of 96 TMEM columns per (dz, dx), so a CTA takes five of the nine
+// (dz, dx) taps or the other four (5 x 96 = 480 of 512 columns), over an equal
+// share of all (slab, plane) positions.  The epilogue warps sum dY's channels
+// (the bias gradient) from the same tiles meanwhile.
 // All waits are bounded; a timeout sets *status.
 #pragma once
 
@@ -56,11 +67,11 @@ constexpr int NLAYER = 4;
 constexpr int TAP_BYTES = 2 * CH * 8 * 2;  // [2 halves][16 rows][8] bf16 = 512
 
 // forward / dgrad
-constexpr int TYF = 4;          // output rows per item
-constexpr int FSLOTS = 2;       // input planes in the shared-memory ring
-constexpr int F_EPI_WARPS = 8;  // one epilogue group: 2 warps per lane quarter
+constexpr int TYF = 8;          // output rows per item
+constexpr int HROWS = TYF / 2;  // rows whose accumulators are handed over together
+constexpr int FSLOTS = 4;       // input planes in the shared-memory ring
+constexpr int F_EPI_WARPS = 4 * HROWS;  // one per lane quarter and row of a half
 constexpr int F_THREADS = 32 * (2 + F_EPI_WARPS);
-constexpr int F_CTAS_PER_SM = 2;  // one CTA's MMAs overlap the other's drain
 // Accumulators: three output planes in a rotating ring (plane z in slot
 // z mod 3), each with the TYF output rows of the slab, column
 // (row * 3 + slot) * 16 + co.  Input row y' (box row i) of input plane j
@@ -72,7 +83,7 @@ constexpr int F_CTAS_PER_SM = 2;  // one CTA's MMAs overlap the other's drain
 constexpr int OSLOTS = 3;
 constexpr int ACC_ROWS = TYF;
 constexpr int NSTACK = 3 * OSLOTS * CH;          // 144
-constexpr uint32_t F_TMEM_COLS = 256;
+constexpr uint32_t F_TMEM_COLS = 512;
 static_assert(ACC_ROWS * OSLOTS * CH <= (int)F_TMEM_COLS, "accumulator ring fits TMEM");
 // B tile of one (rotation j mod 3, dx): rows n = (jrow * 3 + s) * 16 + co
 // hold tap (dz index 2 - ((s - rot + 1) mod 3), dy index 2 - jrow, dx);
@@ -96,10 +107,13 @@ struct OutShape {
 static_assert(OutShape<2>::NB >= 9 * 2, "padded N holds the 18 real columns");
 // every MMA's D block (padded N included) stays inside the allocation
 static_assert((TYF - 1) * OSLOTS * 2 + 32 <= (int)F_TMEM_COLS, "padded blocks fit");
-constexpr int EPI_ROWS = TYF / 2;                // rows per epilogue warp
-// after the weights: 2*FSLOTS + 5 mbarriers, TMEM address, abort flag, 16 biases
-constexpr int F_TAIL_BYTES = 256;
-static_assert((2 * FSLOTS + 5) * 8 + 16 + 64 <= F_TAIL_BYTES, "tail fits");
+// after the weights: 2*FSLOTS + 6 mbarriers, TMEM address, abort flag, and 16
+// biases that are read four at a time
+constexpr int F_TAIL_BYTES = 256, F_BIAS_OFF = 128;
+static_assert((2 * FSLOTS + 6) * 8 + 8 <= F_BIAS_OFF && F_BIAS_OFF % 16 == 0 &&
+                  F_BIAS_OFF + CH * 4 <= F_TAIL_BYTES, "tail fits");
+static_assert(W_TILES * OutShape<16>::WTB % 16 == 0 && W_TILES * OutShape<2>::WTB % 16 == 0,
+              "the tail starts on 16 bytes");
 
 // weight gradient
 constexpr int TYW = 6;            // dY rows of a slab
@@ -161,11 +175,6 @@ __device__ __forceinline__ float tanh_approx(float u) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
   return t;
 }
-__device__ __forceinline__ float gelu(float x) {
-  const float t = tanh_approx(GELU_C * fmaf(GELU_A * x, x * x, x));
-  const float hx = 0.5f * x;
-  return fmaf(hx, t, hx);
-}
 // Two values at once on the packed FP32x2 pipe: u = x (C + C A x^2),
 // gelu = h + h t with h = x / 2, t = tanh(u) (two scalar MUFU operations).
 __device__ __forceinline__ float2 gelu2(float2 x) {
@@ -177,10 +186,16 @@ __device__ __forceinline__ float2 gelu2(float2 x) {
   const float2 h = __fmul2_rn(x, make_float2(0.5f, 0.5f));
   return __ffma2_rn(h, t, h);
 }
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float t = tanh_approx(GELU_C * fmaf(GELU_A * x, x * x, x));
-  const float du = GELU_C * fmaf(3.0f * GELU_A * x, x, 1.0f);
-  return fmaf(0.5f * x * fmaf(-t, t, 1.0f), du, 0.5f * (1.0f + t));
+__device__ __forceinline__ float2 gelu_grad2(float2 x) {
+  constexpr float A3 = 3.0f * GELU_A;
+  const float2 c2 = make_float2(GELU_C, GELU_C), one = make_float2(1.0f, 1.0f),
+               half = make_float2(0.5f, 0.5f);
+  const float2 v = __fmul2_rn(
+      c2, __ffma2_rn(__fmul2_rn(make_float2(GELU_A, GELU_A), x), __fmul2_rn(x, x), x));
+  const float2 t = make_float2(tanh_approx(v.x), tanh_approx(v.y));
+  const float2 du = __fmul2_rn(c2, __ffma2_rn(__fmul2_rn(make_float2(A3, A3), x), x, one));
+  const float2 dt = __ffma2_rn(make_float2(-t.x, -t.y), t, one);
+  return __ffma2_rn(__fmul2_rn(__fmul2_rn(half, x), dt), du, __fmul2_rn(half, __fadd2_rn(one, t)));
 }
 
 __device__ __forceinline__ size_t act_index(int Xp, int Yp, int x, int y, int z, int h) {
@@ -192,38 +207,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// The interior site (x, y, z) and its periodic ghost images (halo 1), in
-// padded coordinates.  Up to three images per axis (n = 1 has both ghosts).
-template <typename F>
-__device__ __forceinline__ void for_images(int x, int y, int z, int nx, int ny, int nz, F f) {
-  const int x1 = x == 0 ? nx + 1 : -1, x2 = x == nx - 1 ? 0 : -1;
-  const int y1 = y == 0 ? ny + 1 : -1, y2 = y == ny - 1 ? 0 : -1;
-  const int z1 = z == 0 ? nz + 1 : -1, z2 = z == nz - 1 ? 0 : -1;
-  if ((x1 & x2 & y1 & y2 & z1 & z2) == -1) {  // interior: no ghost image
-    f(x + 1, y + 1, z + 1);
-    return;
-  }
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const int zp = c == 0 ? z + 1 : (c == 1 ? z1 : z2);
-    if (zp < 0) continue;
-#pragma unroll
-    for (int b = 0; b < 3; b++) {
-      const int yp = b == 0 ? y + 1 : (b == 1 ? y1 : y2);
-      if (yp < 0) continue;
-#pragma unroll
-      for (int a = 0; a < 3; a++) {
-        const int xp = a == 0 ? x + 1 : (a == 1 ? x1 : x2);
-        if (xp < 0) continue;
-        f(xp, yp, zp);
-      }
-    }
-  }
-}
-
-// 16 channels of one site (two 16-byte records) into a [.][.][2][Xp][8]
-// buffer, ghosts included.
-__device__ __forceinline__ void store_act16(__nv_bfloat16* buf, int Xp, int Yp, int nx, int ny,
+// 16 channels of the interior site (x, y, z), whose first half's record is at q,
+// and of its periodic ghost images (halo 1; an axis of one site has both) in a
+// [.][.][2][Xp][8] buffer.  An image lies a whole period away along its axes.
+// Those along x are predicated stores, those along y and z branches that a warp
+// on one row takes as a whole.
+__device__ __forceinline__ void store_act16(__nv_bfloat16* q, int Xp, int Yp, int nx, int ny,
                                             int nz, int x, int y, int z, const float (&a)[16],
                                             bool ghosts) {
   uint4 lo, hi;
@@ -231,15 +220,33 @@ __device__ __forceinline__ void store_act16(__nv_bfloat16* buf, int Xp, int Yp, 
   lo.z = pack_bf16x2(a[4], a[5]);   lo.w = pack_bf16x2(a[6], a[7]);
   hi.x = pack_bf16x2(a[8], a[9]);   hi.y = pack_bf16x2(a[10], a[11]);
   hi.z = pack_bf16x2(a[12], a[13]); hi.w = pack_bf16x2(a[14], a[15]);
-  if (!ghosts) {
-    *reinterpret_cast<uint4*>(buf + act_index(Xp, Yp, x + 1, y + 1, z + 1, 0)) = lo;
-    *reinterpret_cast<uint4*>(buf + act_index(Xp, Yp, x + 1, y + 1, z + 1, 1)) = hi;
-    return;
+  auto put = [&](__nv_bfloat16* r) {
+    *reinterpret_cast<uint4*>(r) = lo;
+    *reinterpret_cast<uint4*>(r + Xp * 8) = hi;
+  };
+  auto row = [&](__nv_bfloat16* r) {
+    put(r);
+    if (!ghosts) return;
+    if (x == 0) put(r + nx * 8);
+    if (x == nx - 1) put(r - nx * 8);
+  };
+  row(q);
+  if (!ghosts) return;
+  const bool y0 = y == 0, y1 = y == ny - 1, z0 = z == 0, z1 = z == nz - 1;
+  if (!(y0 || y1 || z0 || z1)) return;
+  const ptrdiff_t sy = (ptrdiff_t)ny * Xp * 16, sz = (ptrdiff_t)nz * Yp * Xp * 16;
+  if (y0) row(q + sy);
+  if (y1) row(q - sy);
+  if (z0) {
+    row(q + sz);
+    if (y0) row(q + sz + sy);
+    if (y1) row(q + sz - sy);
   }
-  for_images(x, y, z, nx, ny, nz, [&](int xp, int yp, int zp) {
-    *reinterpret_cast<uint4*>(buf + act_index(Xp, Yp, xp, yp, zp, 0)) = lo;
-    *reinterpret_cast<uint4*>(buf + act_index(Xp, Yp, xp, yp, zp, 1)) = hi;
-  });
+  if (z1) {
+    row(q - sz);
+    if (y0) row(q - sz + sy);
+    if (y1) row(q - sz - sy);
+  }
 }
 
 __device__ __forceinline__ void load_act16(const __nv_bfloat16* buf, int Xp, int Yp, int x,
@@ -276,110 +283,123 @@ __device__ __forceinline__ size_t psi_index(const ConvParams& p, int x, int y, i
   return ((size_t)(z + GH) * p.psi_Ny + (y + GH)) * p.psi_Nx + (x + GH);
 }
 
+// off: the site's element offset in an activation buffer.
 template <int EPI>
-__device__ __forceinline__ void epi_load(const ConvParams& p, int x, int y, int z, EpiAux& a) {
+__device__ __forceinline__ void epi_load(const ConvParams& p, int x, int y, int z, size_t off,
+                                         EpiAux& a) {
   if (EPI == EPI_DGELU) {
-    a.lo = *reinterpret_cast<const uint4*>(p.pre_in + act_index(p.Xp, p.Yp, x + 1, y + 1, z + 1, 0));
-    a.hi = *reinterpret_cast<const uint4*>(p.pre_in + act_index(p.Xp, p.Yp, x + 1, y + 1, z + 1, 1));
+    a.lo = *reinterpret_cast<const uint4*>(p.pre_in + off);
+    a.hi = *reinterpret_cast<const uint4*>(p.pre_in + off + p.Xp * 8);
   } else if (EPI == EPI_RESID) {
     a.psi = reinterpret_cast<const float2*>(p.psi)[psi_index(p, x, y, z)];
   }
 }
 
+__device__ __forceinline__ float4 lds_float4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr));
+  return v;
+}
+
+// bias: shared-memory address of the 16 biases.
 template <int EPI>
 __device__ __forceinline__ void conv_epilogue(const ConvParams& p, const float (&acc)[16],
-                                              const float* bias, const EpiAux& aux, int x, int y,
-                                              int z) {
+                                              uint32_t bias, const EpiAux& aux, int x, int y,
+                                              int z, size_t off) {
   if (EPI == EPI_GELU || EPI == EPI_GELU_PRE) {
     float pre[16], a[16];
+    float4 b;
 #pragma unroll
     for (int c = 0; c < 16; c += 2) {
-      const float2 v = __fadd2_rn(make_float2(acc[c], acc[c + 1]), make_float2(bias[c], bias[c + 1]));
+      if (c % 4 == 0) b = lds_float4(bias + c * 4);
+      const float2 v = __fadd2_rn(make_float2(acc[c], acc[c + 1]),
+                                  c % 4 == 0 ? make_float2(b.x, b.y) : make_float2(b.z, b.w));
       const float2 g = gelu2(v);
       pre[c] = v.x;
       pre[c + 1] = v.y;
       a[c] = g.x;
       a[c + 1] = g.y;
     }
-    if (EPI == EPI_GELU_PRE) store_act16(p.pre_out, p.Xp, p.Yp, p.nx, p.ny, p.nz, x, y, z, pre, false);
-    store_act16(p.act_out, p.Xp, p.Yp, p.nx, p.ny, p.nz, x, y, z, a, true);
+    if (EPI == EPI_GELU_PRE) store_act16(p.pre_out + off, p.Xp, p.Yp, p.nx, p.ny, p.nz, x, y, z, pre, false);
+    store_act16(p.act_out + off, p.Xp, p.Yp, p.nx, p.ny, p.nz, x, y, z, a, true);
   } else if (EPI == EPI_DGELU) {
     float g[16];
     const uint32_t w[8] = {aux.lo.x, aux.lo.y, aux.lo.z, aux.lo.w, aux.hi.x, aux.hi.y, aux.hi.z, aux.hi.w};
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
-      g[2 * i] = acc[2 * i] * gelu_grad(f.x);
-      g[2 * i + 1] = acc[2 * i + 1] * gelu_grad(f.y);
+      const float2 r = __fmul2_rn(make_float2(acc[2 * i], acc[2 * i + 1]), gelu_grad2(f));
+      g[2 * i] = r.x;
+      g[2 * i + 1] = r.y;
     }
-    store_act16(p.act_out, p.Xp, p.Yp, p.nx, p.ny, p.nz, x, y, z, g, true);
+    store_act16(p.act_out + off, p.Xp, p.Yp, p.nx, p.ny, p.nz, x, y, z, g, true);
   } else if (EPI == EPI_DELTA) {
     const size_t s = ((size_t)z * p.ny + y) * p.nx + x;
+    const float4 b = lds_float4(bias);
     reinterpret_cast<float2*>(p.delta)[s] =
-        make_float2((acc[0] + bias[0]) * p.out_scale, (acc[1] + bias[1]) * p.out_scale);
+        make_float2((acc[0] + b.x) * p.out_scale, (acc[1] + b.y) * p.out_scale);
   } else {  // EPI_RESID: psi += delta on the solver's field, its periodic ghosts too
+    const float4 b = lds_float4(bias);
     float2 v = aux.psi;
-    v.x += (acc[0] + bias[0]) * p.out_scale;
-    v.y += (acc[1] + bias[1]) * p.out_scale;
+    v.x += (acc[0] + b.x) * p.out_scale;
+    v.y += (acc[1] + b.y) * p.out_scale;
     float2* f = reinterpret_cast<float2*>(p.psi);
-    int gx[3] = {x, NO_GHOST, NO_GHOST}, gy[3] = {y, NO_GHOST, NO_GHOST},
-        gz[3] = {z, NO_GHOST, NO_GHOST};
-    ghost_targets(x, p.nx, 1, GH, gx[1], gx[2]);
-    ghost_targets(y, p.ny, 1, GH, gy[1], gy[2]);
-    ghost_targets(z, p.nz, 1, GH, gz[1], gz[2]);
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      if (gz[c] == NO_GHOST) continue;
-#pragma unroll
-      for (int b = 0; b < 3; b++) {
-        if (gy[b] == NO_GHOST) continue;
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-          if (gx[a] == NO_GHOST) continue;
-          f[psi_index(p, gx[a], gy[b], gz[c])] = v;
-        }
-      }
-    }
+    int gx[2], gy[2], gz[2];
+    ghost_targets(x, p.nx, 1, GH, gx[0], gx[1]);
+    ghost_targets(y, p.ny, 1, GH, gy[0], gy[1]);
+    ghost_targets(z, p.nz, 1, GH, gz[0], gz[1]);
+    auto row = [&](int yt, int zt) {
+      float2* r = f + psi_index(p, 0, yt, zt);
+      r[x] = v;
+      if (gx[0] != NO_GHOST) r[gx[0]] = v;
+      if (gx[1] != NO_GHOST) r[gx[1]] = v;
+    };
+    auto plane = [&](int zt) {
+      row(y, zt);
+      if (gy[0] != NO_GHOST) row(gy[0], zt);
+      if (gy[1] != NO_GHOST) row(gy[1], zt);
+    };
+    plane(z);
+    if (gz[0] != NO_GHOST) plane(gz[0]);
+    if (gz[1] != NO_GHOST) plane(gz[1]);
   }
 }
 
 template <int EPI, int CO>
-__global__ void __launch_bounds__(F_THREADS, F_CTAS_PER_SM)
+__global__ void __launch_bounds__(F_THREADS, 1)
 conv_fwd_kernel(const __grid_constant__ ConvParams p) {
   constexpr int CW = OutShape<CO>::CW, NB = OutShape<CO>::NB, WTB = OutShape<CO>::WTB;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* wsm = ring + FSLOTS * p.slot_bytes + 4096;  // 4 KB of zeros after the ring
+  // 4 KB after the ring: an A operand of 128 sites reads past shorter rows (what
+  // it finds there goes to accumulator lanes past the row, which nothing reads)
+  unsigned char* wsm = ring + FSLOTS * p.slot_bytes + 4096;
   uint64_t* full = reinterpret_cast<uint64_t*>(wsm + W_TILES * WTB);
   uint64_t* empty = full + FSLOTS;
-  uint64_t* accf = empty + FSLOTS;  // MMAs of one input plane done
-  uint64_t* acce = accf + 1;        // the finished output plane's slot is drained
-  uint64_t* drain = acce + 1;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(drain + 1);
+  uint64_t* accf = empty + FSLOTS;  // [2] MMAs of one input plane into a half done
+  uint64_t* acce = accf + 2;        // [2] a half's finished output plane is drained
+  uint64_t* drain = acce + 2;
+  uint64_t* wfull = drain + 1;      // the weights have arrived
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(wfull + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
-  float* bias_s = reinterpret_cast<float*>(tmem_holder + 4);  // [16], 16-byte aligned
+  float* bias_s = reinterpret_cast<float*>(full + F_BIAS_OFF / 8);  // [16]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  {  // weights and the zero pad (generic proxy), then make them visible to the tensor core
-    const uint4* src = reinterpret_cast<const uint4*>(p.w);
-    uint4* dst = reinterpret_cast<uint4*>(wsm);
-    for (int i = threadIdx.x; i < W_TILES * WTB / 16; i += blockDim.x) dst[i] = src[i];
-    // the whole ring and the pad start at zero: rows a copy leaves
-    // untouched (past the grid's last row) and over-reads stay finite
-    uint4* z = reinterpret_cast<uint4*>(ring);
-    for (int i = threadIdx.x; i < (int)(FSLOTS * p.slot_bytes + 4096) / 16; i += blockDim.x)
-      z[i] = make_uint4(0, 0, 0, 0);
-  }
   if (threadIdx.x < 16) bias_s[threadIdx.x] = p.bias ? p.bias[threadIdx.x] : 0.0f;
   if (threadIdx.x == 0) {
     for (int s = 0; s < FSLOTS; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(accf, 1);
-    mbar_init(acce, 32 * F_EPI_WARPS);
+    for (int h = 0; h < 2; h++) {
+      mbar_init(&accf[h], 1);
+      mbar_init(&acce[h], F_EPI_WARPS / 2);
+    }
     mbar_init(drain, 1);
+    mbar_init(wfull, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -392,8 +412,8 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
   const uint64_t lim = p.wait_limit_ns;
   const uint32_t row_bytes = (uint32_t)p.Xp * 16;
   if (warp >= 2) {  // the whole allocation starts at zero
-    const int q = warp & 3, half = (warp - 2) >> 2;
-    for (int a = half; a < (int)F_TMEM_COLS / 16; a += 2)
+    const int q = warp & 3;
+    for (int a = (warp - 2) >> 2; a < (int)F_TMEM_COLS / 16; a += HROWS)
       tc::st_32x32b_x16_zero(tmem + ((uint32_t)(32 * q) << 16) + a * 16);
     tc::wait_st();
   }
@@ -402,9 +422,11 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
   tc::fence_after_sync();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const size_t row_elems = (size_t)p.Hin * p.Xp * 8;
       const size_t plane_elems = (size_t)p.Yp * row_elems;
+      mbar_arrive_expect_tx(wfull, W_TILES * WTB);
+      tc::bulk_load(smem_u32(wsm), p.w, W_TILES * WTB, smem_u32(wfull));
       uint32_t g = 0;
       for (int it = blockIdx.x; it < p.nitems && !*abort_flag; it += gridDim.x) {
         const int slab = it % p.nslab, zc = it / p.nslab;
@@ -430,9 +452,10 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
           set_abort(p.status, abort_flag, 1);
           break;
         }
+      if (!mbar_wait_bounded(wfull, 0, lim)) set_abort(p.status, abort_flag, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr int BROW = OSLOTS * CW;  // B rows / D columns per output row
       const uint32_t idesc1 = tc::idesc_bf16_f32(128, OutShape<CO>::n_of(1), false, false);
       const uint32_t idesc2 = tc::idesc_bf16_f32(128, OutShape<CO>::n_of(2), false, false);
@@ -442,16 +465,17 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
       const uint64_t bdesc0 = tc::smem_desc(w_s, NB * 16, 128);
       const uint64_t adesc0 = tc::smem_desc(ring_s, lbo_a, 128);
       const uint32_t row_step = (uint32_t)p.Hin * row_bytes;
-      uint32_t g = 0, e = 0;  // input planes, steps (one per input plane)
+      uint32_t g = 0;  // input planes
+      if (!mbar_wait_bounded(wfull, 0, lim)) set_abort(p.status, abort_flag, 1);
       for (int it = blockIdx.x; it < p.nitems && !*abort_flag; it += gridDim.x) {
         const int slab = it % p.nslab, zc = it / p.nslab;
         const int y0 = slab * TYF, z0 = zc * p.zchunk;
         const int nout = min(z0 + p.zchunk, p.nz) - z0;
         const int nin = min(TYF, p.ny - y0) + 2;  // input rows y0-1 .. y0+nrows
-        for (int t = 0; t < nout + 2 && !*abort_flag; t++, g++, e++) {
+        for (int t = 0; t < nout + 2 && !*abort_flag; t++, g++) {
           const int j = z0 - 1 + t;  // input plane (may be -1: its ghost plane)
           bool ok = mbar_wait_bounded(&full[g % FSLOTS], (g / FSLOTS) & 1, lim);
-          if (ok && e > 0) ok = mbar_wait_bounded(acce, (e - 1) & 1, lim);
+          if (ok && g > 0) ok = mbar_wait_bounded(&acce[0], (g - 1) & 1, lim);
           if (!ok) {
             set_abort(p.status, abort_flag, 1);
             break;
@@ -459,6 +483,7 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
           tc::fence_after_sync();
           const uint64_t ab = adesc0 + ((g % FSLOTS) * p.slot_bytes >> 4);
           const uint64_t bb = bdesc0 + (uint64_t)(((j + 3) % 3) * 3 * WTB / 16);
+          bool second = false;  // the second half's accumulators are free
 #pragma unroll
           for (int i = 0; i < TYF + 2; i++) {
             // input row i feeds slab rows i-2 .. i: keep those inside [0, TYF)
@@ -468,14 +493,27 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
             const uint32_t idesc = cnt == 3 ? idesc3 : (cnt == 2 ? idesc2 : idesc1);
             const uint32_t d = tmem + (uint32_t)((i - 2 + jlo) * BROW);
             const uint64_t b = bb + (uint64_t)(jlo * BROW * 16 / 16);
+            if (!second && (i - 2 + jlo) * BROW + OutShape<CO>::n_of(cnt) > HROWS * BROW) {
+              if (g > 0 && !mbar_wait_bounded(&acce[1], (g - 1) & 1, lim)) {
+                ok = false;
+                break;
+              }
+              tc::fence_after_sync();
+              second = true;
+            }
             if (i < nin) {
 #pragma unroll
               for (int dx = 0; dx < 3; dx++)
                 tc::mma_bf16(d, ab + ((i * row_step + dx * 16) >> 4), b + (uint64_t)(dx * WTB / 16),
                              idesc, 1u);
             }
+            if (i == HROWS + 1) tc::commit(smem_u32(&accf[0]));  // its rows have all they get
           }
-          tc::commit(smem_u32(accf));
+          if (!ok) {
+            set_abort(p.status, abort_flag, 1);
+            break;
+          }
+          tc::commit(smem_u32(&accf[1]));
           tc::commit(smem_u32(&empty[g % FSLOTS]));
         }
       }
@@ -483,64 +521,65 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
       if (!mbar_wait_bounded(drain, 0, lim)) set_abort(p.status, abort_flag, 1);
     }
   } else {
-    const int q = warp & 3, half = (warp - 2) >> 2;
+    // a warp has two rows of one half, HROWS / 2 apart; the warps of one half
+    // compute while those of the other wait or drain
+    const int q = warp & 3, h = ((warp - 2) >> 2) & 1, r0 = h * HROWS + ((warp - 2) >> 3);
+    constexpr int KROW = HROWS / 2;
     const int x = 32 * q + lane;
-    const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16);
-    uint32_t e = 0;
+    const uint32_t bias = smem_u32(bias_s);
+    const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(r0 * OSLOTS * CW);
+    const size_t plane = (size_t)p.Yp * p.Xp * 16;  // of an activation buffer
+    uint32_t e = 0;  // input planes
     for (int it = blockIdx.x; it < p.nitems && !*abort_flag; it += gridDim.x) {
       const int slab = it % p.nslab, zc = it / p.nslab;
-      const int y0 = slab * TYF, z0 = zc * p.zchunk;
+      const int y0 = slab * TYF + r0, z0 = zc * p.zchunk;
       const int nout = min(z0 + p.zchunk, p.nz) - z0;
-      const int nrows = min(TYF, p.ny - y0);
+      const uint32_t off0 = (uint32_t)((y0 + 1) * 2 * p.Xp + x + 1) * 8;
       bool stop = false;
-      for (int t = 0; t < nout + 2; t++, e++) {
-        if (!mbar_wait_bounded(accf, e & 1, lim)) {
+      for (int t = 0; t < nout + 2 && !stop; t++, e++) {
+        const int zo = z0 - 2 + t;  // output plane finished by input plane zo + 1
+        const uint32_t so = (uint32_t)((zo + 3) % 3);
+        const bool last = t == nout + 1;
+        EpiAux aux[2];
+        float v[2][16];
+        bool mine[2];
+        size_t off[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          mine[k] = zo >= z0 && y0 + k * KROW < p.ny && x < p.nx;
+          off[k] = (size_t)(zo + 1) * plane + off0 + (uint32_t)(k * KROW * p.Xp * 16);
+          if (mine[k]) epi_load<EPI>(p, x, y0 + k * KROW, zo, off[k], aux[k]);
+        }
+        if (!mbar_wait_bounded(&accf[h], e & 1, lim)) {
           set_abort(p.status, abort_flag, 1);
           stop = true;
           break;
         }
         tc::fence_after_sync();
-        const int zo = z0 - 2 + t;  // output plane finished by input plane zo + 1
-        const bool real = zo >= z0;
-        const bool mine = real && x < p.nx;
-        const uint32_t so = (uint32_t)((zo + 3) % 3);
-        EpiAux aux[EPI_ROWS];
-        if (mine) {
 #pragma unroll
-          for (int k = 0; k < EPI_ROWS; k++)
-            if (half + 2 * k < nrows) epi_load<EPI>(p, x, y0 + half + 2 * k, zo, aux[k]);
-        }
-        float v[EPI_ROWS][16];
-        if (real) {
-#pragma unroll
-          for (int k = 0; k < EPI_ROWS; k++) {
-            const int r = half + 2 * k;
-            if (r < nrows) {
-              if (CW == 16) tc::ld_32x32b_x16(tq + (r * OSLOTS + so) * CW, v[k]);
-              else tc::ld_32x32b_x2(tq + (r * OSLOTS + so) * CW, v[k]);
-            }
+        for (int k = 0; k < 2; k++) {
+          const uint32_t tr = tq + (uint32_t)(k * KROW * OSLOTS * CW);
+          if (zo >= z0 && y0 + k * KROW < p.ny) {
+            if (CW == 16) tc::ld_32x32b_x16(tr + so * CW, v[k]);
+            else tc::ld_32x32b_x2(tr + so * CW, v[k]);
           }
-        }
-        const bool last = t == nout + 1;
-        for (int a = half; a < ACC_ROWS; a += 2) {
 #pragma unroll
           for (int ds = 0; ds < 3; ds++) {
             if (ds > 0 && !last) break;  // at the chunk's end: junk of the planes past it
-            const uint32_t col = (a * OSLOTS + (so + ds) % 3) * CW;
-            if (CW == 16) tc::st_32x32b_x16_zero(tq + col);
-            else tc::st_32x32b_x2_zero(tq + col);
+            const uint32_t col = (so + ds) % 3 * CW;
+            if (CW == 16) tc::st_32x32b_x16_zero(tr + col);
+            else tc::st_32x32b_x2_zero(tr + col);
           }
         }
         tc::wait_st();
         tc::fence_before_sync();
-        mbar_arrive(acce);
-        if (mine) {
+        __syncwarp();
+        // the next plane's MMAs run under the arithmetic
+        if (lane == 0) mbar_arrive(&acce[h]);
 #pragma unroll
-          for (int k = 0; k < EPI_ROWS; k++) {
-            const int r = half + 2 * k;
-            if (r < nrows) conv_epilogue<EPI>(p, v[k], bias_s, aux[k], x, y0 + r, zo);
-          }
-        }
+        for (int k = 0; k < 2; k++)
+          if (mine[k])
+            conv_epilogue<EPI>(p, v[k], bias, aux[k], x, y0 + k * KROW, zo, off[k]);
       }
       if (stop) break;
     }
@@ -623,7 +662,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
   tc::fence_after_sync();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const size_t row_elems = (size_t)2 * p.Xp * 8;
       const size_t plane_elems = (size_t)p.Yp * row_elems;
       uint32_t gx = 0, gd = 0;
@@ -674,7 +713,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
         }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const uint32_t xring_s = smem_u32(xring), dring_s = smem_u32(dring);
       uint32_t gx0 = 0, gd = 0, xw = 0;
       const int nxc = p.nx / 16;
@@ -863,7 +902,7 @@ __global__ void loss_kernel(const float* __restrict__ delta, const TS* __restric
     float a[16] = {};
     a[0] = (float)(2.0 * er * inv_n * out_scale);
     a[1] = (float)(2.0 * ei * inv_n * out_scale);
-    store_act16(g, Xp, Yp, nx, ny, nz, x, y, z, a, true);
+    store_act16(g + act_index(Xp, Yp, x + 1, y + 1, z + 1, 0), Xp, Yp, nx, ny, nz, x, y, z, a, true);
   }
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
