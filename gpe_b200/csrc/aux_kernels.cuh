@@ -136,6 +136,7 @@ __device__ __forceinline__ void fill_ghost_rows(TS* __restrict__ f, const Geom& 
 
 template <typename TS>
 __global__ void fill_ghosts_kernel(TS* __restrict__ f, Geom g, int depth) {
+  after_previous();
   fill_ghost_rows<TS>(f, g, depth, blockIdx.x, gridDim.x);
 }
 
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(1024) ghosts_norm_kernel(TS* __restrict__ f, G
                                                             StepResult* res,
                                                             const int* __restrict__ status) {
   __shared__ double s[1024];
+  after_previous();
   if (blockIdx.x > 0) {
     fill_ghost_rows<TS>(f, g, depth, blockIdx.x - 1, gridDim.x - 1);
     return;
@@ -224,6 +226,7 @@ template <typename TS>
 __global__ void rescale_to_kernel(TS* __restrict__ f, size_t nscalars,
                                   const double* __restrict__ target,
                                   const double* __restrict__ current) {
+  after_previous();
   const double s = sqrt(target[0] / current[0]);
   for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < nscalars;
        q += (size_t)gridDim.x * blockDim.x) {
@@ -241,6 +244,7 @@ __global__ void norm_kernel(const TS* __restrict__ f, Geom g,
   __shared__ double s[32];
   const int lane = threadIdx.x & 31;
   double acc = 0.0;
+  after_previous();
   GPE_FOR_ROWS(r, g.ny * g.nz) {
     const int k = r / g.ny, j = r - k * g.ny;
     const typename VT<TS>::T* row =
@@ -273,6 +277,7 @@ __global__ void finalize_kernel(const double* __restrict__ partials, int nblk,
                                 double* __restrict__ series, StepResult* res,
                                 const int* __restrict__ status) {
   __shared__ double s[1024];
+  after_previous();
   reduce_partials(partials, nblk, slot, op, s);
   if (threadIdx.x == 0) {
     const double r = s[0] * scale;

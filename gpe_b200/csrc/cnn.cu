@@ -132,8 +132,7 @@ int launch_conv(gpe_cnn* n, cudaStream_t st, const Act& in, int layer, bool dgra
   auto fn = conv_fwd_kernel<EPI, CO>;
   CNN_CU(n, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = std::min(p.nitems, n->num_sms);
-  fn<<<grid, F_THREADS, smem, st>>>(p);
-  CNN_CU(n, cudaGetLastError());
+  CNN_CU(n, launch_overlapped(true, fn, grid, F_THREADS, smem, st, p));
   n->launches++;
   return GPE_OK;
 }
@@ -164,8 +163,7 @@ int launch_wgrad(gpe_cnn* n, cudaStream_t st, const Act& x, const Act& dy) {
                       (2 * WSLOTS + 2 * DSLOTS + 1) * 8 + 16 + 4 * 8 * 4 + 16;
   CNN_CU(n, cudaFuncSetAttribute(conv_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  conv_wgrad_kernel<<<n->wgrad_grid, W_THREADS, smem, st>>>(p);
-  CNN_CU(n, cudaGetLastError());
+  CNN_CU(n, launch_overlapped(true, conv_wgrad_kernel, n->wgrad_grid, W_THREADS, smem, st, p));
   n->launches++;
   return GPE_OK;
 }
@@ -181,9 +179,8 @@ int check_view(gpe_cnn* n, const FieldView& v) {
 }
 
 int pack_input(gpe_cnn* n, const FieldView& v, const Act& dst) {
-  pack_input_kernel<float><<<n->Zp * n->Yp, 128, 0, v.stream>>>(
-      static_cast<const float*>(v.psi), v.Nx, v.Ny, n->nx, n->ny, n->nz, dst.p, dst.H);
-  CNN_CU(n, cudaGetLastError());
+  CNN_CU(n, launch_overlapped(true, pack_input_kernel<float>, n->Zp * n->Yp, 128, 0, v.stream, v.psi,
+                              v.Nx, v.Ny, n->nx, n->ny, n->nz, dst.p, dst.H));
   n->launches++;
   return GPE_OK;
 }
@@ -255,27 +252,22 @@ int enqueue_train_forward(gpe_cnn* n, const FieldView& v) {
 // Loss and gradients into d_grad (weights then biases); loss partials in d_lpart.
 int enqueue_backward(gpe_cnn* n, const FieldView& v, const void* target, int eb) {
   const int nb = n->ew_blocks;
-  if (eb == 8)
-    loss_kernel<float, float><<<nb, 256, 0, v.stream>>>(
-        n->d_delta, static_cast<const float*>(v.psi), v.Nx, v.Ny,
-        static_cast<const float*>(target), n->nx, n->ny, n->nz, n->prm.out_scale, n->GA.p,
-        n->d_lpart);
-  else
-    loss_kernel<float, double><<<nb, 256, 0, v.stream>>>(
-        n->d_delta, static_cast<const float*>(v.psi), v.Nx, v.Ny,
-        static_cast<const double*>(target), n->nx, n->ny, n->nz, n->prm.out_scale, n->GA.p,
-        n->d_lpart);
-  CNN_CU(n, cudaGetLastError());
+  CNN_CU(n, eb == 8 ? launch_overlapped(true, loss_kernel<float, float>, nb, 256, 0, v.stream,
+                                        n->d_delta, v.psi, v.Nx, v.Ny, target, n->nx, n->ny, n->nz,
+                                        n->prm.out_scale, n->GA.p, n->d_lpart)
+                    : launch_overlapped(true, loss_kernel<float, double>, nb, 256, 0, v.stream,
+                                        n->d_delta, v.psi, v.Nx, v.Ny, target, n->nx, n->ny, n->nz,
+                                        n->prm.out_scale, n->GA.p, n->d_lpart));
   n->launches++;
   Act* g = &n->GA;
   Act* other = &n->GB;
   for (int l = 3; l >= 0; l--) {
     int rc = launch_wgrad(n, v.stream, n->T[l], *g);
     if (rc) return rc;
-    grad_finalize_kernel<<<NTAP + 1, 1024, 0, v.stream>>>(
-        n->d_wpart, n->wgrad_grid, wgrad_role0(n), n->d_bpart, n->d_grad + (size_t)l * NTAP * 256,
-        n->d_grad + GPE_CNN_WEIGHTS + l * 16);
-    CNN_CU(n, cudaGetLastError());
+    CNN_CU(n, launch_overlapped(true, grad_finalize_kernel, NTAP + 1, 1024, 0, v.stream, n->d_wpart,
+                                n->wgrad_grid, wgrad_role0(n), n->d_bpart,
+                                n->d_grad + (size_t)l * NTAP * 256,
+                                n->d_grad + GPE_CNN_WEIGHTS + l * 16));
     n->launches++;
     if (l > 0) {
       ConvParams p;

@@ -388,7 +388,6 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
   float* bias_s = reinterpret_cast<float*>(full + F_BIAS_OFF / 8);  // [16]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x < 16) bias_s[threadIdx.x] = p.bias ? p.bias[threadIdx.x] : 0.0f;
   if (threadIdx.x == 0) {
     for (int s = 0; s < FSLOTS; s++) {
       mbar_init(&full[s], 1);
@@ -417,6 +416,8 @@ conv_fwd_kernel(const __grid_constant__ ConvParams p) {
       tc::st_32x32b_x16_zero(tmem + ((uint32_t)(32 * q) << 16) + a * 16);
     tc::wait_st();
   }
+  after_previous();
+  if (threadIdx.x < 16) bias_s[threadIdx.x] = p.bias ? p.bias[threadIdx.x] : 0.0f;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -660,6 +661,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
+  after_previous();
 
   if (warp == 0) {
     if (tc::elect_one()) {
@@ -868,6 +870,7 @@ __global__ void pack_input_kernel(const TS* __restrict__ psi, int Nx, int Ny, in
   const size_t q0 = ((size_t)(z + GH) * Ny + (y + GH)) * Nx + GH;
   __nv_bfloat16* dst = act + (size_t)row * H * Xp * 8;
   const uint4 zero = make_uint4(0, 0, 0, 0);
+  after_previous();
   for (int xp = threadIdx.x; xp < Xp; xp += blockDim.x) {
     const int x = xp == 0 ? nx - 1 : (xp == nx + 1 ? 0 : xp - 1);
     const size_t q = q0 + x;
@@ -890,6 +893,7 @@ __global__ void loss_kernel(const float* __restrict__ delta, const TS* __restric
   const size_t n = (size_t)nx * ny * nz;
   const double inv_n = 1.0 / (double)n;
   double acc = 0.0;
+  after_previous();
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n;
        s += (size_t)gridDim.x * blockDim.x) {
     const int x = (int)(s % nx);
@@ -924,6 +928,7 @@ __global__ void __launch_bounds__(1024) grad_finalize_kernel(const float* __rest
                                                               float* __restrict__ db) {
   __shared__ float s[4][256];
   const int c = threadIdx.x & 255, g = threadIdx.x >> 8;
+  after_previous();
   if (blockIdx.x == NTAP) {
     if (threadIdx.x < 16) {
       float t = 0.f;

@@ -59,6 +59,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// First statement of a kernel that is launched with launch_overlapped, by every
+// thread: waits until the kernel before it has completed and its memory is
+// visible, and lets the kernel behind it set up its blocks in turn.  In this
+// order: a trigger before the wait would let a third kernel start while the first
+// still runs, and its wait covers the second only (batched steps read stale
+// ghosts then).  Without the launch attribute both are no-ops.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Barrier among the first `nthreads` threads (a multiple of 32) of the CTA.
 __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");

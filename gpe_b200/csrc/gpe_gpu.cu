@@ -18,6 +18,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <mutex>
 #include <string>
 #include <tuple>
 #include <type_traits>
@@ -140,6 +141,58 @@ struct Launch {
 
 // Shared with noalloc.cu, which has no context to hold its messages.
 void gpe_internal_set_last_error(const std::string& msg) { g_last_create_error = msg; }
+
+namespace {
+// Page-locked StepResults, 64 to an allocation: page-locking takes some
+// milliseconds, and an ensemble has a context per run.  An allocation goes when
+// its last result is given back.
+struct ResultPages {
+  struct Page {
+    gpe::StepResult* at;
+    uint64_t used;
+  };
+  std::mutex m;
+  std::vector<Page> pages;
+};
+ResultPages& result_pages() {
+  static ResultPages* p = new ResultPages;  // outlives every context
+  return *p;
+}
+gpe::StepResult* take_result() {
+  ResultPages& r = result_pages();
+  std::lock_guard<std::mutex> lock(r.m);
+  gpe::StepResult* at = nullptr;
+  for (auto& p : r.pages)
+    for (int i = 0; i < 64 && !at; i++)
+      if (!(p.used >> i & 1)) {
+        p.used |= (uint64_t)1 << i;
+        at = p.at + i;
+      }
+  if (!at) {
+    if (cudaHostAlloc(&at, 64 * sizeof(gpe::StepResult),
+                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
+      return nullptr;
+    r.pages.push_back({at, 1});
+  }
+  *at = gpe::StepResult{};
+  return at;
+}
+void give_result(gpe::StepResult* at) {
+  if (!at) return;
+  ResultPages& r = result_pages();
+  std::lock_guard<std::mutex> lock(r.m);
+  for (size_t k = 0; k < r.pages.size(); k++) {
+    auto& p = r.pages[k];
+    if (at < p.at || at >= p.at + 64) continue;
+    p.used &= ~((uint64_t)1 << (at - p.at));
+    if (!p.used) {
+      cudaFreeHost(p.at);
+      r.pages.erase(r.pages.begin() + (long)k);
+    }
+    return;
+  }
+}
+}  // namespace
 
 struct gpe_ctx {
   gpe_params prm;
@@ -793,6 +846,23 @@ KernelFn select_kernel(int R, int* form, const StageSpec& sp, int am, int bm) {
   }
 }
 
+// Launches of this context's step may overlap the end of the one before: not
+// while each is timed by itself, nor in a grid that is split over contexts, whose
+// streams wait for one another, nor in the step control of rk45, whose attempts
+// replay from a graph already (128^3: 284 us an attempt in complex128, 310 with
+// overlapped launches).
+// Nor on fields beyond OVERLAP_BYTES, where the gap is nothing and the blocks of
+// the next kernel only get in the way of this one's last: a step with and without,
+// complex64 order 2: 21.7 and 32.9 us at 64^3, 53 and 66 at 128^3, 269 and 280 at
+// 256^3 (134 MB); complex128: 24.4 and 29.9 at 64^3, 118 and 123 at 128^3;
+// but six steps of complex128 order 4 at 256^3 (268 MB) 4.71 ms either way, four of
+// complex64 order 4 at 512^3 (1 GB) 11.5 and 11.2.
+constexpr size_t OVERLAP_BYTES = (size_t)192 << 20;
+bool overlap(const gpe_ctx* c) {
+  return !c->timing && !c->comm && !c->group && c->prm.scheme != GPE_SCHEME_RK45 &&
+         c->nint * (size_t)c->es <= OVERLAP_BYTES;
+}
+
 // part 0: the whole slab; part 1: its boundary planes z = 0, 1 and nz-2,
 // nz-1 (the planes the z-neighbours' ghosts take); part 2: the planes
 // between them.  Parts 1 and 2 write their per-CTA partials one after the
@@ -851,7 +921,7 @@ int launch_stage_t(gpe_ctx* c, const StageSpec& sp, int part) {
     L.sites = (int64_t)c->nx * c->ny * planes;
     cudaEventRecord(L.a, c->stream);
   }
-  CU_CHECK(c, cudaLaunchKernel(fn, grid, block, args, sh.smem, c->stream));
+  CU_CHECK(c, launch_overlapped(overlap(c), fn, grid, block, args, sh.smem, c->stream));
   if (c->timing) {
     cudaEventRecord(L.b, c->stream);
     c->timed.push_back(L);
@@ -1047,10 +1117,10 @@ int finalize_one(gpe_ctx* c, int nblk, int slot, int op, double scale,
                  int out_index, bool series) {
   Launch L{};
   begin_timed(c, L, GPE_FAM_REDUCE, 0);
-  finalize_kernel<<<1, 1024, 0, c->stream>>>(c->d_partials, nblk, slot, op, scale,
-                                              c->d_scal + out_index, series ? c->step_series : nullptr,
-                                              series ? c->h_res : nullptr, c->d_status);
-  CU_CHECK(c, cudaGetLastError());
+  CU_CHECK(c, launch_overlapped(overlap(c), finalize_kernel, 1, 1024, 0, c->stream, c->d_partials,
+                                nblk, slot, op, scale, c->d_scal + out_index,
+                                series ? c->step_series : nullptr, series ? c->h_res : nullptr,
+                                c->d_status));
   end_timed(c, L);
   c->launches++;
   return allreduce_scalars(c, out_index, 1, op);
@@ -1288,8 +1358,8 @@ int launch_pair_t(gpe_ctx* c, const PairSpec& sp) {
   p.stall_plane = c->stall_plane;
   void* args[] = {&p};
   const unsigned grid = (unsigned)std::min<long>(p.nitems, slots);
-  CU_CHECK(c, cudaLaunchKernel(fn, dim3(grid), dim3(32, (unsigned)sh.threads_y), args, sh.smem,
-                               c->stream));
+  CU_CHECK(c, launch_overlapped(overlap(c), fn, dim3(grid), dim3(32, (unsigned)sh.threads_y), args,
+                                sh.smem, c->stream));
   c->launches++;
   c->last_nblk = p.nitems;
   return GPE_OK;
@@ -1306,11 +1376,14 @@ int ghost_blocks(const gpe_ctx* c, int warps) {
 int fill_ghosts(gpe_ctx* c, int field) {
   const Geom g = geom(c);
   const int depth = c->prm.order, nb = ghost_blocks(c, 8);
+  cudaError_t e;
   if (c->es == 8)
-    fill_ghosts_kernel<float><<<nb, 256, 0, c->stream>>>((float*)c->fld[field], g, depth);
+    e = launch_overlapped(overlap(c), fill_ghosts_kernel<float>, nb, 256, 0, c->stream,
+                          c->fld[field], g, depth);
   else
-    fill_ghosts_kernel<double><<<nb, 256, 0, c->stream>>>((double*)c->fld[field], g, depth);
-  CU_CHECK(c, cudaGetLastError());
+    e = launch_overlapped(overlap(c), fill_ghosts_kernel<double>, nb, 256, 0, c->stream,
+                          c->fld[field], g, depth);
+  CU_CHECK(c, e);
   c->launches++;
   return GPE_OK;
 }
@@ -1330,15 +1403,16 @@ int launch_pair(gpe_ctx* c, const PairSpec& sp) {
 int finish_pairs(gpe_ctx* c) {
   const Geom g = geom(c);
   const int depth = c->prm.order, nb = ghost_blocks(c, 32) + 1;
+  cudaError_t e;
   if (c->es == 8)
-    ghosts_norm_kernel<float><<<nb, 1024, 0, c->stream>>>(
-        (float*)c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk, cell_volume(c), c->d_scal,
-        c->step_series, c->h_res, c->d_status);
+    e = launch_overlapped(overlap(c), ghosts_norm_kernel<float>, nb, 1024, 0, c->stream,
+                          c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk,
+                          cell_volume(c), c->d_scal, c->step_series, c->h_res, c->d_status);
   else
-    ghosts_norm_kernel<double><<<nb, 1024, 0, c->stream>>>(
-        (double*)c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk, cell_volume(c), c->d_scal,
-        c->step_series, c->h_res, c->d_status);
-  CU_CHECK(c, cudaGetLastError());
+    e = launch_overlapped(overlap(c), ghosts_norm_kernel<double>, nb, 1024, 0, c->stream,
+                          c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk,
+                          cell_volume(c), c->d_scal, c->step_series, c->h_res, c->d_status);
+  CU_CHECK(c, e);
   c->launches++;
   return GPE_OK;
 }
@@ -2093,26 +2167,26 @@ int gpe_internal_load_stage(gpe_ctx* c) { return load_dense(c, c->d_stage, c->es
 int gpe_internal_restore_norm(gpe_ctx* c) {
   const Geom g = geom(c);
   const int nb = elementwise_blocks(c->nint);
+  const bool ov = overlap(c);
+  cudaError_t e;
   if (c->es == 8)
-    norm_kernel<float><<<nb, 256, 0, c->stream>>>((const float*)c->fld[c->psi_id], g,
-                                                  c->tabW[0], c->tabW[1], c->tabW[2],
-                                                  c->d_partials);
+    e = launch_overlapped(ov, norm_kernel<float>, nb, 256, 0, c->stream, c->fld[c->psi_id], g,
+                          c->tabW[0], c->tabW[1], c->tabW[2], c->d_partials);
   else
-    norm_kernel<double><<<nb, 256, 0, c->stream>>>((const double*)c->fld[c->psi_id], g,
-                                                   c->tabW[0], c->tabW[1], c->tabW[2],
-                                                   c->d_partials);
-  CU_CHECK(c, cudaGetLastError());
-  finalize_kernel<<<1, 1024, 0, c->stream>>>(c->d_partials, nb, 0, 0, cell_volume(c),
-                                              c->d_scal + 8, nullptr, nullptr, c->d_status);
+    e = launch_overlapped(ov, norm_kernel<double>, nb, 256, 0, c->stream, c->fld[c->psi_id], g,
+                          c->tabW[0], c->tabW[1], c->tabW[2], c->d_partials);
+  CU_CHECK(c, e);
+  CU_CHECK(c, launch_overlapped(ov, finalize_kernel, 1, 1024, 0, c->stream, c->d_partials, nb, 0, 0,
+                                cell_volume(c), c->d_scal + 8, nullptr, nullptr, c->d_status));
   const size_t n = c->npad * 2;
   const int sb = elementwise_blocks(n);
   if (c->es == 8)
-    rescale_to_kernel<float><<<sb, 256, 0, c->stream>>>((float*)c->fld[c->psi_id], n,
-                                                        c->d_scal, c->d_scal + 8);
+    e = launch_overlapped(ov, rescale_to_kernel<float>, sb, 256, 0, c->stream, c->fld[c->psi_id], n,
+                          c->d_scal, c->d_scal + 8);
   else
-    rescale_to_kernel<double><<<sb, 256, 0, c->stream>>>((double*)c->fld[c->psi_id], n,
-                                                         c->d_scal, c->d_scal + 8);
-  CU_CHECK(c, cudaGetLastError());
+    e = launch_overlapped(ov, rescale_to_kernel<double>, sb, 256, 0, c->stream, c->fld[c->psi_id], n,
+                          c->d_scal, c->d_scal + 8);
+  CU_CHECK(c, e);
   c->launches += 3;
   return GPE_OK;
 }
@@ -2642,14 +2716,12 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
     cudaMemset(c->d_time, 0, sizeof(DevTime));
     c->device_bytes += (int64_t)sizeof(DevTime);
   }
-  if (cudaHostAlloc(&c->h_res, sizeof(StepResult), cudaHostAllocMapped | cudaHostAllocPortable) !=
-      cudaSuccess) {
+  c->h_res = take_result();
+  if (!c->h_res) {
     cudaGetLastError();
-    c->h_res = nullptr;
     c->err = "cudaHostAlloc of the step result failed";
     return bail(GPE_ERR_OOM);
   }
-  memset(c->h_res, 0, sizeof(StepResult));
   cudaMemset(c->d_scal, 0, 16 * sizeof(double));
   cudaMemset(c->d_status, 0, sizeof(int));
   if (cudaDeviceSynchronize() != cudaSuccess) {
@@ -2683,7 +2755,7 @@ void gpe_gpu_destroy(gpe_ctx* c) {
   if (c->d_scal) cudaFree(c->d_scal);
   if (c->d_series) cudaFree(c->d_series);
   if (c->d_status) cudaFree(c->d_status);
-  if (c->h_res) cudaFreeHost(c->h_res);
+  give_result(c->h_res);
   if (c->d_stage) cudaFree(c->d_stage);
   rk45_drop_graphs(c);
   if (c->d_time) cudaFree(c->d_time);

@@ -179,6 +179,7 @@ __device__ __forceinline__ void pair_body(const PairParams<T>& p) {
     s_stop = 0;
   }
   __syncthreads();
+  after_previous();
 
   if (warp == NC) {
     // ---------------- producer warp: lane 0 streams the planes -------------

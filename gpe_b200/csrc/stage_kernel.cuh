@@ -221,6 +221,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
     s_stop = 0;
   }
   __syncthreads();
+  after_previous();
 
   if (ty == NW) {
     // ---------------- producer warp: lane 0 streams the planes -------------

@@ -73,3 +73,27 @@ def test_ghosts_follow_whoever_wrote_psi():
                 s.solver()
             out.append(s.get_state(np.complex64))
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("n", [(6, 6, 6), (33, 20, 17), (64, 64, 64), (130, 70, 31)])
+@pytest.mark.parametrize("scheme,order,precision,eqn", [
+    ("euler", 2, 16, 4), ("rk2", 2, 16, 4), ("rk4", 2, 8, 4), ("rk4", 4, 16, 4), ("rk4", 2, 16, 1)])
+def test_overlapped_launches_change_nothing(n, scheme, order, precision, eqn):
+    """Launches whose blocks are set up while the kernel before them ends (off
+    while per-launch timing is on): 200 steps, enqueued together and one by
+    one, give the same bits either way."""
+    kw, st = params(n, scheme, order, 1, precision, False, False, eqn_to_solve=eqn,
+                    Urhs=0.3 if eqn != 4 else 0.0, diss_amp=0.4 if eqn == 1 else 0.0)
+    psi = 1.0 + 0.1 * field(n, seed=sum(n))
+    if precision == 8:
+        psi = psi.astype(np.complex64)
+    out = []
+    for timed in (False, True):
+        with GpeSolver(GpeParams(**kw, **st), dt=1e-4) as s:
+            s.set_timing(timed)
+            s.set_state(psi)
+            s.advance(150)
+            for _ in range(50):
+                s.solver()
+            out.append(s.get_state())
+    assert np.array_equal(*out)
