@@ -567,6 +567,17 @@ constexpr bool occ3_recipe(int np, bool full, bool batch) {
          !batch;
 }
 
+// The recipes that take more than the 112 registers a thread of two CTAs per SM
+// unless told, though ring_shape sizes their rings for two: the last stages of
+// order 4 in complex64 (a stage kernel of 126 registers ran one CTA of a ring
+// meant for two: rk4's last stage at 128^3 35.7 -> 30.7 us, a Kahan step there
+// 80 -> 73).
+template <typename TS, typename TC>
+constexpr bool occ2_recipe(int r, int ns, int np, bool full, bool batch) {
+  return std::is_same<TS, float>::value && std::is_same<TC, float>::value && r == 2 && np >= 3 &&
+         !full && !batch && (110 * 1024 - 128) / (ns * (TX + 4) * 12 * 8 + np * TX * 8 * 8) >= 4;
+}
+
 // The entry of one recipe (only that one is instantiated).
 template <typename TS, typename TC, int R, int NS, int NP, int NOUT, int EPI, int AM, int BM,
           int FORM, bool BATCH>
@@ -577,6 +588,9 @@ KernelFn kernel_for() {
   else if constexpr (occ3_recipe<TS, TC>(NP, FORM == FORM_FULL, BATCH))
     return reinterpret_cast<KernelFn>(
         &stage_kernel_occ3<TS, TC, R, NS, NP, NOUT, EPI, AM, BM, FORM, BATCH>);
+  else if constexpr (occ2_recipe<TS, TC>(R, NS, NP, FORM == FORM_FULL, BATCH))
+    return reinterpret_cast<KernelFn>(
+        &stage_kernel_occ2<TS, TC, R, NS, NP, NOUT, EPI, AM, BM, FORM, BATCH>);
   else
     return reinterpret_cast<KernelFn>(
         &stage_kernel<TS, TC, R, NS, NP, NOUT, EPI, AM, BM, FORM, BATCH>);

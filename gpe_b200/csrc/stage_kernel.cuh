@@ -780,6 +780,14 @@ __global__ void __launch_bounds__(288)
   stage_body<TS, TC, R, NS, NP, NOUT, EPI, AMASK, BMASK, FORM, BATCH>(p);
 }
 
+// Registers capped for two CTAs per SM, where their rings fit (occ2_recipe).
+template <typename TS, typename TC, int R, int NS, int NP, int NOUT, int EPI, int AMASK,
+          int BMASK, int FORM, bool BATCH>
+__global__ void __launch_bounds__(288, 2)
+    stage_kernel_occ2(const __grid_constant__ StageParams<TS, TC> p) {
+  stage_body<TS, TC, R, NS, NP, NOUT, EPI, AMASK, BMASK, FORM, BATCH>(p);
+}
+
 // Registers capped for three resident CTAs per SM: the complex64 recipes
 // that stage only stencil planes, whose warps mostly wait on fixed-latency
 // and shared-memory dependencies, so more warps per scheduler hide more of
