@@ -209,15 +209,32 @@ __global__ void pack_kernel(const TS* __restrict__ src, TO* __restrict__ dst, Ge
   }
 }
 
+// f[q] = op(f[q]) for a whole padded field: 16 bytes a thread and access, four
+// in flight (rows are a multiple of four complexes).  128^3 complex64: 13.4 us one
+// scalar at a time, 8.8 so.
+template <typename TS, typename F>
+__device__ __forceinline__ void for_scalars(TS* __restrict__ f, size_t nscalars, F op) {
+  constexpr int W = 16 / (int)sizeof(TS);
+  struct alignas(16) Vec {
+    TS v[W];
+  };
+  Vec* fv = reinterpret_cast<Vec*>(f);
+  const size_t n = nscalars / W, step = (size_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += step) {
+    Vec a = fv[q];
+#pragma unroll
+    for (int k = 0; k < W; k++) a.v[k] = op(a.v[k]);
+    fv[q] = a;
+  }
+}
+
 // renormalise (src/variables.f90:698-709): f = (sqrt(nn) f) / sqrt(norm)
 // over the whole padded buffer, ghosts included (they stay exact copies).
 template <typename TS>
 __global__ void scale_kernel(TS* __restrict__ f, size_t nscalars, double snn,
                              double sn) {
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < nscalars;
-       q += (size_t)gridDim.x * blockDim.x) {
-    f[q] = (TS)(((double)f[q] * snn) / sn);
-  }
+  for_scalars(f, nscalars, [=](TS v) { return (TS)(((double)v * snn) / sn); });
 }
 
 // The same rescaling with the factor sqrt(target / current) read on the
@@ -228,10 +245,7 @@ __global__ void rescale_to_kernel(TS* __restrict__ f, size_t nscalars,
                                   const double* __restrict__ current) {
   after_previous();
   const double s = sqrt(target[0] / current[0]);
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < nscalars;
-       q += (size_t)gridDim.x * blockDim.x) {
-    f[q] = (TS)((double)f[q] * s);
-  }
+  for_scalars(f, nscalars, [=](TS v) { return (TS)((double)v * s); });
 }
 
 // Weighted |psi|^2 per CTA into partials[2*blk] (get_norm without a stencil).

@@ -179,7 +179,7 @@ int check_view(gpe_cnn* n, const FieldView& v) {
 }
 
 int pack_input(gpe_cnn* n, const FieldView& v, const Act& dst) {
-  CNN_CU(n, launch_overlapped(true, pack_input_kernel<float>, n->Zp * n->Yp, 128, 0, v.stream, v.psi,
+  CNN_CU(n, launch_overlapped(true, pack_input_kernel<float>, (n->Zp * n->Yp + 7) / 8, 256, 0, v.stream, v.psi,
                               v.Nx, v.Ny, n->nx, n->ny, n->nz, dst.p, dst.H));
   n->launches++;
   return GPE_OK;
