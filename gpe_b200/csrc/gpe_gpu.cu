@@ -143,9 +143,10 @@ struct Launch {
 void gpe_internal_set_last_error(const std::string& msg) { g_last_create_error = msg; }
 
 namespace {
-// Page-locked StepResults, 64 to an allocation: page-locking takes some
-// milliseconds, and an ensemble has a context per run.  An allocation goes when
-// its last result is given back.
+// Page-locked StepResults, 64 to an allocation: page-locking takes 3 to 8 ms, as
+// long as the rest of creating a context, and an ensemble has one per run.  An
+// allocation whose last result is given back is freed, but for one (1 KB) that
+// the next context finds.
 struct ResultPages {
   struct Page {
     gpe::StepResult* at;
@@ -162,6 +163,15 @@ gpe::StepResult* take_result() {
   ResultPages& r = result_pages();
   std::lock_guard<std::mutex> lock(r.m);
   gpe::StepResult* at = nullptr;
+  // the kept one is gone if the device was reset meanwhile
+  for (size_t k = r.pages.size(); k-- > 0;) {
+    cudaPointerAttributes a{};
+    if (r.pages[k].used) continue;
+    if (cudaPointerGetAttributes(&a, r.pages[k].at) != cudaSuccess || a.type != cudaMemoryTypeHost) {
+      cudaGetLastError();
+      r.pages.erase(r.pages.begin() + (long)k);
+    }
+  }
   for (auto& p : r.pages)
     for (int i = 0; i < 64 && !at; i++)
       if (!(p.used >> i & 1)) {
@@ -185,7 +195,9 @@ void give_result(gpe::StepResult* at) {
     auto& p = r.pages[k];
     if (at < p.at || at >= p.at + 64) continue;
     p.used &= ~((uint64_t)1 << (at - p.at));
-    if (!p.used) {
+    int empty = 0;
+    for (auto& q : r.pages) empty += !q.used;
+    if (!p.used && empty > 1) {
       cudaFreeHost(p.at);
       r.pages.erase(r.pages.begin() + (long)k);
     }
@@ -2207,10 +2219,10 @@ int gpe_internal_restore_norm(gpe_ctx* c) {
 
 // ==========================================================================
 // Batched ensembles: independent runs of uneven grids stepped by one
-// persistent launch per RK4 stage.  Each member is a full context (fields,
+// persistent launch per pair of RK4 stages (or stage).  Each member is a full context (fields,
 // tables, tensor maps); the batch adds one work list of (run, tile, z-range)
 // items for all members, per-stage arrays of their RunDescs in device memory,
-// and a CUDA graph of one whole step (4 stage launches + per-run norm).
+// and a CUDA graph of one whole step (launches, ghosts, per-run norm).
 
 struct gpe_batch {
   int dev = 0;
