@@ -3,9 +3,9 @@
 The reference runs one grid per job (src/gpe.f90).  A parameter scan of
 trap frequencies, interaction strengths or grid sizes is then a queue of
 small jobs, each too small to fill the GPU.  GpeBatch holds all of them
-resident and steps them together: every rk4 stage is one persistent launch
-whose CTAs walk a shared work list of (run, tile, z-range) items, largest
-first, and one whole step is replayed from a CUDA graph
+resident and steps them together: two rk4 stages (one, where a member's
+right-hand side has no pair) are one persistent launch whose CTAs walk shares
+of a work list of (run, tile, z-range) items, and one whole step is replayed from a CUDA graph
 (include/gpe_gpu.h, gpe_batch_*).  Members are ordinary contexts: each one's
 state, norm and energy are read through GpeSolver's methods.
 """
@@ -23,8 +23,8 @@ from .solver import GpeParams, GpeSolver
 
 @dataclass
 class BatchOpts:
-    tile_y: int = 0        # 0 = auto (8); else 4 or 8
-    zchunk: int = 0        # 0 = auto (min(nz, 64)) planes per work item
+    tile_y: int = 0        # 0 = the tallest built (8, or 16 in complex64 pairs); else 4 or 8
+    zchunk: int = 0        # 0 = auto (an equal share per CTA) planes per work item
     ctas_per_sm: int = 0   # 0 = as many as fit
     use_graph: bool = True
 

@@ -40,8 +40,15 @@
 // antisymmetric term, the x gradient, takes the mirrored sign).  Equation 3's
 // sphere mask has no pair kernel.
 //
-// What bounds it: at order 4 in complex64 the L1 data pipe and DRAM about
-// equally (16-row tiles: 1.33 first-stage sites per site, 24 KB planes).
+// What bounds it, at 512^3 in complex64, order 4, compensated: pair A (0.895 ms,
+// 24 B/site: 0.55 of the copy rate) the L1 data pipe, 86% busy, with 1.33
+// first-stage sites per site; pair B (1.44 ms, 48 B/site: 0.68) the latency of
+// its planes, of which shared memory holds four, one in flight.  DRAM carries the
+// bytes counted above and no more.  complex128 is bound by the registers: 12 warps
+// of 168.  A step of rk4, one stage per launch -> in pairs, ghosts and norm
+// included: 512^3 complex64 compensated order 4 2930 -> 2430 us; 256^3 the same
+// 477 -> 351, at order 2 409 -> 278; 256^3 complex128 order 4 1163 -> 737, order 2
+// 813 -> 454; 64^3 complex128 order 2 41 -> 30 (24 with overlapped launches).
 #pragma once
 
 #include "device_utils.cuh"
@@ -72,8 +79,8 @@ struct PairTile<double> {
 
 // Ring positions in units of one row of 32 site pairs: R rows below, R above,
 // and one unit for the pairs left and right of the tile's rows; two units per
-// ring warp (with the producer that makes 12 warps at R = 2, three per
-// scheduler, which leaves each 168 registers).
+// ring warp (at R = 2, with the producer, 20 warps of 96 registers in complex64
+// and 12 of 168, three per scheduler, in complex128).
 constexpr int RING_UNITS = 2;
 __host__ __device__ constexpr int pair_ring_warps(int r) { return (2 * r + 1 + RING_UNITS - 1) / RING_UNITS; }
 template <typename T>
