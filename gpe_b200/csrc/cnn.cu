@@ -130,7 +130,7 @@ int launch_conv(gpe_cnn* n, cudaStream_t st, const Act& in, int layer, bool dgra
   const size_t smem = 1024 + (size_t)FSLOTS * p.slot_bytes + 4096 +
                       W_TILES * OutShape<CO>::WTB + F_TAIL_BYTES;
   auto fn = conv_fwd_kernel<EPI, CO>;
-  CNN_CU(n, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CNN_CU(n, allow_dynamic_smem(reinterpret_cast<const void*>(fn)));
   const int grid = std::min(p.nitems, n->num_sms);
   CNN_CU(n, launch_overlapped(true, fn, grid, F_THREADS, smem, st, p));
   n->launches++;
@@ -161,8 +161,7 @@ int launch_wgrad(gpe_cnn* n, cudaStream_t st, const Act& x, const Act& dy) {
   const size_t ring = std::max((size_t)WSLOTS * p.xslot_bytes, (size_t)XROWS * 3 * 256 * 4);
   const size_t smem = 1024 + ring + (size_t)DSLOTS * p.dslot_bytes +
                       (2 * WSLOTS + 2 * DSLOTS + 1) * 8 + 16 + 4 * 8 * 4 + 16;
-  CNN_CU(n, cudaFuncSetAttribute(conv_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  CNN_CU(n, allow_dynamic_smem(reinterpret_cast<const void*>(&conv_wgrad_kernel)));
   CNN_CU(n, launch_overlapped(true, conv_wgrad_kernel, n->wgrad_grid, W_THREADS, smem, st, p));
   n->launches++;
   return GPE_OK;

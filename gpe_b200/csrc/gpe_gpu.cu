@@ -539,8 +539,7 @@ int choose_shape(gpe_ctx* c, KernelFn fn, int R, int np, int ns, bool occ3, Laun
   s.rows = (occ3 && ns == 2) ? 2 : 1;  // rows_per_warp of the occ3 recipes
   s.ntx = (c->nx + TX - 1) / TX;
   s.nty = (c->ny + s.TY - 1) / s.TY;
-  CU_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)s.smem));
+  CU_CHECK(c, allow_dynamic_smem(fn));
   int occ = 0;
   CU_CHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 32 * (s.TY / s.rows + 1),
                                                             s.smem));
@@ -1291,7 +1290,7 @@ int pair_shape(gpe_ctx* c, KernelFn fn, int R, const PairSpec& sp, int tile_y, P
   s.d_ring = s.u_ring + U_SLOTS * s.u_stride;
   s.smem = s.d_ring + d_bytes;
   s.threads_y = pair_warps<T>(R, s.TY) + 1;
-  CU_CHECK(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem));
+  CU_CHECK(c, allow_dynamic_smem(fn));
   CU_CHECK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s.occ, fn, 32 * s.threads_y, s.smem));
   if (s.occ < 1) return fail(c, GPE_ERR_INVALID, "pair kernel cannot be resident");
   *out = s;
@@ -2306,7 +2305,7 @@ int batch_prepare_par(gpe_batch* b, cd dt, int par) {
     // two-row recipes: rings for three CTAs per SM, as their registers allow
     LaunchShape sh = ring_shape(b->es, b->R, sp.np, b->TY, ns, rows == 2 ? 3 : 2);
     sh.rows = rows;
-    BCU(b, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+    BCU(b, allow_dynamic_smem(fn));
     int occ = 0;
     BCU(b, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 32 * (sh.TY / sh.rows + 1),
                                                          sh.smem));

@@ -28,6 +28,21 @@ struct FieldView {
   void* stage;        // dense staging buffer, nx ny nz elements of 16 bytes
 };
 
+// Lets every launch of fn take as much dynamic shared memory as a block may
+// have.  The limit is the function's, shared by all contexts, threads and
+// launches of the process, while what a launch needs depends on its grid: a
+// limit set to one launch's need would refuse a larger one of another context.
+// One read of the attributes where the limit is there already.
+inline cudaError_t allow_dynamic_smem(const void* fn) {
+  constexpr int BLOCK_SMEM = 227 * 1024;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, fn);
+  if (e != cudaSuccess) return e;
+  const int most = BLOCK_SMEM - (int)a.sharedSizeBytes;
+  if (a.maxDynamicSharedSizeBytes >= most) return cudaSuccess;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // Launches fn, which begins with after_previous(), so that its blocks are set
 // up while the kernel before it in the stream ends (programmatic dependent
 // launch).  Where kernels last some microseconds the gap between two of them

@@ -177,8 +177,7 @@ int exec(gpe_ctx* c, Spectral* s, const FieldView& v, int dir) {
 template <typename T, int E>
 int launch_spectrum(gpe_ctx* c, Spectral* s, const FieldView& v, const SpecArgs& a,
                     const SpecFinal& f0, size_t smem, int64_t sites) {
-  SP_CU(c, cudaFuncSetAttribute(spectrum_kernel<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
+  SP_CU(c, allow_dynamic_smem(reinterpret_cast<const void*>(&spectrum_kernel<T, E>)));
   int per_sm = 1, sms = 148;
   SP_CU(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spectrum_kernel<T, E>, S_THREADS,
                                                          smem));

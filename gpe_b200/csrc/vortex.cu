@@ -68,8 +68,7 @@ int run(gpe_ctx* c, const FieldView& v, const void* field, bool dense, double* l
   }
   int sms = 148, per_sm = 1;
   VX_CU(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, v.dev));
-  VX_CU(c, cudaFuncSetAttribute(line_cells_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
+  VX_CU(c, allow_dynamic_smem(reinterpret_cast<const void*>(&line_cells_kernel<T>)));
   VX_CU(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_cells_kernel<T>,
                                                          L_THREADS, smem));
   // two waves of resident blocks, each block whole rows in loop order
