@@ -84,7 +84,7 @@ __global__ void unpack_kernel(const TI* __restrict__ src, TS* __restrict__ dst, 
 // warp; of the interior rows four per warp, eight lanes each, copy the
 // x ghosts.
 template <typename TS>
-__device__ __forceinline__ void fill_ghost_rows(TS* __restrict__ f, const Geom& g, int depth,
+__device__ __forceinline__ void fill_ghost_rows(TS* f, const Geom& g, int depth,
                                                 int block, int nblocks) {
   using V = typename VT<TS>::T;
   V* F = reinterpret_cast<V*>(f);
@@ -135,14 +135,14 @@ __device__ __forceinline__ void fill_ghost_rows(TS* __restrict__ f, const Geom& 
 }
 
 template <typename TS>
-__global__ void fill_ghosts_kernel(TS* __restrict__ f, Geom g, int depth) {
+__global__ void fill_ghosts_kernel(TS* f, Geom g, int depth) {
   after_previous();
   fill_ghost_rows<TS>(f, g, depth, blockIdx.x, gridDim.x);
 }
 
 // Fixed-order reduction of slot `slot` of the per-CTA partials by one block
 // (sum, or max for op 1); the result is s[0] for every thread on return.
-__device__ __forceinline__ void reduce_partials(const double* __restrict__ partials, int nblk,
+__device__ __forceinline__ void reduce_partials(const double* partials, int nblk,
                                                 int slot, int op, double* s) {
   double a = 0.0;
   for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
@@ -163,13 +163,11 @@ __device__ __forceinline__ void reduce_partials(const double* __restrict__ parti
 // The end of a step in pairs, blocks of 1024 threads: block 0 reduces the norm
 // as finalize_kernel does, the others fill the new psi's ghosts.
 template <typename TS>
-__global__ void __launch_bounds__(1024) ghosts_norm_kernel(TS* __restrict__ f, Geom g, int depth,
-                                                            const double* __restrict__ partials,
-                                                            int nblk, double scale,
-                                                            double* __restrict__ out,
-                                                            double* __restrict__ series,
-                                                            StepResult* res,
-                                                            const int* __restrict__ status) {
+__global__ void __launch_bounds__(1024) ghosts_norm_kernel(TS* f, Geom g, int depth,
+                                                            const double* partials, int nblk,
+                                                            double scale, double* out,
+                                                            double* series, StepResult* res,
+                                                            const int* status) {
   __shared__ double s[1024];
   after_previous();
   if (blockIdx.x > 0) {
@@ -213,7 +211,7 @@ __global__ void pack_kernel(const TS* __restrict__ src, TO* __restrict__ dst, Ge
 // in flight (rows are a multiple of four complexes).  128^3 complex64: 13.4 us one
 // scalar at a time, 8.8 so.
 template <typename TS, typename F>
-__device__ __forceinline__ void for_scalars(TS* __restrict__ f, size_t nscalars, F op) {
+__device__ __forceinline__ void for_scalars(TS* f, size_t nscalars, F op) {
   constexpr int W = 16 / (int)sizeof(TS);
   struct alignas(16) Vec {
     TS v[W];
@@ -240,9 +238,8 @@ __global__ void scale_kernel(TS* __restrict__ f, size_t nscalars, double snn,
 // The same rescaling with the factor sqrt(target / current) read on the
 // device (both norms left in device memory by earlier reductions).
 template <typename TS>
-__global__ void rescale_to_kernel(TS* __restrict__ f, size_t nscalars,
-                                  const double* __restrict__ target,
-                                  const double* __restrict__ current) {
+__global__ void rescale_to_kernel(TS* f, size_t nscalars, const double* target,
+                                  const double* current) {
   after_previous();
   const double s = sqrt(target[0] / current[0]);
   for_scalars(f, nscalars, [=](TS v) { return (TS)((double)v * s); });
@@ -250,11 +247,9 @@ __global__ void rescale_to_kernel(TS* __restrict__ f, size_t nscalars,
 
 // Weighted |psi|^2 per CTA into partials[2*blk] (get_norm without a stencil).
 template <typename TS>
-__global__ void norm_kernel(const TS* __restrict__ f, Geom g,
-                            const double* __restrict__ wx,
-                            const double* __restrict__ wy,
-                            const double* __restrict__ wz,
-                            double* __restrict__ partials) {
+__global__ void norm_kernel(const TS* f, Geom g, const double* __restrict__ wx,
+                            const double* __restrict__ wy, const double* __restrict__ wz,
+                            double* partials) {
   __shared__ double s[32];
   const int lane = threadIdx.x & 31;
   double acc = 0.0;
@@ -285,11 +280,9 @@ __global__ void norm_kernel(const TS* __restrict__ f, Geom g,
 // Fixed-order reduction of partials[2*b + slot], b < nblk, by one CTA of
 // 1024 threads.  op 0 = sum, 1 = max.  out[0] = result * scale, written to
 // *series too when it is non-null, and with the status word to *res.
-__global__ void finalize_kernel(const double* __restrict__ partials, int nblk,
-                                int slot, int op, double scale,
-                                double* __restrict__ out,
-                                double* __restrict__ series, StepResult* res,
-                                const int* __restrict__ status) {
+__global__ void finalize_kernel(const double* partials, int nblk, int slot, int op,
+                                double scale, double* out, double* series, StepResult* res,
+                                const int* status) {
   __shared__ double s[1024];
   after_previous();
   reduce_partials(partials, nblk, slot, op, s);

@@ -862,8 +862,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
 // four records a lane in flight; bound by the 16 (or 32) bytes written per site
 // (128^3: 12.2 us with a block of 128 threads per row of 130, 11.1 so).
 template <typename TS>
-__global__ void pack_input_kernel(const TS* __restrict__ psi, int Nx, int Ny, int nx, int ny,
-                                  int nz, __nv_bfloat16* __restrict__ act, int H) {
+__global__ void pack_input_kernel(const TS* psi, int Nx, int Ny, int nx, int ny, int nz,
+                                  __nv_bfloat16* act, int H) {
   const int Xp = nx + 2, Yp = ny + 2, rows = Yp * (nz + 2);
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const uint4 zero = make_uint4(0, 0, 0, 0);
@@ -875,11 +875,20 @@ __global__ void pack_input_kernel(const TS* __restrict__ psi, int Nx, int Ny, in
     const int z = zp == 0 ? nz - 1 : (zp == nz + 1 ? 0 : zp - 1);
     const V* src = reinterpret_cast<const V*>(psi) + ((size_t)(z + GH) * Ny + (y + GH)) * Nx + GH;
     uint4* dst = reinterpret_cast<uint4*>(act) + (size_t)row * H * Xp;
-#pragma unroll 4
-    for (int xp = lane; xp < Xp; xp += 32) {
-      const V v = src[xp == 0 ? nx - 1 : (xp == nx + 1 ? 0 : xp - 1)];
-      dst[xp] = make_uint4(pack_bf16x2((float)v.x, (float)v.y), 0, 0, 0);
-      if (H == 2) dst[Xp + xp] = zero;
+    for (int x0 = lane; x0 < Xp; x0 += 128) {
+      V v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int xp = x0 + 32 * q;
+        if (xp < Xp) v[q] = src[xp == 0 ? nx - 1 : (xp == nx + 1 ? 0 : xp - 1)];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int xp = x0 + 32 * q;
+        if (xp >= Xp) break;
+        dst[xp] = make_uint4(pack_bf16x2((float)v[q].x, (float)v[q].y), 0, 0, 0);
+        if (H == 2) dst[Xp + xp] = zero;
+      }
     }
   }
 }
@@ -888,10 +897,9 @@ __global__ void pack_input_kernel(const TS* __restrict__ psi, int Nx, int Ny, in
 // layer's output: e = u + delta - target, loss = sum |e|^2 / n,
 // dL/d(out_c) = 2 e_c out_scale / n into channels 0, 1 of g (others 0).
 template <typename TS, typename TT>
-__global__ void loss_kernel(const float* __restrict__ delta, const TS* __restrict__ u, int Nx,
-                            int Ny, const TT* __restrict__ target, int nx, int ny, int nz,
-                            float out_scale, __nv_bfloat16* __restrict__ g,
-                            double* __restrict__ partials) {
+__global__ void loss_kernel(const float* delta, const TS* u, int Nx, int Ny, const TT* target,
+                            int nx, int ny, int nz, float out_scale, __nv_bfloat16* g,
+                            double* partials) {
   __shared__ double red[32];
   const int Xp = nx + 2, Yp = ny + 2;
   const size_t n = (size_t)nx * ny * nz;
@@ -925,11 +933,9 @@ __global__ void loss_kernel(const float* __restrict__ delta, const TS* __restric
 // dW[tap][co][ci] (fp32) of one layer from the wgrad partials (one block per
 // tap; four groups of threads take every fourth CTA of the tap's role, added in
 // a fixed order), and db from the channel sums (the last block).
-__global__ void __launch_bounds__(1024) grad_finalize_kernel(const float* __restrict__ wpart, int nblk,
-                                                              int role0,
-                                                              const float* __restrict__ bpart,
-                                                              float* __restrict__ dw,
-                                                              float* __restrict__ db) {
+__global__ void __launch_bounds__(1024) grad_finalize_kernel(const float* wpart, int nblk,
+                                                              int role0, const float* bpart,
+                                                              float* dw, float* db) {
   __shared__ float s[4][256];
   const int c = threadIdx.x & 255, g = threadIdx.x >> 8;
   after_previous();

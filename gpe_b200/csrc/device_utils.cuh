@@ -63,8 +63,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // thread: waits until the kernel before it has completed and its memory is
 // visible, and lets the kernel behind it set up its blocks in turn.  In this
 // order: a trigger before the wait would let a third kernel start while the first
-// still runs, and its wait covers the second only (batched steps read stale
-// ghosts then).  Without the launch attribute both are no-ops.
+// still runs, and its wait covers the second only (steps then read ghosts that
+// are not filled yet).  Without the launch attribute both are no-ops.
+// Such a kernel runs while the one before it still writes, so no pointer it is
+// given to memory of the step (read or written) is __restrict__: the qualifier
+// lets the compiler take a load for invariant and move it above this wait, which
+// a memory clobber does not forbid.  Only tables that are constant since the
+// context was created keep it.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
