@@ -476,14 +476,40 @@ __global__ void wait_probe_kernel(unsigned long long limit_ns, int* status) {
   if (threadIdx.x == 0 && !mbar_wait_bounded(&bar, 0, limit_ns)) atomicExch(status, 1);
 }
 
+// A sum held as an unevaluated pair, about 106 bits: add() by Knuth's two-sum.
+// hi alone is the plain sum, so an infinity or NaN shows there as it would.
+struct Sum2 {
+  double hi, lo;
+  __device__ __forceinline__ double value() const { return isfinite(hi) ? hi + lo : hi; }
+  __device__ __forceinline__ void add(double x) {
+    const double s = hi + x, b = s - hi;
+    lo += (hi - (s - b)) + (x - b);
+    hi = s;
+  }
+  __device__ __forceinline__ void add(const Sum2& o) {
+    add(o.hi);
+    lo += o.lo;
+  }
+};
+
 // mass (src/variables.f90:590-610) and momentum (:615-694) in one pass:
-// per block, [4] partials = { sum |psi|^2, and for d = x, y, z the weighted
-// sum of (Re psi - 1) Im(d conj psi) - Im psi Re(d psi) }.  First
+// per block, [8] partials = (hi, lo) of { sum |psi|^2, and for d = x, y, z the
+// weighted sum of (Re psi - 1) Im(d conj psi) - Im psi Re(d psi) }.  First
 // derivatives use the face ghosts: c1 (f+1 - f-1) + c2 (f+2 - f-2).
 // A block owns 32 x 8 sites in (x, y) and marches a chunk of z: the z
 // neighbours come from a register queue, the x and y ones from L1, so DRAM is
 // read about once.  Bound by FP64 and L1 (256^3 complex128: 296 us with every
 // neighbour fetched by its own 64-bit index).
+// Neighbouring sites carry momentum of one sign, so the partial sums of a block
+// are far larger than the total they cancel to, and rounding them costs digits
+// that scattered sites did not (momentum at 256^3: 2.5e-15 of its largest
+// component against 1.5e-15): a thread adds DIAG_RUN planes plainly, and from
+// there on every sum is a Sum2 (3.7e-16).  256^3, plain sums -> these: complex128
+// 144 -> 129 us, complex64 137 both; three blocks per SM, unrolled by two in
+// complex128 only (without the cap 126 registers and 191 us; complex64 unrolled
+// 150).
+constexpr int DIAG_RUN = 8;
+constexpr int DIAG_PARTIALS = 8;  // doubles a block
 struct DiagArgs {
   Geom g;
   double c1[3], c2[3];
@@ -491,11 +517,12 @@ struct DiagArgs {
   int tx, ty, zchunk;  // tiles in x and y, planes per block
 };
 template <typename TS, bool FOURTH>
-__global__ void __launch_bounds__(256) diag_kernel(const TS* __restrict__ f, DiagArgs p,
-                                                    double* __restrict__ partials) {
+__global__ void __launch_bounds__(256, 3) diag_kernel(const TS* __restrict__ f,
+                                                       DiagArgs p,
+                                                       double* __restrict__ partials) {
   using V = typename VT<TS>::T;
-  __shared__ double red[4][8];
-  constexpr int R = FOURTH ? 2 : 1;
+  __shared__ Sum2 red[4][8];
+  constexpr int R = FOURTH ? 2 : 1, UNROLL = sizeof(TS) == 8 ? 2 : 1;
   const V* F = reinterpret_cast<const V*>(f);
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   const int tile = blockIdx.x % (p.tx * p.ty), chunk = blockIdx.x / (p.tx * p.ty);
@@ -503,14 +530,15 @@ __global__ void __launch_bounds__(256) diag_kernel(const TS* __restrict__ f, Dia
   const int z0 = chunk * p.zchunk, z1 = min(z0 + p.zchunk, p.g.nz);
   const int sy = p.g.Nx;
   const size_t sz = (size_t)p.g.Nx * p.g.Ny;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  Sum2 sum[4] = {};
   if (i < p.g.nx && j < p.g.ny) {
     const double wxy = p.w[0][i] * p.w[1][j];
     const V* c = F + padded_index(p.g, i, j, z0);
     V q[2 * R + 1];  // planes z - R .. z + R
 #pragma unroll
     for (int d = 0; d < 2 * R; d++) q[d] = *(c + (ptrdiff_t)(d - R) * (ptrdiff_t)sz);
-#pragma unroll 2
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll UNROLL
     for (int z = z0; z < z1; z++, c += sz) {
       q[2 * R] = c[(size_t)R * sz];
       const double re = (double)q[R].x, im = (double)q[R].y;
@@ -542,37 +570,49 @@ __global__ void __launch_bounds__(256) diag_kernel(const TS* __restrict__ f, Dia
       }
 #pragma unroll
       for (int d = 0; d < 2 * R; d++) q[d] = q[d + 1];
+      if (((z - z0) & (DIAG_RUN - 1)) == DIAG_RUN - 1 || z == z1 - 1)
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+          sum[v].add(acc[v]);
+          acc[v] = 0.0;
+        }
     }
   }
 #pragma unroll
   for (int v = 0; v < 4; v++) {
-    const double t = warp_sum(acc[v]);
+    Sum2 t = sum[v];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      t.add(Sum2{__shfl_down_sync(0xffffffffu, t.hi, o), __shfl_down_sync(0xffffffffu, t.lo, o)});
     if (lane == 0) red[v][row] = t;
   }
   __syncthreads();
   if (threadIdx.x < 4) {
-    double t = 0.0;
-    for (int w = 0; w < 8; w++) t += red[threadIdx.x][w];
-    partials[4 * (size_t)blockIdx.x + threadIdx.x] = t;
+    Sum2 t = red[threadIdx.x][0];
+    for (int w = 1; w < 8; w++) t.add(red[threadIdx.x][w]);
+    double* out = partials + (size_t)DIAG_PARTIALS * blockIdx.x + 2 * threadIdx.x;
+    out[0] = t.hi;
+    out[1] = t.lo;
   }
 }
 
-// [nblk][4] partials -> out[0..3] * scale, fixed order (one CTA of 1024).
+// [nblk][4] pairs -> out[0..3] * scale, fixed order (one CTA of 1024).
 __global__ void __launch_bounds__(1024) diag_finalize_kernel(const double* __restrict__ partials,
                                                               int nblk, double scale,
                                                               double* __restrict__ out) {
-  __shared__ double s[1024];
+  __shared__ Sum2 s[1024];
   // value v of blocks b, b + 256, ...: thread 4 b + v, so loads are contiguous
-  double a = 0.0;
+  Sum2 a = {};
 #pragma unroll 4
-  for (int q = threadIdx.x; q < 4 * nblk; q += 1024) a += partials[q];
+  for (int q = threadIdx.x; q < 4 * nblk; q += 1024)
+    a.add(Sum2{partials[2 * q], partials[2 * q + 1]});
   s[threadIdx.x] = a;
   __syncthreads();
   for (int w = 512; w >= 4; w >>= 1) {
-    if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
+    if ((int)threadIdx.x < w) s[threadIdx.x].add(s[threadIdx.x + w]);
     __syncthreads();
   }
-  if (threadIdx.x < 4) out[threadIdx.x] = s[threadIdx.x] * scale;
+  if (threadIdx.x < 4) out[threadIdx.x] = s[threadIdx.x].value() * scale;
 }
 
 }  // namespace gpe

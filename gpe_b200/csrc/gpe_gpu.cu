@@ -3111,13 +3111,14 @@ int gpe_gpu_diagnostics(gpe_ctx* c, double* mass, double* mom) {
   }
   d.tx = (c->nx + 31) / 32;
   d.ty = (c->ny + 7) / 8;
-  // about eight blocks of 256 per SM, four partials each
+  // about eight blocks of 256 per SM
   const int tiles = d.tx * d.ty;
-  const int room = (int)std::min<size_t>(c->partials_cap / 2 / tiles, (size_t)c->nz);
+  const size_t cap = 2 * c->partials_cap / DIAG_PARTIALS;
+  const int room = (int)std::min<size_t>(cap / tiles, (size_t)c->nz);
   const int chunks = std::max(1, std::min(room, (8 * c->num_sms + tiles - 1) / tiles));
   d.zchunk = (c->nz + chunks - 1) / chunks;
   const int nb = tiles * ((c->nz + d.zchunk - 1) / d.zchunk);
-  if ((size_t)nb * 2 > c->partials_cap) return fail(c, GPE_ERR_INVALID, "partials buffer too small");
+  if ((size_t)nb > cap) return fail(c, GPE_ERR_INVALID, "partials buffer too small");
   const bool fourth = c->prm.order == 4;
   if (c->es == 8) {
     if (fourth) diag_kernel<float, true><<<nb, 256, 0, c->stream>>>((const float*)c->fld[c->psi_id], d, c->d_partials);

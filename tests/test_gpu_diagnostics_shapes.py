@@ -49,3 +49,41 @@ def test_mass_and_momentum_tiles(n, order, precision):
     assert m == pytest.approx(o.mass(psi), rel=1e-12)
     # the signed sums are bounded by their terms' magnitudes, about mass / h
     assert np.abs(mom - exp).max() <= 1e-12 * m / 0.5
+
+
+def odd_near(rng, top, shape):
+    """Odd integers of 2^top plus a few thousands."""
+    return 2 ** top + 2 * rng.integers(0, 2000, size=shape) + 1
+
+
+def total(terms):
+    """The exact sum of an int64 array below 2^62, as a Python integer."""
+    return (int((terms >> 24).sum()) << 24) + int((terms & (2 ** 24 - 1)).sum())
+
+
+@pytest.mark.parametrize("n", [(40, 20, 24), (640, 150, 60)])
+def test_mass_and_momentum_of_integers_are_exact(n):
+    """Fields of integers, whose terms and whose sums over eight planes are
+    exact in 64 bits (below 2^52) while the sums of a block are not (2^56 and
+    more): the totals are the correctly rounded ones, times dx dy dz = 1/8.  The
+    second grid has more than two runs of planes to a block."""
+    rng = np.random.default_rng(n[0])
+    shape = n[::-1]
+    with solver(n) as s:
+        a, b = odd_near(rng, 23, shape), odd_near(rng, 23, shape)
+        s.set_state(a + 1j * b)
+        mass, _ = s.diagnostics()
+        assert mass == float(total(a * a + b * b)) * 0.125
+        # psi = 1 in the outer layers, whose weights are no integers: no term there
+        inner = np.zeros(shape, dtype=bool)
+        inner[3:-3, 3:-3, 3:-3] = True
+        for axis in range(3):
+            x = np.moveaxis(np.broadcast_to(np.arange(shape[axis]), np.moveaxis(a, axis, -1).shape), -1, axis)
+            re1 = np.where(inner, odd_near(rng, 23, shape), 0)
+            im = np.where(inner, odd_near(rng, 22, shape) * (x % 4), 0)
+            s.set_state((re1 + 1) + 1j * im)
+            _, mom = s.diagnostics()
+            # h = 1/2: a first derivative is the difference of the two neighbours
+            di = np.roll(im, -1, axis) - np.roll(im, 1, axis)
+            dr = np.roll(re1, -1, axis) - np.roll(re1, 1, axis)
+            assert mom[2 - axis] == float(total(-re1 * di - im * dr)) * 0.125
