@@ -353,9 +353,9 @@ struct SpecFinal {
 constexpr int F_FIN_THREADS = 1024;
 
 // Sums of the block partials per column: a block takes 32 columns, its lanes
-// lie over them and its warps over the blocks' rows, then a fixed order over
-// the warps.  (One block for all columns, lanes over rows, read every value
-// from its own sector: 51 us for 592 rows of 144.)
+// lie over them and its warps over the blocks' rows; then each warp adds one
+// column's 32 sums as a tree.  (One block for all columns, lanes over rows, read
+// every value from its own sector: 51 us for 592 rows of 144.)
 __global__ void __launch_bounds__(F_FIN_THREADS) spectrum_columns_kernel(
     const double* __restrict__ partials, int nblk, int ncol, double* __restrict__ cols) {
   __shared__ double s[32][33];
@@ -367,12 +367,10 @@ __global__ void __launch_bounds__(F_FIN_THREADS) spectrum_columns_kernel(
     for (int b = warp; b < nblk; b += 32) x += partials[(size_t)b * ncol + c];
   s[warp][lane] = x;
   __syncthreads();
-  if (warp == 0 && c < ncol) {
-    double t = 0.0;
+  x = s[lane][warp];
 #pragma unroll
-    for (int w = 0; w < 32; w++) t += s[w][lane];
-    cols[c] = t;
-  }
+  for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(0xffffffffu, x, d);
+  if (lane == 0 && blockIdx.x * 32 + warp < ncol) cols[blockIdx.x * 32 + warp] = x;
 }
 
 // From the column sums the mass.dat row (src/io.f90:369-382), eta =
