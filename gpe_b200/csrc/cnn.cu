@@ -110,7 +110,7 @@ void conv_items(const gpe_cnn* n, int rows, int* nslab, int* nzc, int* zchunk) {
 }
 
 template <int EPI>
-int launch_conv(gpe_cnn* n, cudaStream_t st, const Act& in, int layer, bool dgrad,
+int launch_conv(gpe_cnn* n, const FieldView& v, const Act& in, int layer, bool dgrad,
                 ConvParams& p) {
   // the last layer's 2 output channels use the N = 32 kernel
   constexpr int CO = (EPI == EPI_RESID || EPI == EPI_DELTA) ? 2 : 16;
@@ -132,7 +132,7 @@ int launch_conv(gpe_cnn* n, cudaStream_t st, const Act& in, int layer, bool dgra
   auto fn = conv_fwd_kernel<EPI, CO>;
   CNN_CU(n, allow_dynamic_smem(reinterpret_cast<const void*>(fn)));
   const int grid = std::min(p.nitems, n->num_sms);
-  CNN_CU(n, launch_overlapped(true, fn, grid, F_THREADS, smem, st, p));
+  CNN_CU(n, launch_overlapped(v.overlap, fn, grid, F_THREADS, smem, v.stream, p));
   n->launches++;
   return GPE_OK;
 }
@@ -142,7 +142,7 @@ int wgrad_role0(const gpe_cnn* n) {
   return std::max(1, std::min(n->wgrad_grid - 1, (n->wgrad_grid * W_TAPS0 + 4) / 9));
 }
 
-int launch_wgrad(gpe_cnn* n, cudaStream_t st, const Act& x, const Act& dy) {
+int launch_wgrad(gpe_cnn* n, const FieldView& v, const Act& x, const Act& dy) {
   WgradParams p;
   memset(&p, 0, sizeof(p));
   p.x = x.p;
@@ -162,7 +162,7 @@ int launch_wgrad(gpe_cnn* n, cudaStream_t st, const Act& x, const Act& dy) {
   const size_t smem = 1024 + ring + (size_t)DSLOTS * p.dslot_bytes +
                       (2 * WSLOTS + 2 * DSLOTS + 1) * 8 + 16 + 4 * 8 * 4 + 16;
   CNN_CU(n, allow_dynamic_smem(reinterpret_cast<const void*>(&conv_wgrad_kernel)));
-  CNN_CU(n, launch_overlapped(true, conv_wgrad_kernel, n->wgrad_grid, W_THREADS, smem, st, p));
+  CNN_CU(n, launch_overlapped(v.overlap, conv_wgrad_kernel, n->wgrad_grid, W_THREADS, smem, v.stream, p));
   n->launches++;
   return GPE_OK;
 }
@@ -178,8 +178,8 @@ int check_view(gpe_cnn* n, const FieldView& v) {
 }
 
 int pack_input(gpe_cnn* n, const FieldView& v, const Act& dst) {
-  CNN_CU(n, launch_overlapped(true, pack_input_kernel<float>, (n->Zp * n->Yp + 7) / 8, 256, 0, v.stream, v.psi,
-                              v.Nx, v.Ny, n->nx, n->ny, n->nz, dst.p, dst.H));
+  CNN_CU(n, launch_overlapped(v.overlap, pack_input_kernel<float>, (n->Zp * n->Yp + 7) / 8, 256, 0,
+                              v.stream, v.psi, v.Nx, v.Ny, n->nx, n->ny, n->nz, dst.p, dst.H));
   n->launches++;
   return GPE_OK;
 }
@@ -205,21 +205,21 @@ int enqueue_apply(gpe_cnn* n, const FieldView& v, int* status) {
   memset(&p, 0, sizeof(p));
   p.status = status;
   p.act_out = n->A1.p;
-  if ((rc = launch_conv<EPI_GELU>(n, v.stream, n->A0, 0, false, p))) return rc;
+  if ((rc = launch_conv<EPI_GELU>(n, v, n->A0, 0, false, p))) return rc;
   memset(&p, 0, sizeof(p));
   p.status = status;
   p.act_out = n->A2.p;
-  if ((rc = launch_conv<EPI_GELU>(n, v.stream, n->A1, 1, false, p))) return rc;
+  if ((rc = launch_conv<EPI_GELU>(n, v, n->A1, 1, false, p))) return rc;
   memset(&p, 0, sizeof(p));
   p.status = status;
   p.act_out = n->A1.p;
-  if ((rc = launch_conv<EPI_GELU>(n, v.stream, n->A2, 2, false, p))) return rc;
+  if ((rc = launch_conv<EPI_GELU>(n, v, n->A2, 2, false, p))) return rc;
   memset(&p, 0, sizeof(p));
   p.status = status;
   p.psi = static_cast<float*>(v.psi);
   p.psi_Nx = v.Nx;
   p.psi_Ny = v.Ny;
-  return launch_conv<EPI_RESID>(n, v.stream, n->A1, 3, false, p);
+  return launch_conv<EPI_RESID>(n, v, n->A1, 3, false, p);
 }
 
 int post_step_hook(void* arg, gpe_ctx* c) {
@@ -240,30 +240,30 @@ int enqueue_train_forward(gpe_cnn* n, const FieldView& v) {
     memset(&p, 0, sizeof(p));
     p.act_out = n->T[l + 1].p;
     p.pre_out = n->P[l].p;
-    if ((rc = launch_conv<EPI_GELU_PRE>(n, v.stream, n->T[l], l, false, p))) return rc;
+    if ((rc = launch_conv<EPI_GELU_PRE>(n, v, n->T[l], l, false, p))) return rc;
   }
   ConvParams p;
   memset(&p, 0, sizeof(p));
   p.delta = n->d_delta;
-  return launch_conv<EPI_DELTA>(n, v.stream, n->T[3], 3, false, p);
+  return launch_conv<EPI_DELTA>(n, v, n->T[3], 3, false, p);
 }
 
 // Loss and gradients into d_grad (weights then biases); loss partials in d_lpart.
 int enqueue_backward(gpe_cnn* n, const FieldView& v, const void* target, int eb) {
   const int nb = n->ew_blocks;
-  CNN_CU(n, eb == 8 ? launch_overlapped(true, loss_kernel<float, float>, nb, 256, 0, v.stream,
+  CNN_CU(n, eb == 8 ? launch_overlapped(v.overlap, loss_kernel<float, float>, nb, 256, 0, v.stream,
                                         n->d_delta, v.psi, v.Nx, v.Ny, target, n->nx, n->ny, n->nz,
                                         n->prm.out_scale, n->GA.p, n->d_lpart)
-                    : launch_overlapped(true, loss_kernel<float, double>, nb, 256, 0, v.stream,
+                    : launch_overlapped(v.overlap, loss_kernel<float, double>, nb, 256, 0, v.stream,
                                         n->d_delta, v.psi, v.Nx, v.Ny, target, n->nx, n->ny, n->nz,
                                         n->prm.out_scale, n->GA.p, n->d_lpart));
   n->launches++;
   Act* g = &n->GA;
   Act* other = &n->GB;
   for (int l = 3; l >= 0; l--) {
-    int rc = launch_wgrad(n, v.stream, n->T[l], *g);
+    int rc = launch_wgrad(n, v, n->T[l], *g);
     if (rc) return rc;
-    CNN_CU(n, launch_overlapped(true, grad_finalize_kernel, NTAP + 1, 1024, 0, v.stream, n->d_wpart,
+    CNN_CU(n, launch_overlapped(v.overlap, grad_finalize_kernel, NTAP + 1, 1024, 0, v.stream, n->d_wpart,
                                 n->wgrad_grid, wgrad_role0(n), n->d_bpart,
                                 n->d_grad + (size_t)l * NTAP * 256,
                                 n->d_grad + GPE_CNN_WEIGHTS + l * 16));
@@ -273,7 +273,7 @@ int enqueue_backward(gpe_cnn* n, const FieldView& v, const void* target, int eb)
       memset(&p, 0, sizeof(p));
       p.act_out = other->p;
       p.pre_in = n->P[l - 1].p;
-      if ((rc = launch_conv<EPI_DGELU>(n, v.stream, *g, l, true, p))) return rc;
+      if ((rc = launch_conv<EPI_DGELU>(n, v, *g, l, true, p))) return rc;
       std::swap(g, other);
     }
   }

@@ -302,6 +302,9 @@ void gpe_internal_set_post_step(gpe_ctx* c, int (*fn)(void*, gpe_ctx*), void* ar
   c->post_arg = arg;
 }
 
+namespace {
+bool stream_overlap(const gpe_ctx* c);
+}
 int gpe_internal_field_view(gpe_ctx* c, gpe::FieldView* v) {
   if (!c || !v) return GPE_ERR_INVALID;
   v->psi = c->fld[c->psi_id];
@@ -316,6 +319,7 @@ int gpe_internal_field_view(gpe_ctx* c, gpe::FieldView* v) {
   v->dx = c->dx; v->dy = c->dy; v->dz = c->dz;
   v->xr = c->prm.xr; v->yr = c->prm.yr; v->zr = c->prm.zr;
   v->stage = c->d_stage;
+  v->overlap = stream_overlap(c);
   c->norm_valid = false;
   return GPE_OK;
 }
@@ -883,10 +887,10 @@ KernelFn select_kernel(int R, int* form, const StageSpec& sp, int am, int bm) {
 // but six steps of complex128 order 4 at 256^3 (268 MB) 4.71 ms either way, four of
 // complex64 order 4 at 512^3 (1 GB) 11.5 and 11.2.
 constexpr size_t OVERLAP_BYTES = (size_t)192 << 20;
-bool overlap(const gpe_ctx* c) {
-  return !c->timing && !c->comm && !c->group && c->prm.scheme != GPE_SCHEME_RK45 &&
-         c->nint * (size_t)c->es <= OVERLAP_BYTES;
+bool stream_overlap(const gpe_ctx* c) {
+  return !c->timing && !c->comm && !c->group && c->nint * (size_t)c->es <= OVERLAP_BYTES;
 }
+bool overlap(const gpe_ctx* c) { return stream_overlap(c) && c->prm.scheme != GPE_SCHEME_RK45; }
 
 // part 0: the whole slab; part 1: its boundary planes z = 0, 1 and nz-2,
 // nz-1 (the planes the z-neighbours' ghosts take); part 2: the planes

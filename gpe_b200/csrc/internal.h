@@ -26,6 +26,7 @@ struct FieldView {
   double dx, dy, dz;  // grid spacings, 2 xr / (nx - 1) etc.
   double xr, yr, zr;  // box half-widths
   void* stage;        // dense staging buffer, nx ny nz elements of 16 bytes
+  bool overlap;       // launches on the stream may overlap (stream_overlap in gpe_gpu.cu)
 };
 
 // Lets every launch of fn take as much dynamic shared memory as a block may

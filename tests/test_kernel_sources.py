@@ -70,3 +70,15 @@ def test_overlapped_kernels_promise_nothing_about_memory_in_flight():
                     if p not in CONSTANT_TABLES:
                         bad.add((k, f, p))
     assert not bad, sorted(bad)
+
+
+def test_every_launch_asks_the_rule_for_overlap():
+    """Launches overlap where the context's rule lets them (not while each is
+    timed by itself, for one): none says so by itself."""
+    calls = []
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith(".cu"):
+            with open(os.path.join(CSRC, f)) as h:
+                calls += re.findall(r"launch_overlapped\(\s*([^,]+),", h.read())
+    assert len(calls) >= 15
+    assert set(calls) <= {"overlap(c)", "ov", "v.overlap"}, sorted(set(calls))
