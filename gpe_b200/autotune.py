@@ -36,12 +36,25 @@ def candidates() -> list[BatchOpts]:
             for ty, zc, cp in itertools.product(TILE_Y, ZCHUNK, CTAS_PER_SM)]
 
 
+# of the batched launches a shape was timed on: raised when they change so that
+# a shape tuned before says nothing about them (1: one stage per launch; 2: two)
+LAUNCHES = 2
+
+
 def signature(batch: GpeBatch, device_name: str) -> str:
+    """What the best shape depends on: the members' grids, the kernels that step
+    them (precision, order, compensation and the terms of the right-hand side,
+    which choose between plain, trap and full kernels, the last one stage per
+    launch) and the build of those."""
     p0 = batch.prms[0]
     shapes = sorted((p.nx, p.ny, p.nz) for p in batch.prms)
+    terms = {"eqn": p0.eqn_to_solve,
+             "trap": any(p.omx or p.omy or p.omz for p in batch.prms),
+             "gradient": any(p.Urhs for p in batch.prms),
+             "sponge": any(p.diss_amp for p in batch.prms)}
     key = json.dumps({"shapes": shapes, "order": p0.order, "bcs": p0.bcs,
-                      "precision": p0.precision, "kahan": bool(p0.kahan),
-                      "device": device_name}, sort_keys=True)
+                      "precision": p0.precision, "kahan": bool(p0.kahan), "terms": terms,
+                      "launches": LAUNCHES, "device": device_name}, sort_keys=True)
     return hashlib.sha1(key.encode()).hexdigest()[:16]
 
 
