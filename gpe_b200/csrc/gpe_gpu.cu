@@ -2044,17 +2044,49 @@ int alloc_field(gpe_ctx* c, int id) {
   return GPE_OK;
 }
 
+// cuMemGetAddressRange, or null (device arrays are then staged).
+PFN_cuMemGetAddressRange_v3020 address_range() {
+  static const PFN_cuMemGetAddressRange_v3020 fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
+  }();
+  return fn;
+}
+
 // Whether a caller's device array can be read or written by this context's
-// kernels directly: memory of the context's own device, aligned to its
-// elements.  Anything else goes through the staging buffer by cudaMemcpyAsync.
-bool direct_array(const gpe_ctx* c, const void* p, int elem_bytes) {
-  if (reinterpret_cast<uintptr_t>(p) % (uintptr_t)elem_bytes != 0) return false;
+// kernels directly (*direct): memory of the context's own device, aligned to its
+// elements and whole inside one allocation.  Anything else goes through the
+// staging buffer by cudaMemcpyAsync, which has checks of its own; an array that
+// ends where no memory follows is an error here, as a kernel has none.
+int direct_array(gpe_ctx* c, const void* p, int elem_bytes, bool* direct) {
+  *direct = false;
+  if (reinterpret_cast<uintptr_t>(p) % (uintptr_t)elem_bytes != 0) return GPE_OK;
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return GPE_OK;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == c->dev;
+  const auto range = address_range();
+  if (a.type != cudaMemoryTypeDevice || a.device != c->dev || !range) return GPE_OK;
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  const size_t bytes = c->nint * (size_t)elem_bytes;
+  CUdeviceptr base = 0, next = 0;
+  size_t size = 0, more = 0;
+  if (range(&base, &size, at) != CUDA_SUCCESS) return GPE_OK;
+  if (at + bytes <= base + size) {
+    *direct = true;
+    return GPE_OK;
+  }
+  if (range(&next, &more, base + size) == CUDA_SUCCESS) return GPE_OK;
+  return fail(c, GPE_ERR_CUDA,
+              "device array of " + std::to_string(bytes) + " bytes ends beyond its allocation of " +
+                  std::to_string(base + size - at));
 }
 
 // A dense array (elements of elem_bytes, the staging buffer or a caller's
@@ -2095,7 +2127,12 @@ int load_dense(gpe_ctx* c, const void* src, int elem_bytes) {
 }
 
 int stage_in(gpe_ctx* c, const void* src, int elem_bytes, bool device) {
-  if (device && direct_array(c, src, elem_bytes)) return load_dense(c, src, elem_bytes);
+  bool direct = false;
+  if (device) {
+    const int rc = direct_array(c, src, elem_bytes, &direct);
+    if (rc) return rc;
+  }
+  if (direct) return load_dense(c, src, elem_bytes);
   const size_t bytes = c->nint * (size_t)elem_bytes;
   CU_CHECK(c, cudaMemcpyAsync(c->d_stage, src, bytes,
                               device ? cudaMemcpyDeviceToDevice
@@ -2133,7 +2170,12 @@ int pack_dense(gpe_ctx* c, int field, void* dst, int elem_bytes) {
 }
 
 int stage_out(gpe_ctx* c, int field, void* dst, int elem_bytes, bool device) {
-  if (device && direct_array(c, dst, elem_bytes)) {
+  bool direct = false;
+  if (device) {
+    const int rc = direct_array(c, dst, elem_bytes, &direct);
+    if (rc) return rc;
+  }
+  if (direct) {
     const int rc = pack_dense(c, field, dst, elem_bytes);
     if (rc) return rc;
     CU_CHECK(c, cudaStreamSynchronize(c->stream));
