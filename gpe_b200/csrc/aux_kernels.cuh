@@ -18,12 +18,13 @@ struct Geom {
   int nx, ny, nz;  // interior
   int Nx, Ny;      // padded pitches
   int bcs;
+  int gh;            // ghost layers on every side
   int zg_lo, zg_hi;  // fill z ghosts below / above locally
 };
 
 __device__ __forceinline__ size_t padded_index(const Geom& g, int i, int j,
                                                int k) {
-  return ((size_t)(k + GH) * g.Ny + (size_t)(j + GH)) * g.Nx + (size_t)(i + GH);
+  return ((size_t)(k + g.gh) * g.Ny + (size_t)(j + g.gh)) * g.Nx + (size_t)(i + g.gh);
 }
 
 // One warp per row of a field: rows r, r + (all warps), ... of `nrows`.
@@ -62,17 +63,17 @@ template <typename TS, typename TI>
 __global__ void unpack_kernel(const TI* __restrict__ src, TS* __restrict__ dst, Geom g) {
   using VI = typename VT<TI>::T;
   const int lane = threadIdx.x & 31;
-  const int Nz = g.nz + 2 * GH;
+  const int gh = g.gh, Nz = g.nz + 2 * gh;
   GPE_FOR_ROWS(r, g.Ny * Nz) {
     const int kp = r / g.Ny, jp = r - kp * g.Ny;
-    const int k = kp - GH, j = jp - GH;
+    const int k = kp - gh, j = jp - gh;
     if ((k < 0 && !g.zg_lo) || (k >= g.nz && !g.zg_hi)) continue;  // a neighbour sends these
     const int ks = ghost_source(k, g.nz, g.bcs), js = ghost_source(j, g.ny, g.bcs);
     const TI* s = src + 2 * ((size_t)ks * g.ny + js) * (size_t)g.nx;
-    TS* d = dst + 2 * ((size_t)r * g.Nx + GH);
+    TS* d = dst + 2 * ((size_t)r * g.Nx + gh);
     copy_row<TS, TI>(d, s, g.nx, lane);
-    if (lane < 2 * GH) {
-      const int i = lane < GH ? lane - GH : g.nx + lane - GH;
+    if (lane < 2 * gh) {
+      const int i = lane < gh ? lane - gh : g.nx + lane - gh;
       const VI v = reinterpret_cast<const VI*>(s)[ghost_source(i, g.nx, g.bcs)];
       st_one<TS>(d + 2 * i, (TS)v.x, (TS)v.y);
     }
@@ -108,7 +109,7 @@ __device__ __forceinline__ void fill_ghost_rows(TS* f, const Geom& g, int depth,
     const size_t from =
         padded_index(g, 0, ghost_source(j, g.ny, g.bcs), ghost_source(k, g.nz, g.bcs));
     const size_t to = padded_index(g, 0, j, k);
-    // 16 bytes a lane (rows start 32-byte aligned, GH complexes in)
+    // 16 bytes a lane (rows start an even number of complexes in)
     constexpr int W = 16 / (int)sizeof(V);
     const float4* s4 = reinterpret_cast<const float4*>(F + from);
     float4* d4 = reinterpret_cast<float4*>(F + to);

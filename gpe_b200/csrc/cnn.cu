@@ -179,7 +179,7 @@ int check_view(gpe_cnn* n, const FieldView& v) {
 
 int pack_input(gpe_cnn* n, const FieldView& v, const Act& dst) {
   CNN_CU(n, launch_overlapped(v.overlap, pack_input_kernel<float>, (n->Zp * n->Yp + 7) / 8, 256, 0,
-                              v.stream, v.psi, v.Nx, v.Ny, n->nx, n->ny, n->nz, dst.p, dst.H));
+                              v.stream, v.psi, v.Nx, v.Ny, v.gh, n->nx, n->ny, n->nz, dst.p, dst.H));
   n->launches++;
   return GPE_OK;
 }
@@ -219,6 +219,7 @@ int enqueue_apply(gpe_cnn* n, const FieldView& v, int* status) {
   p.psi = static_cast<float*>(v.psi);
   p.psi_Nx = v.Nx;
   p.psi_Ny = v.Ny;
+  p.psi_gh = v.gh;
   return launch_conv<EPI_RESID>(n, v, n->A1, 3, false, p);
 }
 
@@ -252,10 +253,10 @@ int enqueue_train_forward(gpe_cnn* n, const FieldView& v) {
 int enqueue_backward(gpe_cnn* n, const FieldView& v, const void* target, int eb) {
   const int nb = n->ew_blocks;
   CNN_CU(n, eb == 8 ? launch_overlapped(v.overlap, loss_kernel<float, float>, nb, 256, 0, v.stream,
-                                        n->d_delta, v.psi, v.Nx, v.Ny, target, n->nx, n->ny, n->nz,
+                                        n->d_delta, v.psi, v.Nx, v.Ny, v.gh, target, n->nx, n->ny, n->nz,
                                         n->prm.out_scale, n->GA.p, n->d_lpart)
                     : launch_overlapped(v.overlap, loss_kernel<float, double>, nb, 256, 0, v.stream,
-                                        n->d_delta, v.psi, v.Nx, v.Ny, target, n->nx, n->ny, n->nz,
+                                        n->d_delta, v.psi, v.Nx, v.Ny, v.gh, target, n->nx, n->ny, n->nz,
                                         n->prm.out_scale, n->GA.p, n->d_lpart));
   n->launches++;
   Act* g = &n->GA;
@@ -572,16 +573,16 @@ int gpe_cnn_restrict(gpe_ctx* fine, void* coarse, int32_t eb) {
   const int nb = (int)std::min<size_t>((nc + 255) / 256, 148 * 8);
   if (v.es == 16 && eb == 16)
     restrict_kernel<double, double><<<nb, 256, 0, v.stream>>>(
-        (const double*)v.psi, v.Nx, v.Ny, nxc, nyc, nzc, (double*)coarse);
+        (const double*)v.psi, v.Nx, v.Ny, v.gh, nxc, nyc, nzc, (double*)coarse);
   else if (v.es == 16)
     restrict_kernel<double, float><<<nb, 256, 0, v.stream>>>(
-        (const double*)v.psi, v.Nx, v.Ny, nxc, nyc, nzc, (float*)coarse);
+        (const double*)v.psi, v.Nx, v.Ny, v.gh, nxc, nyc, nzc, (float*)coarse);
   else if (eb == 16)
     restrict_kernel<float, double><<<nb, 256, 0, v.stream>>>(
-        (const float*)v.psi, v.Nx, v.Ny, nxc, nyc, nzc, (double*)coarse);
+        (const float*)v.psi, v.Nx, v.Ny, v.gh, nxc, nyc, nzc, (double*)coarse);
   else
     restrict_kernel<float, float><<<nb, 256, 0, v.stream>>>(
-        (const float*)v.psi, v.Nx, v.Ny, nxc, nyc, nzc, (float*)coarse);
+        (const float*)v.psi, v.Nx, v.Ny, v.gh, nxc, nyc, nzc, (float*)coarse);
   CNN_CU(nullptr, cudaGetLastError());
   CNN_CU(nullptr, cudaStreamSynchronize(v.stream));
   return GPE_OK;

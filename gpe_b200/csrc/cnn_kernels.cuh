@@ -143,8 +143,8 @@ struct ConvParams {
   __nv_bfloat16* pre_out;           // EPI_GELU_PRE
   const __nv_bfloat16* pre_in;      // EPI_DGELU
   float* delta;                     // EPI_DELTA: dense [nz][ny][nx][2]
-  float* psi;                       // EPI_RESID: solver field (complex64, GH ghosts)
-  int psi_Nx, psi_Ny;
+  float* psi;                       // EPI_RESID: solver field (complex64)
+  int psi_Nx, psi_Ny, psi_gh;       // its pitches and ghost layers
   float out_scale;
   int* status;
   unsigned long long wait_limit_ns;
@@ -281,7 +281,7 @@ struct EpiAux {
 };
 
 __device__ __forceinline__ size_t psi_index(const ConvParams& p, int x, int y, int z) {
-  return ((size_t)(z + GH) * p.psi_Ny + (y + GH)) * p.psi_Nx + (x + GH);
+  return ((size_t)(z + p.psi_gh) * p.psi_Ny + (y + p.psi_gh)) * p.psi_Nx + (x + p.psi_gh);
 }
 
 // off: the site's element offset in an activation buffer.
@@ -348,9 +348,9 @@ __device__ __forceinline__ void conv_epilogue(const ConvParams& p, const float (
     v.y += (acc[1] + b.y) * p.out_scale;
     float2* f = reinterpret_cast<float2*>(p.psi);
     int gx[2], gy[2], gz[2];
-    ghost_targets(x, p.nx, 1, GH, gx[0], gx[1]);
-    ghost_targets(y, p.ny, 1, GH, gy[0], gy[1]);
-    ghost_targets(z, p.nz, 1, GH, gz[0], gz[1]);
+    ghost_targets(x, p.nx, 1, p.psi_gh, gx[0], gx[1]);
+    ghost_targets(y, p.ny, 1, p.psi_gh, gy[0], gy[1]);
+    ghost_targets(z, p.nz, 1, p.psi_gh, gz[0], gz[1]);
     auto row = [&](int yt, int zt) {
       float2* r = f + psi_index(p, 0, yt, zt);
       r[x] = v;
@@ -855,14 +855,14 @@ __global__ void __launch_bounds__(W_THREADS, 1) conv_wgrad_kernel(const __grid_c
 // --------------------------------------------------------------------------
 // Element-wise and reduction kernels.
 
-// Solver field (GH ghosts, pitches Nx, Ny; complex of TS) -> first-layer input
+// Solver field (gh ghosts, pitches Nx, Ny; complex of TS) -> first-layer input
 // (channels Re, Im, 0, ...; H halves), ghosts included.  Every padded site
 // reads its periodic interior source (the solver keeps only the face ghosts
 // a star stencil needs, not edges and corners).  One warp per padded (y, z) row,
 // four records a lane in flight; bound by the 16 (or 32) bytes written per site
 // (128^3: 12.2 us with a block of 128 threads per row of 130, 11.1 so).
 template <typename TS>
-__global__ void pack_input_kernel(const TS* psi, int Nx, int Ny, int nx, int ny, int nz,
+__global__ void pack_input_kernel(const TS* psi, int Nx, int Ny, int gh, int nx, int ny, int nz,
                                   __nv_bfloat16* act, int H) {
   const int Xp = nx + 2, Yp = ny + 2, rows = Yp * (nz + 2);
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -873,7 +873,7 @@ __global__ void pack_input_kernel(const TS* psi, int Nx, int Ny, int nx, int ny,
     const int yp = row % Yp, zp = row / Yp;
     const int y = yp == 0 ? ny - 1 : (yp == ny + 1 ? 0 : yp - 1);
     const int z = zp == 0 ? nz - 1 : (zp == nz + 1 ? 0 : zp - 1);
-    const V* src = reinterpret_cast<const V*>(psi) + ((size_t)(z + GH) * Ny + (y + GH)) * Nx + GH;
+    const V* src = reinterpret_cast<const V*>(psi) + ((size_t)(z + gh) * Ny + (y + gh)) * Nx + gh;
     uint4* dst = reinterpret_cast<uint4*>(act) + (size_t)row * H * Xp;
     for (int x0 = lane; x0 < Xp; x0 += 128) {
       V v[4];
@@ -897,8 +897,8 @@ __global__ void pack_input_kernel(const TS* psi, int Nx, int Ny, int nx, int ny,
 // layer's output: e = u + delta - target, loss = sum |e|^2 / n,
 // dL/d(out_c) = 2 e_c out_scale / n into channels 0, 1 of g (others 0).
 template <typename TS, typename TT>
-__global__ void loss_kernel(const float* delta, const TS* u, int Nx, int Ny, const TT* target,
-                            int nx, int ny, int nz, float out_scale, __nv_bfloat16* g,
+__global__ void loss_kernel(const float* delta, const TS* u, int Nx, int Ny, int gh,
+                            const TT* target, int nx, int ny, int nz, float out_scale, __nv_bfloat16* g,
                             double* partials) {
   __shared__ double red[32];
   const int Xp = nx + 2, Yp = ny + 2;
@@ -911,7 +911,7 @@ __global__ void loss_kernel(const float* delta, const TS* u, int Nx, int Ny, con
     const int x = (int)(s % nx);
     const size_t t = s / nx;
     const int y = (int)(t % ny), z = (int)(t / ny);
-    const size_t q = ((size_t)(z + GH) * Ny + (y + GH)) * Nx + (x + GH);
+    const size_t q = ((size_t)(z + gh) * Ny + (y + gh)) * Nx + (x + gh);
     const double er = (double)u[2 * q] + (double)delta[2 * s] - (double)target[2 * s];
     const double ei = (double)u[2 * q + 1] + (double)delta[2 * s + 1] - (double)target[2 * s + 1];
     acc += er * er + ei * ei;
@@ -1013,11 +1013,11 @@ __global__ void pack_out2_kernel(const float* __restrict__ w, __nv_bfloat16* __r
   wf2[i] = __float2bfloat16_rn(v);
 }
 
-// 2:1 restriction (2x2x2 average) of a solver field (GH ghosts) to a dense
+// 2:1 restriction (2x2x2 average) of a solver field (gh ghosts) to a dense
 // complex array of TO on the coarse grid.
 template <typename TS, typename TO>
-__global__ void restrict_kernel(const TS* __restrict__ f, int Nx, int Ny, int nxc, int nyc,
-                                int nzc, TO* __restrict__ out) {
+__global__ void restrict_kernel(const TS* __restrict__ f, int Nx, int Ny, int gh, int nxc,
+                                int nyc, int nzc, TO* __restrict__ out) {
   const size_t n = (size_t)nxc * nyc * nzc;
   for (size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < n;
        s += (size_t)gridDim.x * blockDim.x) {
@@ -1029,7 +1029,7 @@ __global__ void restrict_kernel(const TS* __restrict__ f, int Nx, int Ny, int nx
       for (int b = 0; b < 2; b++)
         for (int a = 0; a < 2; a++) {
           const size_t q =
-              ((size_t)(2 * z + c + GH) * Ny + (2 * y + b + GH)) * Nx + (2 * x + a + GH);
+              ((size_t)(2 * z + c + gh) * Ny + (2 * y + b + gh)) * Nx + (2 * x + a + gh);
           re += (double)f[2 * q];
           im += (double)f[2 * q + 1];
         }

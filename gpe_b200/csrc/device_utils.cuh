@@ -202,9 +202,10 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// Ghost layers every stored field has on each side of each axis: two stages of
-// an order-4 stencil reach 4 sites, which pair_kernel.cuh evaluates in one
-// launch (the one-stage kernels read and fill the inner 2).
+// Ghost layers on each side of each axis of a field that is stepped two stages at
+// a time: two stages of an order-4 stencil reach 4 sites, which pair_kernel.cuh
+// evaluates in one launch (the one-stage kernels read and fill the inner 2, and
+// fields that only they step have 2).
 constexpr int GH = 4;
 
 // Ghost targets of interior index i along an axis of n points: the ghost
@@ -219,7 +220,7 @@ __device__ __forceinline__ void ghost_targets(int i, int n, int bcs, int depth, 
   g1 = (hi >= n && hi < n + depth && i >= 0 && i < n) ? hi : NO_GHOST;
 }
 
-// Interior index whose value position g (-GH <= g < n + GH) holds.
+// Interior index whose value position g (-n < g < 2 n - 1) holds.
 __device__ __forceinline__ int ghost_source(int g, int n, int bcs) {
   if (bcs == 1) return g < 0 ? g + n : g >= n ? g - n : g;
   return g < 0 ? -g : g >= n ? 2 * (n - 1) - g : g;

@@ -1,7 +1,7 @@
 // gpe_gpu.cu -- context, stage scheduling and the C-ABI of include/gpe_gpu.h.
 //
 // One context = one run on one device.  Fields live in a ghost-padded layout
-// (GH ghost layers on every axis, x pitch rounded to 4 elements) so that each
+// (2 or 4 ghost layers on every axis, x pitch rounded to 4 elements) so that each
 // stage kernel reads its stencil plane as one TMA box; ghosts are refreshed by
 // the kernel that writes the field (see stage_kernel.cuh), which replaces the
 // reference's halo exchange (src/variables.f90:186-358).
@@ -211,6 +211,7 @@ struct gpe_ctx {
   int dev = 0;
   cudaStream_t stream = nullptr;
   int nx, ny, nz, Nx, Ny, Nz;
+  int gh;  // ghost layers of its fields on every side (ghost_layers)
   int num_sms = 148;
   // z-slab of a global grid (single domain: nzg == nz, z_off == 0)
   int nzg = 0, z_off = 0;
@@ -309,7 +310,7 @@ int gpe_internal_field_view(gpe_ctx* c, gpe::FieldView* v) {
   if (!c || !v) return GPE_ERR_INVALID;
   v->psi = c->fld[c->psi_id];
   v->nx = c->nx; v->ny = c->ny; v->nz = c->nz; v->Nx = c->Nx; v->Ny = c->Ny;
-  v->gh = GH;
+  v->gh = c->gh;
   v->es = c->es;
   v->bcs = c->prm.bcs;
   v->dev = c->dev;
@@ -433,11 +434,11 @@ int exchange_ghosts(gpe_ctx* c, int field, cudaStream_t st = nullptr) {
   if (!st) st = c->stream;
   const size_t plane = (size_t)c->Nx * c->Ny * (size_t)c->es;  // bytes
   unsigned char* f = static_cast<unsigned char*>(c->fld[field]);
-  // padded plane index pz = z + GH
-  unsigned char* bottom = f + GH * plane;                        // z = 0, 1
-  unsigned char* top = f + (size_t)(c->nz - 2 + GH) * plane;     // z = nz-2, nz-1
-  unsigned char* ghost_lo = f + (GH - 2) * plane;                // z = -2, -1
-  unsigned char* ghost_hi = f + (size_t)(c->nz + GH) * plane;    // z = nz, nz+1
+  // padded plane index pz = z + gh
+  unsigned char* bottom = f + c->gh * plane;                     // z = 0, 1
+  unsigned char* top = f + (size_t)(c->nz - 2 + c->gh) * plane;  // z = nz-2, nz-1
+  unsigned char* ghost_lo = f + (c->gh - 2) * plane;             // z = -2, -1
+  unsigned char* ghost_hi = f + (size_t)(c->nz + c->gh) * plane; // z = nz, nz+1
   const size_t n = 2 * plane;
   NCCL_CHECK(c, g_nccl.GroupStart());
   if (c->exch_hi) NCCL_CHECK(c, g_nccl.Send(top, n, ncclUint8, c->nbr_hi, c->comm, st));
@@ -754,12 +755,24 @@ bool network_grid(const gpe_ctx* c) {
   return c->es == 8 && c->prm.bcs == 1 && c->nx % 16 == 0 && c->nx <= 128;
 }
 
+// Ghost layers of a context's fields: GH where its steps can run in pairs (see
+// steps_in_pairs), 2 where none can, so that those fields stay as small as the
+// one-stage kernels need (a cube of 32 sites a side: 1.37 times the bytes with GH).
+// Only what members of a slab group share decides, as they copy each other's planes;
+// a slab is created like any context, before it is known to be one, and keeps its
+// layers (its exchange moves two planes).
+int ghost_layers(const gpe_ctx* c) {
+  const bool rk4 = c->prm.scheme == GPE_SCHEME_RK4, rk2 = c->prm.scheme == GPE_SCHEME_RK2;
+  return (rk2 || (rk4 && !network_grid(c))) && c->prm.eqn_to_solve != 3 ? GH : 2;
+}
+
 // Per-run part of a launch that does not depend on its fields: geometry,
 // stencil and right-hand-side coefficients, tables.
 template <typename TS, typename TC>
 void fill_geometry(const gpe_ctx* c, int R, const RhsForm& f, RunDesc<TS, TC>* rd) {
   rd->nx = c->nx; rd->ny = c->ny; rd->nz = c->nz; rd->Nx = c->Nx; rd->Ny = c->Ny;
   rd->bcs = c->prm.bcs;
+  rd->gh = c->gh;
   rd->acc_first = network_grid(c) ? 0 : 1;
   rd->zg_lo = c->exch_lo ? 0 : 1;
   rd->zg_hi = c->exch_hi ? 0 : 1;
@@ -987,15 +1000,15 @@ int group_exchange(gpe_group* g, int field, cudaStream_t st = nullptr) {
     if (c->exch_lo) {
       const gpe_ctx* lo = g->m[c->nbr_lo];
       const unsigned char* src = static_cast<const unsigned char*>(lo->fld[field]) +
-                                 (size_t)(lo->nz - 2 + GH) * plane;  // its z = nz-2, nz-1
-      CU_CHECK(c, cudaMemcpyAsync(f + (GH - 2) * plane, src, 2 * plane,
+                                 (size_t)(lo->nz - 2 + lo->gh) * plane;  // its z = nz-2, nz-1
+      CU_CHECK(c, cudaMemcpyAsync(f + (c->gh - 2) * plane, src, 2 * plane,
                                   cudaMemcpyDeviceToDevice, st));
     }
     if (c->exch_hi) {
       const gpe_ctx* hi = g->m[c->nbr_hi];
       const unsigned char* src = static_cast<const unsigned char*>(hi->fld[field]) +
-                                 GH * plane;  // its z = 0, 1
-      CU_CHECK(c, cudaMemcpyAsync(f + (size_t)(c->nz + GH) * plane, src, 2 * plane,
+                                 hi->gh * plane;  // its z = 0, 1
+      CU_CHECK(c, cudaMemcpyAsync(f + (size_t)(c->nz + c->gh) * plane, src, 2 * plane,
                                   cudaMemcpyDeviceToDevice, st));
     }
   }
@@ -1114,6 +1127,7 @@ Geom geom(const gpe_ctx* c) {
   Geom g;
   g.nx = c->nx; g.ny = c->ny; g.nz = c->nz; g.Nx = c->Nx; g.Ny = c->Ny;
   g.bcs = c->prm.bcs;
+  g.gh = c->gh;
   g.zg_lo = c->exch_lo ? 0 : 1;
   g.zg_hi = c->exch_hi ? 0 : 1;
   return g;
@@ -2727,12 +2741,13 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
     return bail(GPE_ERR_CUDA);
   }
   c->nx = p.nx; c->ny = p.ny; c->nz = p.nz;
-  c->Nx = (int)round_up((size_t)p.nx + 2 * GH, 4);
-  c->Ny = p.ny + 2 * GH;
-  c->Nz = p.nz + 2 * GH;
+  c->es = p.precision;
+  c->gh = ghost_layers(c);
+  c->Nx = (int)round_up((size_t)p.nx + 2 * c->gh, 4);
+  c->Ny = p.ny + 2 * c->gh;
+  c->Nz = p.nz + 2 * c->gh;
   c->npad = (size_t)c->Nx * c->Ny * c->Nz;
   c->nint = (size_t)p.nx * p.ny * p.nz;
-  c->es = p.precision;
   c->nzg = p.nz;
   c->z_off = 0;
   // get_grid, src/ic.f90:32-69
@@ -2904,7 +2919,7 @@ int gpe_gpu_get_site(gpe_ctx* c, int32_t i, int32_t j, int32_t k, double* re_im)
   if (!re_im) return fail(c, GPE_ERR_INVALID, "null output");
   if (i < 0 || i >= c->nx || j < 0 || j >= c->ny || k < 0 || k >= c->nz)
     return fail(c, GPE_ERR_INVALID, "site outside the grid");
-  const size_t q = ((size_t)(k + GH) * c->Ny + (size_t)(j + GH)) * c->Nx + (size_t)(i + GH);
+  const size_t q = ((size_t)(k + c->gh) * c->Ny + (size_t)(j + c->gh)) * c->Nx + (size_t)(i + c->gh);
   unsigned char buf[16];
   CU_CHECK(c, cudaMemcpyAsync(buf, static_cast<const unsigned char*>(c->fld[c->psi_id]) +
                                        q * (size_t)c->es,
@@ -2927,7 +2942,7 @@ int gpe_gpu_get_plane(gpe_ctx* c, int32_t k, void* out, int32_t elem_bytes) {
   rc = check_elem(c, elem_bytes, out);
   if (rc) return rc;
   if (k < 0 || k >= c->nz) return fail(c, GPE_ERR_INVALID, "plane outside the grid");
-  const size_t first = ((size_t)(k + GH) * c->Ny + GH) * c->Nx + GH;
+  const size_t first = ((size_t)(k + c->gh) * c->Ny + c->gh) * c->Nx + c->gh;
   const unsigned char* src = static_cast<const unsigned char*>(c->fld[c->psi_id]) +
                              first * (size_t)c->es;
   const size_t n = (size_t)c->nx * c->ny;

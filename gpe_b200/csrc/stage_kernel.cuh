@@ -98,6 +98,7 @@ struct alignas(64) RunDesc {
   int Nx, Ny;           // padded pitches (complex elements)
   int ntx, nty, zchunk, nchunks;
   int bcs;
+  int gh;                 // ghost layers of the fields
   int zg_lo, zg_hi;     // fill the z ghosts below / above locally (else a
                         // neighbouring rank sends them)
   const TS* stencil;    // stencil field (padded layout), warm-up planes
@@ -259,20 +260,21 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
             fence_proxy_async();
           }
           unsigned char* st = sbase + (size_t)slot * stride;
+          const int gh = rd.gh;
           const bool with_pt = (NP > 0) && (u >= R);
           mbar_arrive_expect_tx(&full[slot],
                                 NS * p.halo_box_bytes + (with_pt ? NP * p.pt_box_bytes : 0u));
-          tma_load_3d(st, &rd.maps.halo, &full[slot], W * (tile_x * TX + GH - 2),
-                      tile_y * TY + GH - R, w.z0 + u + GH);
+          tma_load_3d(st, &rd.maps.halo, &full[slot], W * (tile_x * TX + gh - 2),
+                      tile_y * TY + gh - R, w.z0 + u + gh);
           if (NS == 2)
-            tma_load_3d(st + p.halo_smem_bytes, &rd.maps.halo2, &full[slot], W * (tile_x * TX + GH - 2),
-                        tile_y * TY + GH - R, w.z0 + u + GH);
+            tma_load_3d(st + p.halo_smem_bytes, &rd.maps.halo2, &full[slot], W * (tile_x * TX + gh - 2),
+                        tile_y * TY + gh - R, w.z0 + u + gh);
           if (with_pt) {
 #pragma unroll
             for (int qq = 0; qq < NP; qq++)
               tma_load_3d(st + hstride + (size_t)qq * p.pt_smem_bytes,
-                          &rd.maps.pt[qq], &full[slot], W * (tile_x * TX + GH),
-                          tile_y * TY + GH, w.z0 + u - R + GH);
+                          &rd.maps.pt[qq], &full[slot], W * (tile_x * TX + gh),
+                          tile_y * TY + gh, w.z0 + u - R + gh);
           }
           s_issued = ++issued;
           if (++slot == S) {
@@ -416,7 +418,7 @@ __device__ __forceinline__ void stage_body(const StageParams<TS, TC>& p) {
     }
   }
   // element offset of this thread's first site (first row) in plane z0
-  size_t base = (size_t)(z0 + GH) * NxNy + (size_t)(j0 + GH) * Nx + (size_t)(i0 + GH);
+  size_t base = (size_t)(z0 + rd.gh) * NxNy + (size_t)(j0 + rd.gh) * Nx + (size_t)(i0 + rd.gh);
 
   // z-queues, one per row: physical slot of push number c is c % QN; after
   // push c the plane d above the one being computed sits in slot
