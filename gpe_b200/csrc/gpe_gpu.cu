@@ -212,6 +212,7 @@ struct gpe_ctx {
   cudaStream_t stream = nullptr;
   int nx, ny, nz, Nx, Ny, Nz;
   int gh;  // ghost layers of its fields on every side (ghost_layers)
+  int layout = 0;  // counts the changes of its fields' or tables' addresses
   int num_sms = 148;
   // z-slab of a global grid (single domain: nzg == nz, z_off == 0)
   int nzg = 0, z_off = 0;
@@ -233,6 +234,7 @@ struct gpe_ctx {
   double* tabW[3] = {};
   double* tabX[3] = {};
   void* d_tables = nullptr;
+  size_t table_bytes = 0;
   double* d_partials = nullptr;
   size_t partials_cap = 0;  // CTAs
   double* d_scal = nullptr;  // [0] norm [1] E [2] H4 [3] errmax
@@ -282,6 +284,7 @@ struct gpe_ctx {
   cudaGraphExec_t rk_exec[2] = {nullptr, nullptr};
   int rk_psi[2] = {-1, -1};  // psi buffer each captured step starts from
   bool ghosts_dirty = false;  // psi loaded alone; its z ghosts await the group
+  bool lost = false;  // no fields: a new layout could not be allocated
   bool wide = false;  // psi's ghosts are filled 2R deep, edges included (pair_kernel.cuh)
   std::string err;
 };
@@ -307,7 +310,7 @@ namespace {
 bool stream_overlap(const gpe_ctx* c);
 }
 int gpe_internal_field_view(gpe_ctx* c, gpe::FieldView* v) {
-  if (!c || !v) return GPE_ERR_INVALID;
+  if (!c || !v || c->lost) return GPE_ERR_INVALID;
   v->psi = c->fld[c->psi_id];
   v->nx = c->nx; v->ny = c->ny; v->nz = c->nz; v->Nx = c->Nx; v->Ny = c->Ny;
   v->gh = c->gh;
@@ -759,8 +762,9 @@ bool network_grid(const gpe_ctx* c) {
 // steps_in_pairs), 2 where none can, so that those fields stay as small as the
 // one-stage kernels need (a cube of 32 sites a side: 1.37 times the bytes with GH).
 // Only what members of a slab group share decides, as they copy each other's planes;
-// a slab is created like any context, before it is known to be one, and keeps its
-// layers (its exchange moves two planes).
+// a slab is created like any context and narrowed when it is placed
+// (gpe_gpu_set_slab), and a context whose fields do not fit with GH is created
+// with 2.
 int ghost_layers(const gpe_ctx* c) {
   const bool rk4 = c->prm.scheme == GPE_SCHEME_RK4, rk2 = c->prm.scheme == GPE_SCHEME_RK2;
   return (rk2 || (rk4 && !network_grid(c))) && c->prm.eqn_to_solve != 3 ? GH : 2;
@@ -1260,17 +1264,17 @@ struct PairSpec {
   int family = GPE_FAM_OTHER;
 };
 
-// A context steps with pairs unless its z ghosts come from neighbours (two
-// planes are exchanged, a pair needs four), per-launch timing is on, whose
-// families are single stages, the equation has the sphere mask, rk4 keeps the
-// increments apart (network_grid), or the full form, whose terms
+// A context steps with pairs unless its fields have no room for their ghosts (the
+// equation has the sphere mask, rk4 keeps the increments apart, the grid is a
+// slab: ghost_layers), its z ghosts come from neighbours (two planes are
+// exchanged, a pair needs four), per-launch timing is on, whose families are
+// single stages, or the full form, whose terms
 // spill the pair's registers, except in complex64 at order 2 (equation 1 at
 // 150 x 93 x 71, rk4, us a step in pairs and in stages: 54 and 59 there;
 // complex128 95 and 97 at order 2, 182 and 125 at order 4; rk2 at 200 x 193 x
 // 171, complex128, order 2: 223 and 209).
 bool steps_in_pairs(const gpe_ctx* c) {
-  if (c->comm || c->group || c->nzg != c->nz || c->timing || c->prm.eqn_to_solve == 3) return false;
-  if (c->prm.scheme == GPE_SCHEME_RK4 && network_grid(c)) return false;
+  if (c->gh < GH || c->comm || c->group || c->nzg != c->nz || c->timing) return false;
   return (c->prm.order == 2 && c->es == 8) || !rhs_form(c).full;
 }
 
@@ -1982,7 +1986,8 @@ int build_tables(gpe_ctx* c) {
     }
   }
   CU_CHECK(c, cudaMalloc(&c->d_tables, off));
-  c->device_bytes += (int64_t)off;
+  c->device_bytes += (int64_t)off - (int64_t)c->table_bytes;
+  c->table_bytes = off;
   std::vector<unsigned char> h(off, 0);
   for (int a = 0; a < 3; a++) {
     float* vf = reinterpret_cast<float*>(&h[offs[a][0]]);
@@ -2058,6 +2063,51 @@ int alloc_field(gpe_ctx* c, int id) {
   return GPE_OK;
 }
 
+// Pitches and size of the fields from the grid and the ghost layers.
+void set_layout(gpe_ctx* c, int gh) {
+  c->gh = gh;
+  c->Nx = (int)round_up((size_t)c->nx + 2 * gh, 4);
+  c->Ny = c->ny + 2 * gh;
+  c->Nz = c->nz + 2 * gh;
+  c->npad = (size_t)c->Nx * c->Ny * c->Nz;
+}
+
+void free_fields(gpe_ctx* c) {
+  for (void*& f : c->fld) {
+    if (!f) continue;
+    cudaFree(f);
+    f = nullptr;
+    c->device_bytes -= (int64_t)(c->npad * (size_t)c->es);
+  }
+}
+
+// The fields of the context's scheme; one whose fields do not fit with room for
+// pairs gets the layers that single stages need.
+int alloc_fields(gpe_ctx* c) {
+  std::vector<int> need = {F_PSI, F_ALT};
+  switch (c->prm.scheme) {
+    case GPE_SCHEME_RK2: need.push_back(F_UA); break;
+    case GPE_SCHEME_RK4:
+      need.insert(need.end(), {F_UB, F_ACC});
+      break;
+    case GPE_SCHEME_RK45:
+      need.insert(need.end(), {F_UA, F_UB, F_K1, F_K2, F_K3, F_K4, F_K5});
+      break;
+    default: break;
+  }
+  if (c->prm.kahan) {
+    need.push_back(F_C);
+    if (c->prm.scheme == GPE_SCHEME_RK45) need.push_back(F_CALT);
+  }
+  for (;;) {
+    int rc = GPE_OK;
+    for (size_t k = 0; k < need.size() && !rc; k++) rc = alloc_field(c, need[k]);
+    if (rc != GPE_ERR_OOM || c->gh == 2) return rc;
+    free_fields(c);
+    set_layout(c, 2);
+  }
+}
+
 // cuMemGetAddressRange, or null (device arrays are then staged).
 PFN_cuMemGetAddressRange_v3020 address_range() {
   static const PFN_cuMemGetAddressRange_v3020 fn = [] {
@@ -2104,13 +2154,13 @@ int direct_array(gpe_ctx* c, const void* p, int elem_bytes, bool* direct) {
 }
 
 // A dense array (elements of elem_bytes, the staging buffer or a caller's
-// device array) -> psi with ghosts.
-int load_dense(gpe_ctx* c, const void* src, int elem_bytes) {
+// device array) -> a field with ghosts.
+int unpack_dense(gpe_ctx* c, const void* src, int field, int elem_bytes) {
   Launch L{};
   begin_timed(c, L, GPE_FAM_COPY, (int64_t)c->nint);
   const Geom g = geom(c);
   const int nb = row_blocks((size_t)c->Ny * c->Nz);
-  void* dst = c->fld[c->psi_id];
+  void* dst = c->fld[field];
   if (c->es == 8) {
     if (elem_bytes == 8)
       unpack_kernel<float, float><<<nb, 256, 0, c->stream>>>(
@@ -2129,6 +2179,13 @@ int load_dense(gpe_ctx* c, const void* src, int elem_bytes) {
   CU_CHECK(c, cudaGetLastError());
   end_timed(c, L);
   c->launches++;
+  return GPE_OK;
+}
+
+// The same -> psi, with no compensation yet.
+int load_dense(gpe_ctx* c, const void* src, int elem_bytes) {
+  const int rc = unpack_dense(c, src, c->psi_id, elem_bytes);
+  if (rc) return rc;
   if (c->prm.kahan && c->fld[c->c_id])
     CU_CHECK(c, cudaMemsetAsync(c->fld[c->c_id], 0, c->npad * (size_t)c->es,
                                 c->stream));
@@ -2138,6 +2195,32 @@ int load_dense(gpe_ctx* c, const void* src, int elem_bytes) {
   // be loaded yet: the group refreshes them before its next step
   if (c->group) c->ghosts_dirty = true;
   return exchange_ghosts(c, c->psi_id);
+}
+
+int pack_dense(gpe_ctx* c, int field, void* dst, int elem_bytes);
+
+// Fields with two ghost layers in place of GH, psi and its compensation kept
+// (both fit the staging buffer: only complex64 fields have one).
+int narrow_fields(gpe_ctx* c) {
+  unsigned char* st = static_cast<unsigned char*>(c->d_stage);
+  unsigned char* comp = st + c->nint * (size_t)c->es;
+  int rc = pack_dense(c, c->psi_id, st, c->es);
+  if (!rc && c->prm.kahan) rc = pack_dense(c, c->c_id, comp, c->es);
+  if (rc) return rc;
+  CU_CHECK(c, cudaStreamSynchronize(c->stream));
+  free_fields(c);
+  set_layout(c, 2);
+  c->maps.clear();
+  c->layout++;
+  for (auto& e : c->ext) e.reset();  // plans on the field's pitches
+  c->lost = true;  // until the smaller fields are there
+  rc = alloc_fields(c);
+  if (!rc) rc = unpack_dense(c, st, c->psi_id, c->es);
+  if (!rc && c->prm.kahan) rc = unpack_dense(c, comp, c->c_id, c->es);
+  if (rc) return rc;
+  CU_CHECK(c, cudaStreamSynchronize(c->stream));
+  c->lost = false;
+  return GPE_OK;
 }
 
 int stage_in(gpe_ctx* c, const void* src, int elem_bytes, bool device) {
@@ -2208,6 +2291,7 @@ int stage_out(gpe_ctx* c, int field, void* dst, int elem_bytes, bool device) {
 int check_ctx(gpe_ctx* c) {
   if (!c) return GPE_ERR_INVALID;
   CU_CHECK(c, cudaSetDevice(c->dev));
+  if (c->lost) return fail(c, GPE_ERR_OOM, "the context lost its fields (gpe_gpu_set_slab)");
   return GPE_OK;
 }
 
@@ -2323,6 +2407,7 @@ struct gpe_batch {
   cd prepared_dt = cd(0.0, 0.0);
   bool prepared = false;
   std::vector<int> prepared_psi;  // each member's psi buffer that [0] starts from
+  std::vector<int> prepared_layout;
   cudaGraph_t graph[2] = {nullptr, nullptr};
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
   double* graph_series = nullptr;
@@ -2475,7 +2560,11 @@ int batch_prepare(gpe_batch* b, cd dt) {
   b->prepared_dt = dt;
   b->prepared = true;
   b->prepared_psi.clear();
-  for (auto* c : b->runs) b->prepared_psi.push_back(c->psi_id);
+  b->prepared_layout.clear();
+  for (auto* c : b->runs) {
+    b->prepared_psi.push_back(c->psi_id);
+    b->prepared_layout.push_back(c->layout);
+  }
   return GPE_OK;
 }
 
@@ -2507,6 +2596,12 @@ const char* bad_opts(const gpe_batch_opts& o) {
   if (o.tile_y != 0 && o.tile_y != 4 && o.tile_y != 8) return "tile_y must be 0, 4 or 8";
   if (o.zchunk < 0 || o.ctas_per_sm < 0) return "zchunk and ctas_per_sm must be >= 0";
   return nullptr;
+}
+
+bool batch_pairs(const gpe_batch* b) {
+  bool all = b->form != FORM_FULL;
+  for (const auto* c : b->runs) all = all && c->gh >= GH;
+  return all;
 }
 
 // Rows per tile: 16 for complex64 pairs (pair_shape), else 8.
@@ -2742,11 +2837,7 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
   }
   c->nx = p.nx; c->ny = p.ny; c->nz = p.nz;
   c->es = p.precision;
-  c->gh = ghost_layers(c);
-  c->Nx = (int)round_up((size_t)p.nx + 2 * c->gh, 4);
-  c->Ny = p.ny + 2 * c->gh;
-  c->Nz = p.nz + 2 * c->gh;
-  c->npad = (size_t)c->Nx * c->Ny * c->Nz;
+  set_layout(c, ghost_layers(c));
   c->nint = (size_t)p.nx * p.ny * p.nz;
   c->nzg = p.nz;
   c->z_off = 0;
@@ -2761,25 +2852,6 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
 
   int rc = build_tables(c);
   if (rc) return bail(rc);
-  std::vector<int> need = {F_PSI, F_ALT};
-  switch (p.scheme) {
-    case GPE_SCHEME_RK2: need.push_back(F_UA); break;
-    case GPE_SCHEME_RK4:
-      need.insert(need.end(), {F_UB, F_ACC});
-      break;
-    case GPE_SCHEME_RK45:
-      need.insert(need.end(), {F_UA, F_UB, F_K1, F_K2, F_K3, F_K4, F_K5});
-      break;
-    default: break;
-  }
-  if (p.kahan) {
-    need.push_back(F_C);
-    if (p.scheme == GPE_SCHEME_RK45) need.push_back(F_CALT);
-  }
-  for (int id : need) {
-    rc = alloc_field(c, id);
-    if (rc) return bail(rc);
-  }
   // partials: upper bound over every launch shape (TY >= 4, zchunk >= 1)
   const size_t ntiles_max = (size_t)((p.nx + TX - 1) / TX) * ((p.ny + 3) / 4);
   c->partials_cap = std::max<size_t>(ntiles_max * (size_t)p.nz, 148 * 16);
@@ -2808,6 +2880,8 @@ int gpe_gpu_create(const gpe_params* prm, gpe_ctx** out) {
     c->err = "cudaHostAlloc of the step result failed";
     return bail(GPE_ERR_OOM);
   }
+  rc = alloc_fields(c);
+  if (rc) return bail(rc);
   cudaMemset(c->d_scal, 0, 16 * sizeof(double));
   cudaMemset(c->d_status, 0, sizeof(int));
   if (cudaDeviceSynchronize() != cudaSuccess) {
@@ -3322,6 +3396,11 @@ int gpe_gpu_set_slab(gpe_ctx* c, int32_t nz_global, int32_t z_offset) {
     return fail(c, GPE_ERR_INVALID, "reflective slabs need at least 4 planes");
   CU_CHECK(c, cudaStreamSynchronize(c->stream));
   rk45_drop_graphs(c);
+  // (with a communicator the layers are the same on every rank and stay)
+  if (nz_global > c->nz && c->gh > 2 && !c->group && !c->comm) {
+    rc = narrow_fields(c);
+    if (rc) return rc;
+  }
   c->nzg = nz_global;
   c->z_off = z_offset;
   // get_grid on the global axis, keeping this slab's planes
@@ -3333,6 +3412,7 @@ int gpe_gpu_set_slab(gpe_ctx* c, int32_t nz_global, int32_t z_offset) {
   }
   rc = build_tables(c);
   if (rc) return rc;
+  c->layout++;
   c->wide = false;
   c->norm_valid = false;
   return GPE_OK;
@@ -3408,7 +3488,7 @@ int gpe_group_create(gpe_ctx* const* members, int32_t n, gpe_group** out) {
   int z = 0;
   for (int r = 0; r < n; r++) {
     const gpe_ctx* c = members[r];
-    if (!c) return gfail(nullptr, GPE_ERR_INVALID, "null member");
+    if (!c || c->lost) return gfail(nullptr, GPE_ERR_INVALID, "null member");
     if (c->group || c->comm)
       return gfail(nullptr, GPE_ERR_INVALID, "member already in a group or joined to a communicator");
     const gpe_params &a = c->prm, &b = c0->prm;
@@ -3640,9 +3720,8 @@ int gpe_batch_create(const gpe_params* prms, int32_t nruns, const gpe_batch_opts
     b->form = std::max(b->form, form_of(rhs_form(c)));
     b->sites += (int64_t)c->nint;
   }
-  b->pairs = b->form != FORM_FULL;
+  b->pairs = batch_pairs(b);
   for (auto* c : b->runs) {
-    b->pairs = b->pairs && !network_grid(c);
     b->ghost_blocks = std::max(b->ghost_blocks, std::min(ghost_blocks(c, 16), 256));
   }
   if (cudaSetDevice(b->dev) != cudaSuccess ||
@@ -3761,9 +3840,18 @@ int gpe_batch_advance(gpe_batch* b, int64_t nsteps, double dt_re, double dt_im,
     BCU(b, cudaMalloc(&b->d_series, sizeof(double) * cap * nr));
     b->series_cap = cap;
   }
-  bool moved = false;  // a member was stepped on its own since the batch prepared
+  for (const auto* c : b->runs)
+    if (c->lost) return bfail(b, GPE_ERR_OOM, "a member lost its fields (gpe_gpu_set_slab)");
+  if (b->pairs && !batch_pairs(b)) {  // a member became a slab
+    batch_drop_graph(b);
+    b->pairs = false;
+    const int rc = batch_plan(b);
+    if (rc) return rc;
+  }
+  bool moved = false;  // a member was stepped or placed on its own since the batch prepared
   for (size_t r = 0; r < nr && b->prepared; r++)
-    moved = moved || b->prepared_psi[r] != b->runs[r]->psi_id;
+    moved = moved || b->prepared_psi[r] != b->runs[r]->psi_id ||
+            b->prepared_layout[r] != b->runs[r]->layout;
   if (!b->prepared || dt != b->prepared_dt || moved) {
     batch_drop_graph(b);
     const int rc = batch_prepare(b, dt);
