@@ -1438,8 +1438,9 @@ int fill_ghosts(gpe_ctx* c, int field) {
 // psi's ghosts for a pair, where the last writer filled fewer.
 int widen_ghosts(gpe_ctx* c) {
   if (c->wide) return GPE_OK;
-  c->wide = true;
-  return fill_ghosts(c, c->psi_id);
+  const int rc = fill_ghosts(c, c->psi_id);
+  c->wide = rc == GPE_OK;
+  return rc;
 }
 
 int launch_pair(gpe_ctx* c, const PairSpec& sp) {
