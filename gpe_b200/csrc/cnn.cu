@@ -171,7 +171,8 @@ int check_view(gpe_cnn* n, const FieldView& v) {
   if (v.nx != n->nx || v.ny != n->ny || v.nz != n->nz)
     return cfail(n, GPE_ERR_INVALID, "context grid differs from the network's grid");
   if (v.es != 8) return cfail(n, GPE_ERR_INVALID, "the learned correction needs complex64 psi");
-  if (v.bcs != 1) return cfail(n, GPE_ERR_INVALID, "the learned correction needs periodic bcs");
+  if (!network_fits(v.nx, v.es, v.bcs))
+    return cfail(n, GPE_ERR_INVALID, "the learned correction needs periodic bcs");
   if (!v.single_domain) return cfail(n, GPE_ERR_INVALID, "z-slab contexts are not supported");
   if (v.dev != n->dev) return cfail(n, GPE_ERR_INVALID, "context on another device");
   return GPE_OK;
@@ -335,7 +336,7 @@ int gpe_cnn_create(const gpe_cnn_params* p, gpe_cnn** out) {
   *out = nullptr;
   if (p->struct_size != (int32_t)sizeof(gpe_cnn_params))
     return cfail(nullptr, GPE_ERR_INVALID, "gpe_cnn_params struct_size mismatch");
-  if (p->nx < 16 || p->nx > 128 || p->nx % 16 != 0)
+  if (!network_nx(p->nx))
     return cfail(nullptr, GPE_ERR_INVALID, "nx must be a multiple of 16 in [16, 128]");
   if (p->ny < 1 || p->nz < 1) return cfail(nullptr, GPE_ERR_INVALID, "ny, nz must be >= 1");
   if (!(std::isfinite(p->out_scale) && p->out_scale != 0.f))

@@ -747,15 +747,14 @@ void recipe_masks(const StageSpec& sp, int* am, int* bm) {
   }
 }
 
-// A grid that a correction network can be attached to (gpe_cnn_create:
-// complex64, periodic, nx a multiple of 16 up to 128).  The network rounds psi
+// A grid that a correction network can be attached to.  The network rounds psi
 // to bfloat16, which makes last-bit differences of psi differences of 1e-5, so
 // rk4 keeps on these grids the summation order its weights were trained with,
 // d4, d2, d3 one after another, attached or not; on all others the pointwise
 // increments are summed first, which lets two stages share a launch with one
 // stored sum (pair_kernel.cuh).
 bool network_grid(const gpe_ctx* c) {
-  return c->es == 8 && c->prm.bcs == 1 && c->nx % 16 == 0 && c->nx <= 128;
+  return gpe::network_fits(c->nx, c->es, c->prm.bcs);
 }
 
 // Ghost layers of a context's fields: GH where its steps can run in pairs (see

@@ -29,6 +29,12 @@ struct FieldView {
   bool overlap;       // launches on the stream may overlap (stream_overlap in gpe_gpu.cu)
 };
 
+// Whether a correction network can work on a grid: rows of nx sites (a multiple
+// of an MMA's 16, up to its 128 rows), complex of es bytes, boundary bcs.  Asked by
+// the network's own checks and by rk4, which keeps its order of summation there.
+inline bool network_nx(int nx) { return nx >= 16 && nx <= 128 && nx % 16 == 0; }
+inline bool network_fits(int nx, int es, int bcs) { return network_nx(nx) && es == 8 && bcs == 1; }
+
 // Lets every launch of fn take as much dynamic shared memory as a block may
 // have.  The limit is the function's, shared by all contexts, threads and
 // launches of the process, while what a launch needs depends on its grid: a
