@@ -187,15 +187,17 @@ __global__ void __launch_bounds__(1024) ghosts_norm_kernel(TS* f, Geom g, int de
   }
 }
 
-// The ghosts of one field per member of a batch (blockIdx.y).
+// The ghosts of one field per member of a batch, nblocks blocks a member (all along
+// the grid's x, which has room for any number of members).
 struct GhostRun {
   void* field;
   Geom g;
 };
 template <typename TS>
-__global__ void batch_ghosts_kernel(const GhostRun* __restrict__ runs, int depth) {
-  const GhostRun r = runs[blockIdx.y];
-  fill_ghost_rows<TS>(static_cast<TS*>(r.field), r.g, depth, blockIdx.x, gridDim.x);
+__global__ void batch_ghosts_kernel(const GhostRun* __restrict__ runs, int depth, int nblocks) {
+  const int run = blockIdx.x / nblocks;
+  const GhostRun r = runs[run];
+  fill_ghost_rows<TS>(static_cast<TS*>(r.field), r.g, depth, blockIdx.x - run * nblocks, nblocks);
 }
 
 // Padded field -> dense interior array of TO, one warp per row.

@@ -2577,11 +2577,12 @@ int batch_enqueue_step(gpe_batch* b, int par) {
     BCU(b, cudaLaunchKernel(S.fn, dim3((unsigned)S.grid), dim3(32, (unsigned)S.warps), args, S.smem,
                             b->stream));
     if (b->pairs) {
-      const dim3 grid((unsigned)b->ghost_blocks, (unsigned)b->runs.size());
+      const int nb = b->ghost_blocks;
+      const unsigned grid = (unsigned)nb * (unsigned)b->runs.size();
       if (b->es == 8)
-        batch_ghosts_kernel<float><<<grid, 256, 0, b->stream>>>(b->d_ghosts[par][s], 2 * b->R);
+        batch_ghosts_kernel<float><<<grid, 256, 0, b->stream>>>(b->d_ghosts[par][s], 2 * b->R, nb);
       else
-        batch_ghosts_kernel<double><<<grid, 256, 0, b->stream>>>(b->d_ghosts[par][s], 2 * b->R);
+        batch_ghosts_kernel<double><<<grid, 256, 0, b->stream>>>(b->d_ghosts[par][s], 2 * b->R, nb);
     }
   }
   batch_finalize_kernel<<<(unsigned)b->runs.size(), 256, 0, b->stream>>>(

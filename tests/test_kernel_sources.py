@@ -82,3 +82,11 @@ def test_every_launch_asks_the_rule_for_overlap():
                 calls += re.findall(r"launch_overlapped\(\s*([^,]+),", h.read())
     assert len(calls) >= 15
     assert set(calls) <= {"overlap(c)", "ov", "v.overlap"}, sorted(set(calls))
+
+
+def test_members_of_a_batch_lie_along_the_x_of_a_grid():
+    """A grid has 65535 blocks along y and z: a launch with one per member there
+    would refuse batches that the others take."""
+    for name, defs in functions().items():
+        for _, body in defs:
+            assert "blockIdx.y" not in body and "blockIdx.z" not in body, name
