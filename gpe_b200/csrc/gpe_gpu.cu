@@ -2654,6 +2654,24 @@ long batch_deal(const gpe_batch* b, const std::vector<WorkItem>& items, int ctas
   return longest;
 }
 
+// CTAs that both pair launches of the batch can have on an SM at its tile height:
+// lists beyond them would run after the others, not beside them.
+template <typename T>
+int batch_pair_occupancy(gpe_batch* b, int* occ) {
+  PairSpec sp[2];
+  rk4_pairs(b->runs[0], cd(0.0), sp);
+  *occ = 1 << 20;
+  for (const PairSpec& q : sp) {
+    KernelFn fn = pair_kernel_fn(b->es, b->R, q.kind, q.comp >= 0, b->form, true);
+    if (!fn) return bfail(b, GPE_ERR_INVALID, "no batched pair kernel");
+    PairShape sh;
+    const int rc = pair_shape<T>(b->runs[0], fn, b->R, q, b->TY, &sh);
+    if (rc) return bfail(b, rc, b->runs[0]->err);
+    *occ = std::min(*occ, sh.occ);
+  }
+  return GPE_OK;
+}
+
 // The work list of b->opts: one stage per launch, the members' items by the
 // sites they touch (warm-up planes included), largest first, walked round-robin
 // by the persistent CTAs; pairs, a list per CTA (batch_deal), with the chunk
@@ -2664,7 +2682,11 @@ int batch_plan(gpe_batch* b) {
   std::vector<WorkItem> items, sorted;
   std::vector<int> starts;
   if (b->pairs) {
-    const int per_sm = o.ctas_per_sm > 0 ? o.ctas_per_sm : b->TY <= 4 ? 2 : 1;
+    int per_sm = 1;
+    const int rc = b->es == 8 ? batch_pair_occupancy<float>(b, &per_sm)
+                              : batch_pair_occupancy<double>(b, &per_sm);
+    if (rc) return rc;
+    if (o.ctas_per_sm > 0) per_sm = std::min(per_sm, o.ctas_per_sm);
     const int ctas = per_sm * b->runs[0]->num_sms;
     int zc = o.zchunk;
     if (zc <= 0) {
