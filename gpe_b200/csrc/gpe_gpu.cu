@@ -3419,8 +3419,8 @@ int gpe_gpu_set_slab(gpe_ctx* c, int32_t nz_global, int32_t z_offset) {
     return fail(c, GPE_ERR_INVALID, "reflective slabs need at least 4 planes");
   CU_CHECK(c, cudaStreamSynchronize(c->stream));
   rk45_drop_graphs(c);
-  // (with a communicator the layers are the same on every rank and stay)
-  if (nz_global > c->nz && c->gh > 2 && !c->group && !c->comm) {
+  // (members of a group and ranks have two layers already)
+  if (nz_global > c->nz && c->gh > 2) {
     rc = narrow_fields(c);
     if (rc) return rc;
   }
@@ -3461,6 +3461,12 @@ int gpe_gpu_comm_init(gpe_ctx* c, const void* id128, int32_t rank, int32_t nrank
   if (c->comm) return fail(c, GPE_ERR_INVALID, "communicator already set");
   std::string why;
   if (!load_nccl(&why)) return fail(c, GPE_ERR_CUDA, why);
+  // ranks send each other whole padded planes, so all have the layers that a
+  // stage needs, also where one of them got no more (alloc_fields)
+  if (c->gh > 2) {
+    rc = narrow_fields(c);
+    if (rc) return rc;
+  }
   ncclUniqueId id;
   memcpy(&id, id128, sizeof(id));
   NCCL_CHECK(c, g_nccl.CommInitRank(&c->comm, nranks, id, rank));

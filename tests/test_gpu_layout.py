@@ -68,6 +68,21 @@ def test_a_slab_has_two_layers_and_keeps_its_state(scheme, precision, kahan):
         assert np.array_equal(s.get_state(dtype), t.get_state(dtype))
 
 
+@pytest.mark.parametrize("scheme,precision,kahan", [("rk4", 8, True), ("rk2", 16, False)])
+def test_a_rank_has_two_layers(scheme, precision, kahan):
+    """Ranks exchange whole padded planes, whose size follows from the layers: all
+    have two."""
+    from gpe_b200.dist import SlabSolver
+    n = (30, 21, 12)
+    prm = GpeParams(nx=n[0], ny=n[1], nz=n[2], xr=3.0, yr=3.0, zr=3.0, order=4, bcs=1,
+                    scheme=scheme, precision=precision, kahan=kahan)
+    fields = {"rk4": 4, "rk2": 3}[scheme] + kahan
+    sites = lambda g: rounded(n[0] + 2 * g) * (n[1] + 2 * g) * (n[2] + 2 * g)  # noqa: E731
+    with GpeSolver(prm, dt=1e-3) as s, SlabSolver(prm, rank=0, nranks=1, dist=None, dt=1e-3) as r:
+        saved = lib().gpe_gpu_device_bytes(s.handle) - lib().gpe_gpu_device_bytes(r._ctx)
+        assert saved == fields * precision * (sites(4) - sites(2))
+
+
 def test_a_batch_follows_a_member_that_is_placed():
     """Placing a member moves its tables and fields: the batch steps on the new
     ones, one stage per launch from then on."""
