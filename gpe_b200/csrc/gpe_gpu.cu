@@ -143,8 +143,9 @@ struct Launch {
 void gpe_internal_set_last_error(const std::string& msg) { g_last_create_error = msg; }
 
 namespace {
-// Page-locked StepResults, 64 to an allocation: page-locking takes 3 to 8 ms, as
-// long as the rest of creating a context, and an ensemble has one per run.  An
+// Page-locked StepResults, 64 to an allocation: an ensemble has one per run.  Locking
+// takes 1.6 ms the first time in a process (some microseconds after that), beside
+// the 50 ms in which a process's first context comes up and loads its state.  An
 // allocation whose last result is given back is freed, but for one (1 KB) that
 // the next context finds.
 struct ResultPages {

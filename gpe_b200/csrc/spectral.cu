@@ -70,8 +70,7 @@ struct Spectral : Extension {
   cufftHandle plan_psi = 0;  // padded psi interior -> dense staging buffer
   bool has_plan = false, has_plan_psi = false;
   double* d_axes = nullptr;      // ax[nx], ay[ny], az[nz]
-  double* d_partials = nullptr;  // [nblk][HEAD + nf]
-  double* d_cols = nullptr;      // [HEAD + nf] column sums of the partials
+  double* d_partials = nullptr;  // [nblk][HEAD + nf], and a row of the columns' sums
   double* d_out = nullptr;       // [21 + nf]
   int nblk = 0, nf = 0;
   ~Spectral() override {
@@ -79,7 +78,6 @@ struct Spectral : Extension {
     if (has_plan_psi && g_fft.ok) g_fft.Destroy(plan_psi);
     cudaFree(d_axes);
     cudaFree(d_partials);
-    cudaFree(d_cols);
     cudaFree(d_out);
   }
 };
@@ -188,15 +186,13 @@ int launch_spectrum(gpe_ctx* c, Spectral* s, const FieldView& v, const SpecArgs&
   const int nblk = (int)(want < cap ? want : cap);
   if (nblk != s->nblk || f0.nf != s->nf) {
     cudaFree(s->d_partials);
-    cudaFree(s->d_cols);
     cudaFree(s->d_out);
-    s->d_partials = s->d_cols = s->d_out = nullptr;
+    s->d_partials = s->d_out = nullptr;
     // mark the cache empty first: a failed allocation below must not leave
     // sizes that let the next call launch on null buffers
     s->nblk = 0;
     s->nf = -1;
-    SP_CU(c, cudaMalloc(&s->d_partials, sizeof(double) * (size_t)nblk * (HEAD + f0.nf)));
-    SP_CU(c, cudaMalloc(&s->d_cols, sizeof(double) * (size_t)(HEAD + f0.nf)));
+    SP_CU(c, cudaMalloc(&s->d_partials, sizeof(double) * (size_t)(nblk + 1) * (HEAD + f0.nf)));
     SP_CU(c, cudaMalloc(&s->d_out, sizeof(double) * (size_t)(21 + f0.nf)));
     s->nblk = nblk;
     s->nf = f0.nf;
@@ -215,10 +211,11 @@ int launch_spectrum(gpe_ctx* c, Spectral* s, const FieldView& v, const SpecArgs&
   gpe_internal_time_end(c, &t1);
   gpe_internal_time_begin(c, &t2, GPE_FAM_REDUCE, 0);
   const int ncol = HEAD + f.nf;
+  double* cols = s->d_partials + (size_t)nblk * ncol;
   spectrum_columns_kernel<<<(ncol + 31) / 32, F_FIN_THREADS, 0, v.stream>>>(s->d_partials, nblk, ncol,
-                                                                          s->d_cols);
+                                                                          cols);
   SP_CU(c, cudaGetLastError());
-  spectrum_finalize_kernel<T><<<1, F_FIN_THREADS, fsmem, v.stream>>>(buf, s->d_cols, f);
+  spectrum_finalize_kernel<T><<<1, F_FIN_THREADS, fsmem, v.stream>>>(buf, cols, f);
   SP_CU(c, cudaGetLastError());
   gpe_internal_time_end(c, &t2);
   gpe_internal_count_launches(c, 3);
