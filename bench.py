@@ -55,10 +55,11 @@ KMAX = 1.0
 # algorithmic bytes per site per RK4 step with complex64 + Kahan.  Two stages per
 # launch (single grids): the first pair reads psi and writes psi + d3 and the
 # increments' sum (3 x 8 B), the second reads both, psi and c and writes psi', c
-# (6 x 8 B) -> 72 B/site.  One stage per launch (z-slabs), increment form: stage 1 reads psi and writes d2 (2 x 8 B); stages 2-3 read psi and d
-# (both as stencils) and write the next d (3 x 8 B each); stage 4 reads psi,
-# d4, d2, d3, c and writes psi', c (7 x 8 B) -> 120 B/site (the stage-value +
-# accumulator form moves 152)
+# (6 x 8 B) -> 72 B/site.  One stage per launch (z-slabs, and grids that a
+# network can correct), increment form: stage 1 reads psi and writes d2 (2 x 8 B);
+# stages 2-3 read psi and d (both as stencils) and write the next d (3 x 8 B
+# each); stage 4 reads psi, d4, d2, d3, c and writes psi', c (7 x 8 B) -> 120
+# B/site (the stage-value + accumulator form moves 152)
 BYTES_PER_FAMILY = {"stage_first": 16, "stage_mid": 24, "stage_last": 56}
 BYTES_PER_STEP = 120
 BYTES_PER_STEP_PAIRS = 72
@@ -236,10 +237,9 @@ ENS_RUNS = 64
 ENS_SIZES = (32, 48, 64, 96, 128)
 ENS_DT = 0.01
 ENS_KMAX = 0.8
-# complex64 without compensation, increment form: stage 1 reads psi, writes
-# d2 (16 B); stages 2-3 read psi, d and write the next d (24 B each); stage 4
-# reads psi, d4, d2, d3 and writes psi' (40 B)
-ENS_BYTES_PER_SITE = 56  # two stages per launch, no compensation: 24 + 32
+# complex64 without compensation, two stages per launch: the first pair reads psi
+# and writes two fields (24 B), the second reads three and writes psi' (32 B)
+ENS_BYTES_PER_SITE = 56
 
 
 def ensemble_members(seed=0):
@@ -959,13 +959,21 @@ def main():
                     "families": fam}
     else:
         kernel_ms_step = ms / args.steps
-        step_gbs = BYTES_PER_STEP_PAIRS * sites / (kernel_ms_step / 1e3) / 1e9
-        roofline = {"bound": "hbm", "kernel": "pair_kernel (both pairs of the step, with the "
-                                              "ghost and norm launches after them)",
+        # a step is four launches in pairs (each pair and what follows it), five
+        # one stage at a time
+        pairs = launches < 5 * args.steps
+        per_site = BYTES_PER_STEP_PAIRS if pairs else BYTES_PER_STEP
+        step_gbs = per_site * sites / (kernel_ms_step / 1e3) / 1e9
+        # (the traffic was measured on the default grid)
+        traffic = load_traffic().get("pairs") if pairs and sites == N_GRID ** 3 else None
+        roofline = {"bound": "hbm",
+                    "kernel": ("pair_kernel (both pairs of the step, with the ghost and norm "
+                               "launches after them)" if pairs else
+                               "stage_kernel (the four stages of the step and the norm)"),
                     "achieved": step_gbs, "peak": peak, "unit": "GB/s", "frac": step_gbs / peak,
-                    "peak_source": peak_kind, "traffic": load_traffic().get("pairs"),
-                    "alg_bytes_per_step": BYTES_PER_STEP_PAIRS * sites,
-                    "step": {"alg_bytes_per_site": BYTES_PER_STEP_PAIRS,
+                    "peak_source": peak_kind, "traffic": traffic,
+                    "alg_bytes_per_step": per_site * sites,
+                    "step": {"alg_bytes_per_site": per_site,
                              "kernel_ms_per_step": kernel_ms_step,
                              "frac_vs_nominal_8000": step_gbs / 8000.0}}
 
