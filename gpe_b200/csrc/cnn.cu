@@ -122,8 +122,7 @@ int launch_conv(gpe_cnn* n, const FieldView& v, const Act& in, int layer, bool d
   p.Xp = n->Xp; p.Yp = n->Yp; p.Zp = n->Zp; p.Hin = in.H;
   conv_items(n, TYF, &p.nslab, &p.nzc, &p.zchunk);
   p.nitems = p.nslab * p.nzc;
-  p.box_bytes = (uint32_t)((TYF + 2) * in.H * n->Xp * 16);
-  p.slot_bytes = round1k(p.box_bytes);
+  p.slot_bytes = round1k((uint32_t)((TYF + 2) * in.H * n->Xp * 16));
   p.out_scale = n->prm.out_scale;
   if (!p.status) p.status = n->d_status;
   p.wait_limit_ns = CNN_WAIT_LIMIT_NS;

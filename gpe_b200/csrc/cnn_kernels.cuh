@@ -65,7 +65,6 @@ namespace cnn {
 constexpr int CH = 16;
 constexpr int NTAP = 27;
 constexpr int NLAYER = 4;
-constexpr int TAP_BYTES = 2 * CH * 8 * 2;  // [2 halves][16 rows][8] bf16 = 512
 
 // forward / dgrad
 constexpr int TYF = 8;          // output rows per item
@@ -138,7 +137,7 @@ struct ConvParams {
   const float* bias;                // [16] or null
   int nx, ny, nz, Xp, Yp, Zp, Hin;
   int nslab, nzc, zchunk, nitems;
-  uint32_t slot_bytes, box_bytes;
+  uint32_t slot_bytes;
   __nv_bfloat16* act_out;           // [Zp][Yp][2][Xp][8]
   __nv_bfloat16* pre_out;           // EPI_GELU_PRE
   const __nv_bfloat16* pre_in;      // EPI_DGELU
@@ -247,20 +246,6 @@ __device__ __forceinline__ void store_act16(__nv_bfloat16* q, int Xp, int Yp, in
     row(q - sz);
     if (y0) row(q - sz + sy);
     if (y1) row(q - sz - sy);
-  }
-}
-
-__device__ __forceinline__ void load_act16(const __nv_bfloat16* buf, int Xp, int Yp, int x,
-                                           int y, int z, float (&a)[16]) {
-  const uint4 lo = *reinterpret_cast<const uint4*>(buf + act_index(Xp, Yp, x + 1, y + 1, z + 1, 0));
-  const uint4 hi = *reinterpret_cast<const uint4*>(buf + act_index(Xp, Yp, x + 1, y + 1, z + 1, 1));
-  const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
-    const float2 f = __bfloat1622float2(v);
-    a[2 * i] = f.x;
-    a[2 * i + 1] = f.y;
   }
 }
 

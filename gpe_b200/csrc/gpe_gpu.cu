@@ -1261,7 +1261,6 @@ struct PairSpec {
   int s = F_PSI, base = -1, acc = -1, comp = -1;  // fields read
   int out0 = F_ALT, out1 = -1;                    // fields written (out1: no ghosts)
   cd a[2] = {cd(0), cd(0)};
-  int family = GPE_FAM_OTHER;
 };
 
 // A context steps with pairs unless its fields have no room for their ghosts (the
@@ -1474,7 +1473,6 @@ void rk4_pairs(const gpe_ctx* c, cd dt, PairSpec sp[2]) {
   sp[0].out0 = F_UB;
   sp[0].out1 = c->alt_id;
   sp[0].a[0] = sp[0].a[1] = 0.5 * dt;
-  sp[0].family = GPE_FAM_STAGE_FIRST;
   sp[1] = PairSpec();
   sp[1].kind = PAIR_RK4_B;
   sp[1].s = F_UB;
@@ -1484,7 +1482,6 @@ void rk4_pairs(const gpe_ctx* c, cd dt, PairSpec sp[2]) {
   sp[1].a[0] = dt;
   sp[1].a[1] = dt / 6.0;
   if (c->prm.kahan) sp[1].comp = sp[1].out1 = c->c_id;
-  sp[1].family = GPE_FAM_STAGE_LAST;
 }
 
 int step_rk4_pairs(gpe_ctx* c, cd dt) {
@@ -1507,7 +1504,6 @@ int step_rk2_pair(gpe_ctx* c, cd dt) {
   sp.a[0] = 0.5 * dt;
   sp.a[1] = dt;
   if (c->prm.kahan) sp.comp = sp.out1 = c->c_id;
-  sp.family = GPE_FAM_STAGE_LAST;
   int rc = widen_ghosts(c);
   if (!rc) rc = launch_pair(c, sp);
   if (rc) return rc;
