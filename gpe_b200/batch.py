@@ -24,8 +24,8 @@ from .solver import GpeParams, GpeSolver
 @dataclass
 class BatchOpts:
     tile_y: int = 0        # 0 = the tallest built (8, or 16 in complex64 pairs); else 4 or 8
-    zchunk: int = 0        # 0 = auto (an equal share per CTA) planes per work item
-    ctas_per_sm: int = 0   # 0 = as many as fit
+    zchunk: int = 0        # planes per work item; 0 = auto (64; pairs: the shortest longest CTA share)
+    ctas_per_sm: int = 0   # 0 = as many as fit; no more than that
     use_graph: bool = True
 
     def to_c(self) -> GpeBatchOptsC:

@@ -389,8 +389,9 @@ typedef struct gpe_batch gpe_batch;
 typedef struct gpe_batch_opts {
   int32_t struct_size;  /* sizeof(gpe_batch_opts) */
   int32_t tile_y;       /* 0 = the tallest built (8, or 16 in complex64 pairs); else 4 or 8 */
-  int32_t zchunk;       /* 0 = auto, an equal share per CTA; z-planes per work item */
-  int32_t ctas_per_sm;  /* 0 = as many as fit */
+  int32_t zchunk;       /* z-planes per work item; 0 = auto: 64, or in pairs the
+                           length whose longest CTA share is shortest */
+  int32_t ctas_per_sm;  /* 0 = as many as fit; no more than that */
   int32_t use_graph;    /* 1 = replay a captured CUDA graph per step */
 } gpe_batch_opts;
 void gpe_batch_default_opts(gpe_batch_opts* opts);
