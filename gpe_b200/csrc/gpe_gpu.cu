@@ -1451,6 +1451,7 @@ int finish_pairs(gpe_ctx* c) {
   const Geom g = geom(c);
   const int depth = c->prm.order, nb = ghost_blocks(c, 32) + 1;
   cudaError_t e;
+  c->wide = false;  // until the launch is accepted
   if (c->es == 8)
     e = launch_overlapped(overlap(c), ghosts_norm_kernel<float>, nb, 1024, 0, c->stream,
                           c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk,
@@ -1460,6 +1461,7 @@ int finish_pairs(gpe_ctx* c) {
                           c->fld[c->psi_id], g, depth, c->d_partials, c->last_nblk,
                           cell_volume(c), c->d_scal, c->step_series, c->h_res, c->d_status);
   CU_CHECK(c, e);
+  c->wide = true;
   c->launches++;
   return GPE_OK;
 }
@@ -3887,6 +3889,7 @@ int gpe_batch_advance(gpe_batch* b, int64_t nsteps, double dt_re, double dt_im,
     for (auto* c : b->runs) {
       const int rc = widen_ghosts(c);
       if (rc) return bfail(b, rc, c->err);
+      c->wide = false;  // until the steps are queued
     }
   // members' own kernels (state loads) must be done before the batch runs
   for (auto* c : b->runs) BCU(b, cudaStreamSynchronize(c->stream));
@@ -3918,7 +3921,7 @@ int gpe_batch_advance(gpe_batch* b, int64_t nsteps, double dt_re, double dt_im,
   if (nsteps & 1) batch_flip(b);
   for (auto* c : b->runs) {
     c->norm_valid = false;
-    if (!b->pairs && nsteps > 0) c->wide = false;
+    if (nsteps > 0) c->wide = b->pairs;
   }
   if (norms && nsteps > 0) {
     // series is [run][cap]: copy the first nsteps of each run
