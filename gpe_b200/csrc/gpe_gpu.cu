@@ -1267,11 +1267,14 @@ struct PairSpec {
 // equation has the sphere mask, rk4 keeps the increments apart, the grid is a
 // slab: ghost_layers), its z ghosts come from neighbours (two planes are
 // exchanged, a pair needs four), per-launch timing is on, whose families are
-// single stages, or the full form, whose terms
-// spill the pair's registers, except in complex64 at order 2 (equation 1 at
-// 150 x 93 x 71, rk4, us a step in pairs and in stages: 54 and 59 there;
-// complex128 95 and 97 at order 2, 182 and 125 at order 4; rk2 at 200 x 193 x
-// 171, complex128, order 2: 223 and 209).
+// single stages, or the full form except in complex64 at order 2.  Equation 1 with
+// gradient and sponge, us a step in pairs and in stages: there 21.7 and 26.3 at
+// 64^3, 40.9 and 56.1 at 150 x 93 x 71, 340 and 535 at 256^3 (rk4; rk2 11.3 and
+// 14.0, 20.7 and 25.2, 167 and 229).  Complex128 spills: 95 and 97 at order 2, 182
+// and 125 at order 4 (rk4, 150 x 93 x 71), rk2 at 200 x 193 x 171 223 and 209.
+// Complex64 at order 4 has none built: it would lose the smallest grids and gain
+// the others (35.5 and 32.0, 68.8 and 77.0, 712 and 781; rk2 16.9 and 16.4, 32.4
+// and 36.4, 334 and 347).
 bool steps_in_pairs(const gpe_ctx* c) {
   if (c->gh < GH || c->comm || c->group || c->nzg != c->nz || c->timing) return false;
   return (c->prm.order == 2 && c->es == 8) || !rhs_form(c).full;
