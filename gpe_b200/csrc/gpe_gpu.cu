@@ -2293,7 +2293,7 @@ int stage_out(gpe_ctx* c, int field, void* dst, int elem_bytes, bool device) {
 int check_ctx(gpe_ctx* c) {
   if (!c) return GPE_ERR_INVALID;
   CU_CHECK(c, cudaSetDevice(c->dev));
-  if (c->lost) return fail(c, GPE_ERR_OOM, "the context lost its fields (gpe_gpu_set_slab)");
+  if (c->lost) return fail(c, GPE_ERR_OOM, "the context lost its fields as they were made smaller");
   return GPE_OK;
 }
 
@@ -3872,7 +3872,7 @@ int gpe_batch_advance(gpe_batch* b, int64_t nsteps, double dt_re, double dt_im,
     b->series_cap = cap;
   }
   for (const auto* c : b->runs)
-    if (c->lost) return bfail(b, GPE_ERR_OOM, "a member lost its fields (gpe_gpu_set_slab)");
+    if (c->lost) return bfail(b, GPE_ERR_OOM, "a member lost its fields as they were made smaller");
   if (b->pairs && !batch_pairs(b)) {  // a member became a slab
     batch_drop_graph(b);
     b->pairs = false;

@@ -337,7 +337,10 @@ int gpe_gpu_set_real_time(gpe_ctx* ctx, int32_t real_time);
  *
  * gpe_gpu_set_slab: this context (created with nz = the slab's planes) holds
  * planes z_offset .. z_offset+nz-1 of a global axis of nz_global planes
- * (prm->zr is the global half-width).  Call before gpe_gpu_set_state. */
+ * (prm->zr is the global half-width).  Call before gpe_gpu_set_state.
+ * Placing a context, or joining it to a communicator, moves its fields into
+ * smaller ones (slabs have two ghost layers); should those not be allocated,
+ * GPE_ERR_OOM is returned and the context can only be destroyed. */
 int gpe_gpu_set_slab(gpe_ctx* ctx, int32_t nz_global, int32_t z_offset);
 /* A 128-byte NCCL unique id, made on one rank; the caller broadcasts it. */
 int gpe_gpu_comm_unique_id(void* id128);
@@ -354,10 +357,10 @@ int gpe_gpu_comm_init(gpe_ctx* ctx, const void* id128, int32_t rank,
 
 /* Batched ensembles (no reference counterpart; the reference runs one grid
  * per job).  Independent runs of uneven grids, each a full member context,
- * are stepped together with rk4: every stage is ONE persistent launch over a
- * work list of (run, tile, z-range) items of all members, and a whole step
- * (4 stage launches + per-run norm) is captured once in a CUDA graph and
- * replayed.  Members share scheme (rk4), order, bcs, equation, precision,
+ * are stepped together with rk4: two stages (one, where a member's right-hand
+ * side or grid has no pair) are ONE persistent launch over a work list of
+ * (run, tile, z-range) items of all members, and a whole step (the launches,
+ * ghosts, per-run norm) is captured once in a CUDA graph and replayed.  Members share scheme (rk4), order, bcs, equation, precision,
  * kahan, device and time direction; grids, box sizes, g, mu and trap may
  * differ. */
 /* In-process slab group: z-slab contexts of one grid on one device (each
